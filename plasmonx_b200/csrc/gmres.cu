@@ -363,20 +363,75 @@ __device__ __forceinline__ void zrot_(double2 &x, double2 &y, double c, double2 
     y = ny;
 }
 
-// Givens update of column j for every active column (one thread each).
+__device__ __forceinline__ double2 shfl2(double2 v, int lane) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+__device__ __forceinline__ double2 shfl_up2(double2 v, int o) {
+    return make_double2(__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o));
+}
+
+// Givens update of column j, one warp per active column.
 // Hcols[j] points to the slab of H column j ([C][hstride] complex).
-__global__ void givens(int count, int j, const int32_t *__restrict__ act,
-                       double2 *const *__restrict__ Hcols, int hstride, double *__restrict__ cs,
-                       double2 *__restrict__ sn, double2 *__restrict__ g, int gstride, int cstride,
-                       double *__restrict__ resid) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// The j earlier rotations form a chain: with a_0 = h_0 the i-th rotation gives
+// h_i' = c_i a_i + s_i h_{i+1} and passes on a_{i+1} = c_i h_{i+1} - conj(s_i) a_i.
+// One thread walking it pays a dependent global load and ~6 FP64 latencies per
+// rotation (2.1 us per 16 rotations).  The chain is a composition of maps
+// a -> p a + q, so a warp takes 32 rotations at a time (coalesced loads) and
+// composes them with a 5-step scan; |p| <= 1 throughout, so the composition is
+// as stable as the chain.  The result depends on j alone, not on the batch.
+// Latency bound; per launch, before -> after: 81 -> 6.1 us at 61 columns and 130
+// steps on average, 94 -> 8.5 us at 4 columns and 360 steps.
+constexpr int kGivensWarps = 2;
+
+__global__ void __launch_bounds__(32 * kGivensWarps) givens(int count, int j, const int32_t *__restrict__ act,
+                                                            double2 *const *__restrict__ Hcols, int hstride,
+                                                            double *__restrict__ cs, double2 *__restrict__ sn,
+                                                            double2 *__restrict__ g, int gstride, int cstride,
+                                                            double *__restrict__ resid) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= count) return;
-    int c = act[k];
+    const int c = act[k];
     double2 *h = Hcols[j] + (int64_t)c * hstride;
     double *csc = cs + (int64_t)c * cstride;
     double2 *snc = sn + (int64_t)c * cstride;
-    for (int i = 0; i < j; ++i) zrot_(h[i], h[i + 1], csc[i], snc[i]);
-    double2 ca = h[j], cb = h[j + 1];
+    double2 *gc = g + (int64_t)c * gstride;
+    double2 a = h[0];                        // chain value entering the tile (same in every lane)
+    double2 cb = h[j + 1], g0 = gc[j], g1 = gc[j + 1];
+    double ci = lane < j ? csc[lane] : 1.0;
+    double2 si = lane < j ? snc[lane] : make_double2(0.0, 0.0);
+    double2 hn = lane < j ? h[lane + 1] : make_double2(0.0, 0.0);
+    for (int i0 = 0; i0 < j; i0 += 32) {
+        const int i = i0 + lane, in = i + 32;
+        // the next tile's loads, in flight during this tile's scan
+        const double cin = in < j ? csc[in] : 1.0;
+        const double2 sin_ = in < j ? snc[in] : make_double2(0.0, 0.0);
+        const double2 hnn = in < j ? h[in + 1] : make_double2(0.0, 0.0);
+        double2 p = i < j ? make_double2(-si.x, si.y) : make_double2(1.0, 0.0);      // -conj(s)
+        double2 q = i < j ? make_double2(ci * hn.x, ci * hn.y) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double2 pp = shfl_up2(p, o), qq = shfl_up2(q, o);
+            if (lane >= o) {
+                const double2 t = cmul(p, qq);
+                q.x += t.x;
+                q.y += t.y;
+                p = cmul(p, pp);
+            }
+        }
+        const double2 t = cmul(p, a);
+        const double2 out = make_double2(t.x + q.x, t.y + q.y);      // a after this lane's rotation
+        double2 ai = shfl_up2(out, 1);                               // a before it
+        if (lane == 0) ai = a;
+        if (i < j)
+            h[i] = make_double2(ci * ai.x + (si.x * hn.x - si.y * hn.y), ci * ai.y + (si.x * hn.y + si.y * hn.x));
+        a = shfl2(out, 31);
+        ci = cin;
+        si = sin_;
+        hn = hnn;
+    }
+    if (lane != 0) return;
+    double2 ca = a;
     double cj;
     double2 sj;
     if (cabs_(ca) == 0.0) {
@@ -395,43 +450,94 @@ __global__ void givens(int count, int j, const int32_t *__restrict__ act,
     }
     csc[j] = cj;
     snc[j] = sj;
-    double2 *gc = g + (int64_t)c * gstride;
-    zrot_(gc[j], gc[j + 1], cj, sj);
-    zrot_(h[j], h[j + 1], cj, sj);
+    zrot_(g0, g1, cj, sj);
+    gc[j] = g0;
+    gc[j + 1] = g1;
+    zrot_(ca, cb, cj, sj);
+    h[j] = ca;
     h[j + 1] = make_double2(0.0, 0.0);
-    resid[k] = cabs_(gc[j + 1]);
+    resid[k] = cabs_(g1);
 }
 
-// y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'): one
-// warp per triggered column, column-oriented back substitution with the
-// updates of y spread over the lanes; y stored compactly [k][j+1].
-__global__ void tri_solve(int count, int j, const int32_t *__restrict__ act,
-                          double2 *const *__restrict__ Hcols, int hstride,
-                          const double2 *__restrict__ g, int gstride, double2 *__restrict__ y) {
+// y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
+// per triggered column, y stored compactly [k][j+1].  Back substitution in
+// blocks of 32 columns: the 32 x 32 triangle is staged in shared memory and
+// solved by one warp in registers, then the whole block subtracts the 32
+// solved unknowns from the rows above (each row in descending column order,
+// as the unblocked substitution does) while it stages the next triangle.  One
+// warp reading the columns of R from global memory, one dependent load per
+// unknown, took 326 us at 61-130 unknowns and 1,125 us at 700; now 100 and
+// 333 us (latency bound: ~32 dependent multiplications a block).
+constexpr int kTriB = 32;
+
+__global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t *__restrict__ act,
+                                                 double2 *const *__restrict__ Hcols, int hstride,
+                                                 const double2 *__restrict__ g, int gstride,
+                                                 double2 *__restrict__ y) {
     extern __shared__ double2 ys[];
-    int k = blockIdx.x;
+    __shared__ double2 tri[kTriB][kTriB + 1];        // tri[column][row]
+    const int k = blockIdx.x;
     if (k >= count) return;
-    int c = act[k];
-    int m = j + 1;
-    for (int i = threadIdx.x; i < m; i += 32) ys[i] = g[(int64_t)c * gstride + i];
-    __syncwarp();
-    for (int i = m - 1; i >= 0; --i) {
-        const double2 *col = Hcols[i] + (int64_t)c * hstride;
-        double2 rii = col[i];
-        double d = rii.x * rii.x + rii.y * rii.y;
-        double2 v = ys[i];
-        double2 yi = make_double2((v.x * rii.x + v.y * rii.y) / d, (v.y * rii.x - v.x * rii.y) / d);
-        __syncwarp();
-        if (threadIdx.x == 0) ys[i] = yi;
-        for (int l = threadIdx.x; l < i; l += 32) {
-            double2 p = cmul(col[l], yi);
-            ys[l].x -= p.x;
-            ys[l].y -= p.y;
+    const int c = act[k];
+    const int m = j + 1;
+    const int64_t off = (int64_t)c * hstride;
+    auto stage = [&](int b0) {                       // triangle of columns and rows b0 .. b0 + 31
+        for (int e = threadIdx.x; e < kTriB * kTriB; e += blockDim.x) {
+            const int col = e / kTriB, row = e % kTriB;
+            tri[col][row] = (b0 + col < m && row <= col) ? Hcols[b0 + col][off + b0 + row] : make_double2(0.0, 0.0);
         }
-        __syncwarp();
+    };
+    for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = g[(int64_t)c * gstride + i];
+    int b0 = (m - 1) / kTriB * kTriB;
+    stage(b0);
+    __syncthreads();
+    for (; b0 >= 0; b0 -= kTriB) {
+        const int nb = min(kTriB, m - b0);
+        if (threadIdx.x < 32) {
+            const int l = threadIdx.x;
+            double2 v = l < nb ? ys[b0 + l] : make_double2(0.0, 0.0);
+            const double2 r = l < nb ? tri[l][l] : make_double2(1.0, 0.0);
+            const double d = r.x * r.x + r.y * r.y;
+            const double2 ri = make_double2(r.x / d, -r.y / d);
+            for (int i = nb - 1; i >= 0; --i) {
+                const double2 yi = shfl2(cmul(v, ri), i);
+                if (l == i) v = yi;
+                if (l < i) {
+                    const double2 p = cmul(tri[i][l], yi);
+                    v.x -= p.x;
+                    v.y -= p.y;
+                }
+            }
+            if (l < nb) ys[b0 + l] = v;
+        }
+        __syncthreads();
+        if (b0 > 0) {
+            for (int l = threadIdx.x; l < b0; l += blockDim.x) {
+                double2 v = ys[l];
+                for (int i0 = nb; i0 > 0; i0 -= 8) {
+                    double2 r[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        r[q] = i0 - 1 - q >= 0 ? Hcols[b0 + i0 - 1 - q][off + l] : make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (i0 - 1 - q >= 0) {
+                            const double2 p = cmul(r[q], ys[b0 + i0 - 1 - q]);
+                            v.x -= p.x;
+                            v.y -= p.y;
+                        }
+                }
+                ys[l] = v;
+            }
+            stage(b0 - kTriB);
+            __syncthreads();
+        }
     }
-    for (int i = threadIdx.x; i < m; i += 32) y[(int64_t)k * m + i] = ys[i];
+    for (int i = threadIdx.x; i < m; i += blockDim.x) y[(int64_t)k * m + i] = ys[i];
 }
+
+// a thread per row above the last triangle, at most a block's worth
+int tri_threads(int m) { return std::min(256, std::max(64, (m + 31) / 32 * 32)); }
 
 // R[k] = B[c] - AX[k] with c = act[k]; in place into AX.
 __global__ void residual(int n, const int32_t *__restrict__ act, const double *__restrict__ B,
@@ -637,7 +743,7 @@ class GmresRun final : public GmresStepper {
         prof_begin(ctx_);
         normalize<VT><<<dim3(grid_rows(2LL * n), na), 256, 0, st_>>>(n, d_act_.p, nrm_.p, Wa_.p, slabs_[j + 1].p,
                                                                     hcols_[j].p, hstride_, j + 1);
-        givens<<<n_blocks(na, 128), 128, 0, st_>>>(na, j, d_act_.p, d_hcols_.p, hstride_, cs_.p, sn_.p, gv_.p,
+        givens<<<n_blocks(na, kGivensWarps), 32 * kGivensWarps, 0, st_>>>(na, j, d_act_.p, d_hcols_.p, hstride_, cs_.p, sn_.p, gv_.p,
                                                   hstride_, m_, nrm_.p);
         ctx_->launches += 2;
         prof_end(ctx_, PROF_LSQ, 0.0, 0.0);
@@ -661,7 +767,7 @@ class GmresRun final : public GmresStepper {
             // inner solve of a refinement: take the least-squares solution as is
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            tri_solve<<<nt, 32, (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
+            tri_solve<<<nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
                                                                   hstride_, ybuf_.p);
             ctx_->launches += 1 + combine_chunked(st_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
             if (jac_) {
@@ -676,7 +782,7 @@ class GmresRun final : public GmresStepper {
         } else if (!trig.empty()) {
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            tri_solve<<<nt, 32, (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
+            tri_solve<<<nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
                                                                   hstride_, ybuf_.p);
             ctx_->launches += combine_chunked(st_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
             gather_x<<<dim3(grid_rows(2LL * n), nt), 256, 0, st_>>>(n, d_cols_.p, d_X_, Xa_.p);
