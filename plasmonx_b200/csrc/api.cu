@@ -242,6 +242,7 @@ plx_status plx_geometry_create(plx_ctx *ctx, const plx_geometry_desc *d, int32_t
         PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_par.p, par.data(), par.size() * 8, cudaMemcpyHostToDevice, st));
         PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_type.p, g->atom_type.data(), N * 4, cudaMemcpyHostToDevice, st));
         PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_frac.p, g->frac.data(), g->frac.size() * 8, cudaMemcpyHostToDevice, st));
+        upload_pair_widths(g);
         build_conductance(g);
         if (store_t) build_dense_t(g);
     });

@@ -176,6 +176,30 @@ void build_dense_t(plx_geom *g) {
     g->has_T = true;
 }
 
+// The pair table of pair_tiles.cuh from the widths of the atom types.
+void upload_pair_widths(plx_geom *g) {
+    const int nt = g->n_types;
+    const bool fmu = g->model == PLX_WFQFMU;
+    std::vector<PairWidths> w((size_t)nt * nt);
+    for (int a = 0; a < nt; ++a)
+        for (int b = 0; b < nt; ++b) {
+            const double qi = g->r_q[a], qj = g->r_q[b], mi = g->r_mu[a], mj = g->r_mu[b];
+            const double qq = std::sqrt(qi * qi + qj * qj), qm = std::sqrt(qi * qi + mj * mj),
+                         mq = std::sqrt(qj * qj + mi * mi), mm = std::sqrt(mi * mi + mj * mj);
+            const double top = fmu ? std::max(std::max(qq, qm), std::max(mq, mm)) : qq;
+            // a zero or non-finite width has no distance beyond which it is undamped: its tile
+            // is evaluated (and is not a number where the formulas are not)
+            const bool ok = std::isfinite(top) && (!fmu || (qq > 0.0 && qm > 0.0 && mq > 0.0 && mm > 0.0));
+            const double far = PLX_FAR_WIDTHS * top;
+            w[a + (size_t)nt * b] = {1.0 / qq, 1.0 / qm, 1.0 / mq, 1.0 / mm, 4.0 / (PLX_SQRT_PI * mm * mm * mm),
+                                     ok ? far * far : INFINITY};
+        }
+    g->d_widths.alloc(g->ctx, w.size());
+    PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_widths.p, w.data(), w.size() * sizeof(PairWidths), cudaMemcpyHostToDevice,
+                                   g->ctx->stream));
+    PLX_CHECK_CUDA(cudaStreamSynchronize(g->ctx->stream));
+}
+
 // Per-frequency tables.  Charge diagonal -z(w) with
 // z = w (-w tau - i) / (2 n tau) (new_gmres_diagonal_shift_wfq,
 // wfq_module.f90:398-424); dipole diagonal sum_t f_t,i / alpha_t(w)

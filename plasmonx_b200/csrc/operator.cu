@@ -108,168 +108,232 @@ __global__ void __launch_bounds__(kTiledThreads) tiled_partial(int R, int n, int
 }
 
 // ---------------------------------------------------------------------------
-// S^T = X^T T with T generated in place (matrix-free, R > 16): the tiled
-// product above with its T slab computed from the pair formulas
-// (plx_t_element) instead of loaded, so every element of T is evaluated once
-// per 64-column row tile of X^T and a batch of many columns costs about one
-// dense FP64 product.  Same K chunks and per-element FMA order as the stored
-// kernels.
+// S = T X generated on the fly (matrix-free), at most CB columns per launch:
+// one or several warps per target atom, the lanes over the source atoms.
+//
+// FP64 bound: a near pair costs three erf and two exp (alloy pairs four and
+// three), a distant one about 40 operations, each column 32 FMAs.  One thread
+// per target atom walking every source (the first form of this kernel) ran 16
+// CTAs for 1,961 atoms: 3,383 us for one column; with the sources spread over the
+// lanes, the width table and the undamped distant tile 96 us.  700 atoms, 4
+// columns: 1,213 -> 34.5 us.
+//
+// Each lane adds its sources in ascending order with explicit FMAs, the lanes are
+// added by a fixed exchange tree and the warps of a target in order; the number
+// of warps depends on the number of atoms alone, so a column's sums depend
+// neither on the batch nor on CB.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n, int kchunk, int N, int fmu,
+constexpr int kOtfWarps = 8;
+constexpr int kOtfFewCols = 4;              // columns up to which it is used; the tiled form above
+
+// Warps per target atom: enough of them for ~24 warps on every SM.
+int otf_warps(int N) {
+    int w = 1;
+    while (w < kOtfWarps && (int64_t)N * w < 148 * 24) w *= 2;
+    return w;
+}
+
+// Adds v[0..V) over the lanes: every lane ends with the sums of the values whose
+// index bits it owns, V / 32 of them (at least one); returns the first one's index.
+template <int V>
+__device__ __forceinline__ int lane_sums(double (&v)[V], int lane) {
+    int base = 0;
+    int len = V;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (len > 1) {
+            const bool up = lane & o;
+            len >>= 1;
+#pragma unroll
+            for (int k = 0; k < V / 2; ++k)
+                if (k < len) {
+                    const double send = up ? v[k] : v[k + len], keep = up ? v[k + len] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            if (up) base += len;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return base;
+}
+
+template <int CB, bool FMU>
+__global__ void __launch_bounds__(32 * kOtfWarps) otf_contract(int N, int wt, int count, int nv, int nt,
+                                                               const double *__restrict__ pos,
+                                                               const double *__restrict__ par,
+                                                               const int32_t *__restrict__ type,
+                                                               const PairWidths *__restrict__ widths,
+                                                               const double *__restrict__ X, double *__restrict__ S) {
+    constexpr int NC = FMU ? 4 : 1;            // components per atom
+    constexpr int V = NC * 2 * CB;             // values per target: [component][part][column]
+    __shared__ double red[kOtfWarps][V];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * (kOtfWarps / wt) + warp / wt, part = warp % wt;
+    double acc[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc[k] = 0.0;
+    if (i < N) {
+        const double xi = pos[i], yi = pos[N + i], zi = pos[2 * N + i];
+        const int ti = type[i];
+        for (int j = part * 32 + lane; j < N; j += 32 * wt) {
+            double xq[2 * CB];
+#pragma unroll
+            for (int k = 0; k < 2 * CB; ++k) xq[k] = (k >> 1) < count ? X[(int64_t)k * nv + j] : 0.0;
+            if (j == i) {
+                const double eta = par[2 * N + i];
+#pragma unroll
+                for (int k = 0; k < 2 * CB; ++k) acc[k] = fma(eta, xq[k], acc[k]);
+                continue;
+            }
+            const double dx = xi - pos[j], dy = yi - pos[N + j], dz = zi - pos[2 * N + j];
+            const int tj = type[j];
+            if (!FMU) {
+                const double q = plx_pair_qq_w(dx, dy, dz, widths[ti + nt * tj]);
+#pragma unroll
+                for (int k = 0; k < 2 * CB; ++k) acc[k] = fma(q, xq[k], acc[k]);
+                continue;
+            }
+            PairTile tl;
+            plx_pair_tile_w(dx, dy, dz, widths[ti + nt * tj], ti == tj, tl);
+#pragma unroll
+            for (int k = 0; k < 2 * CB; ++k) {
+                const double *xm = X + (int64_t)k * nv + N + 3LL * j;
+                const bool in = (k >> 1) < count;
+                const double m0 = in ? xm[0] : 0.0, m1 = in ? xm[1] : 0.0, m2 = in ? xm[2] : 0.0;
+                acc[k] = fma(tl.qm[2], m2, fma(tl.qm[1], m1, fma(tl.qm[0], m0, fma(tl.qq, xq[k], acc[k]))));
+                constexpr int P = 2 * CB;
+                if (NC > 1) {
+                    acc[P % V + k] = fma(tl.mm[2], m2, fma(tl.mm[1], m1, fma(tl.mm[0], m0,
+                                         fma(tl.mq[0], xq[k], acc[P % V + k]))));
+                    acc[2 * P % V + k] = fma(tl.mm[4], m2, fma(tl.mm[3], m1, fma(tl.mm[1], m0,
+                                             fma(tl.mq[1], xq[k], acc[2 * P % V + k]))));
+                    acc[3 * P % V + k] = fma(tl.mm[5], m2, fma(tl.mm[4], m1, fma(tl.mm[2], m0,
+                                             fma(tl.mq[2], xq[k], acc[3 * P % V + k]))));
+                }
+            }
+        }
+    }
+    const int base = lane_sums<V>(acc, lane);
+    constexpr int L = V > 32 ? V / 32 : 1;      // sums a lane owns
+    constexpr int G = V < 32 ? 32 / V : 1;      // lanes that own the same sum
+    if (lane % G == 0) {
+#pragma unroll
+        for (int k = 0; k < L; ++k) red[warp][base + k] = acc[k];
+    }
+    __syncthreads();
+    if (i >= N || part != 0) return;
+    for (int e = lane; e < V; e += 32) {
+        double s = red[warp][e];
+        for (int w = 1; w < wt; ++w) s += red[warp + w][e];
+        const int comp = e / (2 * CB), k = e % (2 * CB);
+        if ((k >> 1) < count) S[(int64_t)k * nv + (comp == 0 ? i : N + 3 * i + comp - 1)] = s;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same for many columns: the tiled product above with its T slab generated
+// in shared memory, split over source atoms and reduced by skinny_reduce.  Rows
+// and columns run atom by atom (an atom's charge, then its three dipole
+// components), so a thread evaluates one pair of atoms and writes its 4 x 4
+// block: the slab's erf and exp are evaluated once per pair instead of once per
+// element.  BM rows of X^T a block (16, 32, 48 or 64): the fewest that hold the
+// batch, so that 42 rows do not run as 64.  Every output is one FMA chain over
+// the unknowns of a chunk in order, whatever BM.
+// Measured at 13,528 unknowns and 42 rows: 5,085 us element by element in 64
+// rows, now 1,429 us (average of four launches).
+// ---------------------------------------------------------------------------
+template <int BM, bool FMU>
+__global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n, int jchunk, int N, int nt,
                                                                    const double *__restrict__ pos,
                                                                    const double *__restrict__ par,
+                                                                   const int32_t *__restrict__ type,
+                                                                   const PairWidths *__restrict__ widths,
                                                                    const double *__restrict__ Xt,
                                                                    double *__restrict__ part) {
-    __shared__ double As[BM][BK + 1];
-    __shared__ double Bs[BK][BN];
+    constexpr int NC = FMU ? 4 : 1;
+    constexpr int KA = 16 / NC;                // source atoms a slab (16 unknowns)
+    constexpr int CA = BN / NC;                // target atoms a block
+    constexpr int RM = BM / 8;                 // rows a thread
+    __shared__ double As[BM][16 + 1];
+    __shared__ double Bs[16][BN];
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-    const int kbeg = blockIdx.z * kchunk, kend = min(n, kbeg + kchunk);
-    double acc[8][8];
+    const int row0 = blockIdx.y * BM, i0 = blockIdx.x * CA;
+    const int jbeg = blockIdx.z * jchunk, jend = min(N, jbeg + jchunk);
+    double acc[RM][8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+    for (int u = 0; u < RM; ++u)
 #pragma unroll
         for (int v = 0; v < 8; ++v) acc[u][v] = 0.0;
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
+    for (int j0 = jbeg; j0 < jend; j0 += KA) {
         __syncthreads();
-        for (int e = threadIdx.x; e < BM * BK; e += kTiledThreads) {
-            const int r = e / BK, k = e % BK, gr = row0 + r, gk = k0 + k;
-            As[r][k] = (gr < R && gk < kend) ? Xt[(int64_t)gr * n + gk] : 0.0;
+        for (int e = threadIdx.x; e < BM * 16; e += kTiledThreads) {
+            const int r = e / 16, k = e % 16, gr = row0 + r, j = j0 + k / NC, comp = k % NC;
+            As[r][k] = (gr < R && j < jend) ? Xt[(int64_t)gr * n + (comp == 0 ? j : N + 3 * j + comp - 1)] : 0.0;
         }
 #pragma unroll 1
-        for (int e = threadIdx.x; e < BK * BN; e += kTiledThreads) {
-            const int k = e / BN, c = e % BN, gk = k0 + k, gc = col0 + c;
-            Bs[k][c] = (gk < kend && gc < n) ? plx_t_element(N, fmu != 0, pos, par, gk, gc) : 0.0;
+        for (int e = threadIdx.x; e < KA * CA; e += kTiledThreads) {
+            const int jl = e / CA, il = e % CA, i = i0 + il, j = j0 + jl;
+            if (!FMU) {
+                double q = 0.0;
+                if (i < N && j < jend)
+                    q = i == j ? par[2 * N + i]
+                               : plx_pair_qq_w(pos[i] - pos[j], pos[N + i] - pos[N + j], pos[2 * N + i] - pos[2 * N + j],
+                                               widths[type[i] + nt * type[j]]);
+                Bs[jl][il] = q;
+                continue;
+            }
+            PairTile t;
+            t.qq = 0.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) t.qm[k] = t.mq[k] = 0.0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) t.mm[k] = 0.0;
+            if (i < N && j < jend) {
+                if (i == j) {
+                    t.qq = par[2 * N + i];
+                } else {
+                    const int ti = type[i], tj = type[j];
+                    plx_pair_tile_w(pos[i] - pos[j], pos[N + i] - pos[N + j], pos[2 * N + i] - pos[2 * N + j],
+                                    widths[ti + nt * tj], ti == tj, t);
+                }
+            }
+            // element [source component][target component]
+            double2 *b = reinterpret_cast<double2 *>(&Bs[(NC * jl) % 16][(NC * il) % BN]);
+            constexpr int ld = BN / 2;
+            b[0] = make_double2(t.qq, t.mq[0]);
+            b[1] = make_double2(t.mq[1], t.mq[2]);
+            b[ld] = make_double2(t.qm[0], t.mm[0]);
+            b[ld + 1] = make_double2(t.mm[1], t.mm[2]);
+            b[2 * ld] = make_double2(t.qm[1], t.mm[1]);
+            b[2 * ld + 1] = make_double2(t.mm[3], t.mm[4]);
+            b[3 * ld] = make_double2(t.qm[2], t.mm[2]);
+            b[3 * ld + 1] = make_double2(t.mm[4], t.mm[5]);
         }
         __syncthreads();
-        const int kn = min(BK, kend - k0);
+        const int kn = min(16, NC * (jend - j0));
+#pragma unroll 4
         for (int k = 0; k < kn; ++k) {
-            double a[8], b[8];
+            double a[RM], b[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = As[ty * 8 + u][k];
+            for (int u = 0; u < RM; ++u) a[u] = As[ty * RM + u][k];
 #pragma unroll
             for (int v = 0; v < 8; ++v) b[v] = Bs[k][tx + 16 * v];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < RM; ++u)
 #pragma unroll
                 for (int v = 0; v < 8; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
         }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int gr = row0 + ty * 8 + u;
+    for (int u = 0; u < RM; ++u) {
+        const int gr = row0 + ty * RM + u;
         if (gr >= R) continue;
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
-            const int gc = col0 + tx + 16 * v;
-            if (gc < n) part[((int64_t)blockIdx.z * R + gr) * n + gc] = acc[u][v];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// S = T X generated on the fly (matrix-free), CB columns per launch.
-// One thread per target atom; source atoms staged in shared memory.
-// ---------------------------------------------------------------------------
-constexpr int kOtfThreads = 128;
-
-template <int CB, bool FMU>
-__global__ void __launch_bounds__(kOtfThreads) otf_contract(int N, int count, int nv,
-                                                            const double *__restrict__ pos,
-                                                            const double *__restrict__ par,
-                                                            const double *__restrict__ X,
-                                                            double *__restrict__ S) {
-    constexpr int NC = FMU ? 4 : 1;            // components per atom
-    __shared__ double sp[kOtfThreads][5];       // x, y, z, r_q, r_mu
-    __shared__ double sxv[kOtfThreads][NC * 2 * CB];
-    int i = blockIdx.x * kOtfThreads + threadIdx.x;
-    bool live = i < N;
-    double xi = 0, yi = 0, zi = 0, rqi = 1, rmi = 1, etai = 0;
-    if (live) {
-        xi = pos[i];
-        yi = pos[N + i];
-        zi = pos[2 * N + i];
-        rqi = par[i];
-        rmi = par[N + i];
-        etai = par[2 * N + i];
-    }
-    double acc[NC][2][CB];
-#pragma unroll
-    for (int a = 0; a < NC; ++a)
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int c = 0; c < CB; ++c) acc[a][p][c] = 0.0;
-    for (int j0 = 0; j0 < N; j0 += kOtfThreads) {
-        int j = j0 + threadIdx.x;
-        __syncthreads();
-        if (j < N) {
-            sp[threadIdx.x][0] = pos[j];
-            sp[threadIdx.x][1] = pos[N + j];
-            sp[threadIdx.x][2] = pos[2 * N + j];
-            sp[threadIdx.x][3] = par[j];
-            sp[threadIdx.x][4] = par[N + j];
-#pragma unroll
-            for (int c = 0; c < CB; ++c) {
-                const double *xc = X + (int64_t)c * 2 * nv;
-                for (int p = 0; p < 2; ++p) {
-                    sxv[threadIdx.x][(0 * 2 + p) * CB + c] = (c < count) ? xc[p * nv + j] : 0.0;
-                    if (FMU)
-                        for (int k = 0; k < 3; ++k)
-                            sxv[threadIdx.x][((1 + k) * 2 + p) * CB + c] =
-                                (c < count) ? xc[p * nv + N + 3 * j + k] : 0.0;
-                }
-            }
-        }
-        __syncthreads();
-        if (!live) continue;
-        int jn = min(kOtfThreads, N - j0);
-        for (int t = 0; t < jn; ++t) {
-            int jj = j0 + t;
-            const double *xv = sxv[t];
-            if (jj == i) {
-#pragma unroll
-                for (int p = 0; p < 2; ++p)
-#pragma unroll
-                    for (int c = 0; c < CB; ++c) acc[0][p][c] = fma(etai, xv[p * CB + c], acc[0][p][c]);
-                continue;
-            }
-            double dx = xi - sp[t][0], dy = yi - sp[t][1], dz = zi - sp[t][2];
-            if (!FMU) {
-                double q = plx_pair_qq(dx, dy, dz, rqi, sp[t][3]);
-#pragma unroll
-                for (int p = 0; p < 2; ++p)
-#pragma unroll
-                    for (int c = 0; c < CB; ++c) acc[0][p][c] = fma(q, xv[p * CB + c], acc[0][p][c]);
-                continue;
-            }
-            PairTile tl;
-            plx_pair_tile(dx, dy, dz, rqi, rmi, sp[t][3], sp[t][4], tl);
-#pragma unroll
-            for (int p = 0; p < 2; ++p)
-#pragma unroll
-                for (int c = 0; c < CB; ++c) {
-                    double xq = xv[(0 * 2 + p) * CB + c];
-                    double m0 = xv[(1 * 2 + p) * CB + c];
-                    double m1 = xv[(2 * 2 + p) * CB + c];
-                    double m2 = xv[(3 * 2 + p) * CB + c];
-                    acc[0][p][c] += tl.qq * xq + tl.qm[0] * m0 + tl.qm[1] * m1 + tl.qm[2] * m2;
-                    acc[1][p][c] += tl.mq[0] * xq + tl.mm[0] * m0 + tl.mm[1] * m1 + tl.mm[2] * m2;
-                    acc[2][p][c] += tl.mq[1] * xq + tl.mm[1] * m0 + tl.mm[3] * m1 + tl.mm[4] * m2;
-                    acc[3][p][c] += tl.mq[2] * xq + tl.mm[2] * m0 + tl.mm[4] * m1 + tl.mm[5] * m2;
-                }
-        }
-    }
-    if (!live) return;
-#pragma unroll
-    for (int c = 0; c < CB; ++c) {
-        if (c >= count) break;
-        double *sc = S + (int64_t)c * 2 * nv;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            sc[p * nv + i] = acc[0][p][c];
-            if (FMU)
-                for (int k = 0; k < 3; ++k) sc[p * nv + N + 3 * i + k] = acc[1 + k][p][c];
+            const int c = tx + 16 * v, i = i0 + c / NC, comp = c % NC;
+            if (i < N)
+                part[((int64_t)blockIdx.z * R + gr) * n + (comp == 0 ? i : N + 3 * i + comp - 1)] = acc[u][v];
         }
     }
 }
@@ -636,35 +700,56 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
     cudaStream_t st = ctx->stream;
     const int n = g->n_var;
     const int R = 2 * count;
-    if (on_the_fly && R > 16) {
-        // many columns: tiled product with T generated per slab
-        int ks, kchunk;
-        skinny_split(n, ks, kchunk);
-        size_t need = (size_t)ks * R * n;
-        if (g->d_part.n < need) g->d_part.alloc(ctx, need);
-        dim3 grid(n_blocks(n, BN), n_blocks(R, BM), ks);
-        otf_tiled_partial<<<grid, kTiledThreads, 0, st>>>(R, n, kchunk, g->n_atoms, g->model == PLX_WFQFMU,
-                                                          g->d_pos.p, g->d_par.p, X, g->d_part.p);
-        skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, ks, g->d_part.p, S);
-        ctx->launches += 2;
-        PLX_CHECK_CUDA(cudaGetLastError());
-        return;
-    }
     if (on_the_fly) {
         const bool fmu = g->model == PLX_WFQFMU;
-        for (int c0 = 0; c0 < count; c0 += 4) {
-            int cb = std::min(4, count - c0);
-            const double *Xc = X + (int64_t)c0 * 2 * n;
-            double *Sc = S + (int64_t)c0 * 2 * n;
-            int blocks = n_blocks(g->n_atoms, kOtfThreads);
-            if (fmu)
-                otf_contract<4, true><<<blocks, kOtfThreads, 0, st>>>(g->n_atoms, cb, n, g->d_pos.p,
-                                                                     g->d_par.p, Xc, Sc);
-            else
-                otf_contract<4, false><<<blocks, kOtfThreads, 0, st>>>(g->n_atoms, cb, n, g->d_pos.p,
-                                                                      g->d_par.p, Xc, Sc);
-            ctx->launches++;
+        const int N = g->n_atoms;
+        if (count > kOtfFewCols) {
+            // many columns: tiled product with T generated per slab; the split over the
+            // sources depends on the number of atoms only
+            const int ca = fmu ? BN / 4 : BN, ka = fmu ? 4 : 16;
+            const int tiles = n_blocks(N, ca);
+            int js = std::max(1, std::min(64, (592 + tiles - 1) / tiles));
+            const int jchunk = n_blocks(n_blocks(N, js), ka) * ka;
+            js = n_blocks(N, jchunk);
+            const size_t need = (size_t)js * R * n;
+            if (g->d_part.n < need) g->d_part.alloc(ctx, need);
+            const int bm = R <= 16 ? 16 : R <= 32 ? 32 : (R <= 48 ? 48 : 64);
+            const dim3 grid(tiles, n_blocks(R, bm), js);
+#define PLX_OTF(BMV, F)                                                                                             \
+    otf_tiled_partial<BMV, F><<<grid, kTiledThreads, 0, st>>>(R, n, jchunk, N, g->n_types, g->d_pos.p, g->d_par.p, \
+                                                              g->d_type.p, g->d_widths.p, X, g->d_part.p)
+            if (fmu) {
+                if (bm == 16) PLX_OTF(16, true);
+                else if (bm == 32) PLX_OTF(32, true);
+                else if (bm == 48) PLX_OTF(48, true);
+                else PLX_OTF(64, true);
+            } else {
+                if (bm == 16) PLX_OTF(16, false);
+                else if (bm == 32) PLX_OTF(32, false);
+                else if (bm == 48) PLX_OTF(48, false);
+                else PLX_OTF(64, false);
+            }
+#undef PLX_OTF
+            skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, js, g->d_part.p, S);
+            ctx->launches += 2;
+            PLX_CHECK_CUDA(cudaGetLastError());
+            return;
         }
+        const int wt = otf_warps(N), blocks = n_blocks(N, kOtfWarps / wt);
+#define PLX_OTF(CB, F)                                                                                            \
+    otf_contract<CB, F><<<blocks, 32 * kOtfWarps, 0, st>>>(N, wt, count, n, g->n_types, g->d_pos.p, g->d_par.p, \
+                                                           g->d_type.p, g->d_widths.p, X, S)
+        if (fmu) {
+            if (count == 1) PLX_OTF(1, true);
+            else if (count == 2) PLX_OTF(2, true);
+            else PLX_OTF(4, true);
+        } else {
+            if (count == 1) PLX_OTF(1, false);
+            else if (count == 2) PLX_OTF(2, false);
+            else PLX_OTF(4, false);
+        }
+#undef PLX_OTF
+        ctx->launches++;
         PLX_CHECK_CUDA(cudaGetLastError());
         return;
     }

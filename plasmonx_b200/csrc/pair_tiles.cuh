@@ -14,6 +14,8 @@
 // T_qq and zero for the dipole blocks of the w-models.
 #pragma once
 
+#include "plx_internal.h"
+
 #define PLX_SQRT_PI 1.7724538509055160273
 
 struct PairTile {
@@ -63,6 +65,58 @@ __device__ __forceinline__ void plx_pair_tile(double dx, double dy, double dz, d
     t.mm[3] = a * dy * dy + dd;
     t.mm[4] = a * dy * dz;
     t.mm[5] = a * dz * dz + dd;
+}
+
+// For u = r/R >= 7, erfc(u) < 5e-23, the exponential part of f(r, R) is below
+// 5e-21 and fD2 r below 5e-19 of fD1 / r^2: all under half an ulp (5.5e-17) of
+// the terms they are added to, so the tile is the undamped one.
+#define PLX_FAR_WIDTHS 7.0
+
+// The tile of plx_pair_tile from the pair table, with the undamped tile for
+// distant pairs (about half the pairs of a 40 Angstrom particle, most of a
+// larger one) and f(r, R_mq) = f(r, R_qm) for two atoms of one type.
+__device__ __forceinline__ void plx_pair_tile_w(double dx, double dy, double dz, const PairWidths &w, bool same,
+                                                PairTile &t) {
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double ir = rsqrt(r2);
+    const double ir2 = ir * ir, ir3 = ir2 * ir;
+    double f1 = ir3, f2 = ir3, dd = ir3, a = -3.0 * (ir3 * ir2);
+    t.qq = ir;
+    if (!(r2 > w.far2)) {
+        const double r = r2 * ir;
+        t.qq = erf(r * w.iqq) * ir;
+        const double u1 = r * w.iqm;
+        f1 = (erf(u1) - (2.0 / PLX_SQRT_PI) * u1 * exp(-(u1 * u1))) * ir3;
+        f2 = f1;
+        if (!same) {
+            const double u2 = r * w.imq;
+            f2 = (erf(u2) - (2.0 / PLX_SQRT_PI) * u2 * exp(-(u2 * u2))) * ir3;
+        }
+        const double um = r * w.imm, em = exp(-(um * um));
+        const double fD1 = erf(um) - (2.0 / PLX_SQRT_PI) * um * em;
+        dd = ir3 * fD1;
+        a = fma(a, fD1, w.c2 * em * ir2);
+    }
+    t.qm[0] = dx * f1;
+    t.qm[1] = dy * f1;
+    t.qm[2] = dz * f1;
+    t.mq[0] = -dx * f2;
+    t.mq[1] = -dy * f2;
+    t.mq[2] = -dz * f2;
+    const double ax = a * dx, ay = a * dy, az = a * dz;
+    t.mm[0] = fma(ax, dx, dd);
+    t.mm[1] = ax * dy;
+    t.mm[2] = ax * dz;
+    t.mm[3] = fma(ay, dy, dd);
+    t.mm[4] = ay * dz;
+    t.mm[5] = fma(az, dz, dd);
+}
+
+// Charge-charge element only (wFQ), from the pair table.
+__device__ __forceinline__ double plx_pair_qq_w(double dx, double dy, double dz, const PairWidths &w) {
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double ir = rsqrt(r2);
+    return r2 > w.far2 ? ir : erf(r2 * ir * w.iqq) * ir;
 }
 
 // Charge-charge element only (wFQ).

@@ -77,6 +77,16 @@ struct DevArray {
 
 }  // namespace plx
 
+// Constants of an ordered atom-type pair (type of i, type of j), the table
+// [ti + n_types * tj] that geometries upload once: reciprocals of the damping
+// widths, 4 / (sqrt(pi) R_mm^3) and the squared distance beyond which every
+// damping factor of the pair is one in double precision.
+struct PairWidths {
+    double iqq, iqm, imq, imm;   // 1/R_qq, 1/R_qm (rq_i, rmu_j), 1/R_mq (rmu_i, rq_j), 1/R_mm
+    double c2;                   // 4 / (sqrt(pi) R_mm^3)
+    double far2;
+};
+
 struct plx_ctx {
     int device = 0;
     uint64_t budget = 0;
@@ -116,6 +126,7 @@ struct plx_geom {
     plx::DevArray<int32_t> d_type;      // N
     plx::DevArray<double> d_par;        // [4][N]: r_q, r_mu, eta, a_ij of the atom's type
     plx::DevArray<double> d_frac;       // n_types x N
+    plx::DevArray<PairWidths> d_widths; // n_types x n_types: damping widths of a type pair
     // device: conductance K in CSR (off-diagonal entries with K_ij or K_ji != 0)
     plx::DevArray<int32_t> d_rowptr;    // N + 1
     plx::DevArray<int32_t> d_col;       // nnz
@@ -205,6 +216,7 @@ inline bool is_bem(const plx_geom *g) { return g->model == PLX_BEM_DPCM || g->mo
 // geometry.cu
 void build_conductance(plx_geom *g);
 void build_dense_t(plx_geom *g);
+void upload_pair_widths(plx_geom *g);
 void upload_frequency_tables(plx_geom *g);
 
 // operator.cu
