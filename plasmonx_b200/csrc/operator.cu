@@ -11,6 +11,7 @@
 #include "pair_tiles.cuh"
 #include "plx_internal.h"
 #include "skinny.cuh"
+#include "warp_sums.cuh"
 
 namespace plx {
 
@@ -131,31 +132,6 @@ int otf_warps(int N) {
     int w = 1;
     while (w < kOtfWarps && (int64_t)N * w < 148 * 24) w *= 2;
     return w;
-}
-
-// Adds v[0..V) over the lanes: every lane ends with the sums of the values whose
-// index bits it owns, V / 32 of them (at least one); returns the first one's index.
-template <int V>
-__device__ __forceinline__ int lane_sums(double (&v)[V], int lane) {
-    int base = 0;
-    int len = V;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        if (len > 1) {
-            const bool up = lane & o;
-            len >>= 1;
-#pragma unroll
-            for (int k = 0; k < V / 2; ++k)
-                if (k < len) {
-                    const double send = up ? v[k] : v[k + len], keep = up ? v[k + len] : v[k];
-                    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                }
-            if (up) base += len;
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-        }
-    }
-    return base;
 }
 
 template <int CB, bool FMU>
@@ -695,6 +671,36 @@ void contract_t(plx_geom *g, int count, const double *X, double *S, Contraction 
              2.0 * nn * nn * 2.0 * count, tbytes + 2.0 * 8.0 * nn * 2.0 * count);
 }
 
+// S = X T for R rows X [R][n] and a row-major n x n FP64 matrix (S^T = T^T X^T):
+// the split-K products above, the partial sums in `scratch` (grown on demand).
+// A row's result does not depend on R within R <= 16 or above it.
+void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const double *X, const double *T, double *S) {
+    // K split: depends on n only (not on the batch), see tiled_partial
+    const int cb = n_blocks(n, kSkinnyCols);
+    int ks, kchunk;
+    skinny_split(n, ks, kchunk);
+    size_t need = (size_t)ks * R * n;
+    if (scratch.n < need) scratch.alloc(ctx, need);
+    double *part = scratch.p;
+    cudaStream_t st = ctx->stream;
+    if (R <= 16) {
+        dim3 grid(cb, ks);
+        switch (R) {
+#define PLX_SK(RR) \
+    case RR: skinny_partial<RR><<<grid, kSkinnyCols, 0, st>>>(n, kchunk, X, T, part); break;
+            PLX_SK(2) PLX_SK(4) PLX_SK(6) PLX_SK(8) PLX_SK(10) PLX_SK(12) PLX_SK(14) PLX_SK(16)
+#undef PLX_SK
+            default: throw Error(PLX_ERR_ARG, "bad skinny row count");
+        }
+    } else {
+        dim3 grid(n_blocks(n, BN), n_blocks(R, BM), ks);
+        tiled_partial<<<grid, kTiledThreads, 0, st>>>(R, n, kchunk, X, T, part);
+    }
+    skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, ks, part, S);
+    ctx->launches += 2;
+    PLX_CHECK_CUDA(cudaGetLastError());
+}
+
 void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on_the_fly) {
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
@@ -754,29 +760,7 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
         return;
     }
     if (!g->has_T) throw Error(PLX_ERR_ARG, "geometry was created without the dense T matrix");
-    // K split: depends on n only (not on the batch), see tiled_partial
-    const int cb = n_blocks(n, kSkinnyCols);
-    int ks, kchunk;
-    skinny_split(n, ks, kchunk);
-    size_t need = (size_t)ks * R * n;
-    if (g->d_part.n < need) g->d_part.alloc(ctx, need);
-    double *part = g->d_part.p;
-    if (R <= 16) {
-        dim3 grid(cb, ks);
-        switch (R) {
-#define PLX_SK(RR) \
-    case RR: skinny_partial<RR><<<grid, kSkinnyCols, 0, st>>>(n, kchunk, X, g->d_T.p, part); break;
-            PLX_SK(2) PLX_SK(4) PLX_SK(6) PLX_SK(8) PLX_SK(10) PLX_SK(12) PLX_SK(14) PLX_SK(16)
-#undef PLX_SK
-            default: throw Error(PLX_ERR_ARG, "bad skinny row count");
-        }
-    } else {
-        dim3 grid(n_blocks(n, BN), n_blocks(R, BM), ks);
-        tiled_partial<<<grid, kTiledThreads, 0, st>>>(R, n, kchunk, X, g->d_T.p, part);
-    }
-    skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, ks, part, S);
-    ctx->launches += 2;
-    PLX_CHECK_CUDA(cudaGetLastError());
+    stored_product(ctx, g->d_part, R, n, X, g->d_T.p, S);
 }
 
 static void finish_rows(plx_geom *g, const OpBatch &b, const double *S, const double *X,
