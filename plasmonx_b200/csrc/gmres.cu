@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <type_traits>
 
 #include "plx_internal.h"
 
@@ -64,16 +65,26 @@ __device__ __forceinline__ void block_sum2(double &a, double &b) {
     }
 }
 
-// Copies column act[k] of slab j into the compact batch X[k].
+// X[k] = P[c] v elementwise for column c = act[k] of slab j (P = 1 when null): the
+// input of a step's product.  Only for the first step and when columns have left
+// the batch; otherwise `normalize_givens` has written it with the basis vector.
 template <typename VT>
 __global__ void gather_cols(int n, const int32_t *__restrict__ act, const VT *__restrict__ slab,
-                            double *__restrict__ X) {
-    int k = blockIdx.y;
-    const VT *src = slab + (int64_t)act[k] * 2 * n;
+                            const double *__restrict__ P, double *__restrict__ X) {
+    const int k = blockIdx.y, c = act[k];
+    const VT *src = slab + (int64_t)c * 2 * n;
+    const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
     double *dst = X + (int64_t)k * 2 * n;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < 2LL * n;
-         r += (int64_t)gridDim.x * blockDim.x)
-        dst[r] = src[r];
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        double re = (double)src[r], im = (double)src[n + r];
+        if (p) {
+            const double pr = p[r], pi = p[n + r], t = pr * re - pi * im;
+            im = pr * im + pi * re;
+            re = t;
+        }
+        dst[r] = re;
+        dst[n + r] = im;
+    }
 }
 
 // Partial complex dots conj(V_i[c]) . W[k] for i in [i0, i1) over one chunk of
@@ -140,7 +151,10 @@ __global__ void __launch_bounds__(kThreads) dots_partial(int n, int i0, int i1,
 // each warp takes whole basis vectors, 32 rows per lane with the loads of 16
 // rows in flight, so one warp reduction serves 1,024 rows of a vector (the
 // kernel above pays one per 128 rows and keeps only 8 loads in flight a warp).
-// Same chunking and partial layout as dots_partial.
+// Same chunking and partial layout as dots_partial.  A batch whose columns times
+// row chunks leave SMs idle spreads the vectors over blockIdx.z (the sums are the
+// same): 893 unknowns, 61 columns 47 -> 17 us a launch, 2,800 unknowns, 4
+// columns (12 CTAs before) 86 -> 7.6 us.
 template <typename VT>
 __global__ void __launch_bounds__(kThreads) dots_wide(int n, int i0, int i1,
                                                       const int32_t *__restrict__ act,
@@ -159,7 +173,7 @@ __global__ void __launch_bounds__(kThreads) dots_wide(int n, int i0, int i1,
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ni = i1 - i0;
-    for (int ii = warp; ii < ni; ii += kThreads / 32) {
+    for (int ii = warp + (kThreads / 32) * blockIdx.z; ii < ni; ii += (kThreads / 32) * gridDim.z) {
         const VT *v = slabs[i0 + ii] + (int64_t)c * 2 * n + r0;
         double re = 0.0, im = 0.0;
         constexpr int kBatch = 16;
@@ -221,78 +235,173 @@ __global__ void dots_finish(int nchunk, int ni, int i0, const int32_t *__restric
 
 // W[k] -= sum_{ii} V_{i0+ii}[c] h[k][ii]   (sign = -1), or X[c] += ... (sign = +1,
 // target indexed by column instead of compact position when by_col != 0).
-// Each thread owns kCombineRows rows (strided by the block); the loads of a
-// batch of basis vectors are issued before their products are summed (the
-// per-row sum runs over ii in ascending order whatever the batching).  Four
-// rows per thread measured the same as one (0.65 s of orthogonalisation per two
-// spectra of the 41,892-unknown sphere either way), so one it is.
-constexpr int kCombineRows = 1;
-template <typename VT>
+//
+// A block owns 256 / G rows of one column; its G groups of threads take every G-th
+// basis vector each (loads of a batch of them in flight together) and the groups'
+// sums are added in order.  G = 4 up to 16,384 unknowns, where one thread per row
+// leaves the chip idle whenever few columns are active (2,800 unknowns, 4 columns:
+// 44 CTAs, 36 us a launch, now 10.3 us; 893 unknowns, 61 columns 27 -> 15 us), and
+// 1 above, where a thread per row suffices.  G depends on n and ni alone, so a
+// column's sums do not depend on its batch.
+//
+// FIN: `h` holds the projections' chunk partials [k][ndot][ni], which every block
+// sums itself (up to four chunks: a launch less); the first block of a column also
+// adds them to H.  npart (optional): the sum of squares of the block's new rows.
+constexpr int kCombineFin = 4;
+template <typename VT, int G, bool FIN>
 __global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int hld, int hoff,
                                                     const int32_t *__restrict__ act,
                                                     VT *const *__restrict__ slabs,
-                                                    const double2 *__restrict__ h, double sign,
-                                                    double *__restrict__ Y, int by_col) {
+                                                    const double2 *__restrict__ h, int ndot, double sign,
+                                                    double *__restrict__ Y, int by_col, double *__restrict__ npart,
+                                                    double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    constexpr int RB = kThreads / G;
     extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
+    __shared__ double2 red[G > 1 ? kThreads : 1];
     const VT **col = reinterpret_cast<const VT **>(sh + ni);
-    int k = blockIdx.y, c = act[k];
+    const int k = blockIdx.y, c = act[k];
     for (int t = threadIdx.x; t < ni; t += blockDim.x) {
-        sh[t] = h[(int64_t)k * hld + hoff + t];
+        double2 v;
+        if (FIN) {
+            v = make_double2(0.0, 0.0);
+            for (int b = 0; b < ndot; ++b) {
+                const double2 p = h[((int64_t)k * ndot + b) * hld + hoff + t];
+                v.x += p.x;
+                v.y += p.y;
+            }
+            if (blockIdx.x == 0) {
+                double2 *dst = Hcol + (int64_t)c * hstride + i0 + t;
+                *dst = accumulate ? make_double2(dst->x + v.x, dst->y + v.y) : v;
+            }
+        } else {
+            v = h[(int64_t)k * hld + hoff + t];
+        }
+        sh[t] = v;
         col[t] = slabs[i0 + t] + (int64_t)c * 2 * n;
     }
     __syncthreads();
-    constexpr int RW = kCombineRows;
-    const int rbase = blockIdx.x * (kThreads * RW) + threadIdx.x;
-    if (rbase >= n) return;
-    int rr[RW];
-    bool in[RW];
-#pragma unroll
-    for (int u = 0; u < RW; ++u) {
-        rr[u] = rbase + kThreads * u;
-        in[u] = rr[u] < n;
-        if (!in[u]) rr[u] = rbase;          // a valid row; its sum is not stored
-    }
-    double ar[RW], ai[RW];
-#pragma unroll
-    for (int u = 0; u < RW; ++u) ar[u] = ai[u] = 0.0;
-    constexpr int kBatch = RW == 1 ? 8 : 4;   // basis vectors whose loads are in flight together
-    int ii = 0;
-    for (; ii + kBatch <= ni; ii += kBatch) {
-        VT vr[kBatch][RW], vi[kBatch][RW];
-#pragma unroll
-        for (int q = 0; q < kBatch; ++q)
-#pragma unroll
-            for (int u = 0; u < RW; ++u) {
-                vr[q][u] = col[ii + q][rr[u]];
-                vi[q][u] = col[ii + q][n + rr[u]];
-            }
+    const int row = threadIdx.x % RB, grp = threadIdx.x / RB;
+    const int r = blockIdx.x * RB + row;
+    const bool in = r < n;
+    const int rr = in ? r : n - 1;                        // a valid row; its sum is not stored
+    double ar = 0.0, ai = 0.0;
+    constexpr int kBatch = 8;                             // basis vectors whose loads are in flight together
+    int ii = grp;
+    for (; ii + (kBatch - 1) * G < ni; ii += kBatch * G) {
+        VT vr[kBatch], vi[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
-            const double2 hh = sh[ii + q];
+            vr[q] = col[ii + q * G][rr];
+            vi[q] = col[ii + q * G][n + rr];
+        }
 #pragma unroll
-            for (int u = 0; u < RW; ++u) {
-                ar[u] += (double)vr[q][u] * hh.x - (double)vi[q][u] * hh.y;
-                ai[u] += (double)vr[q][u] * hh.y + (double)vi[q][u] * hh.x;
+        for (int q = 0; q < kBatch; ++q) {
+            const double2 hh = sh[ii + q * G];
+            ar += (double)vr[q] * hh.x - (double)vi[q] * hh.y;
+            ai += (double)vr[q] * hh.y + (double)vi[q] * hh.x;
+        }
+    }
+    for (; ii < ni; ii += G) {
+        const VT *v = col[ii];
+        const double2 hh = sh[ii];
+        const double vr = (double)v[rr], vi = (double)v[n + rr];
+        ar += vr * hh.x - vi * hh.y;
+        ai += vr * hh.y + vi * hh.x;
+    }
+    if (G > 1) {
+        red[threadIdx.x] = make_double2(ar, ai);
+        __syncthreads();
+        if (grp == 0) {
+#pragma unroll
+            for (int g = 1; g < G; ++g) {
+                ar += red[g * RB + row].x;
+                ai += red[g * RB + row].y;
             }
         }
     }
-    for (; ii < ni; ++ii) {
-        const VT *v = col[ii];
-        const double2 hh = sh[ii];
+    double sq = 0.0;
+    if (in && grp == 0) {
+        double *y = Y + (int64_t)(by_col ? c : k) * 2 * n;
+        const double yr = y[r] + sign * ar, yi = y[n + r] + sign * ai;
+        y[r] = yr;
+        y[n + r] = yi;
+        sq = yr * yr + yi * yi;
+    }
+    if (npart) {                                          // the same for the whole grid
+        double dummy = 0.0;
+        block_sum2(sq, dummy);
+        if (threadIdx.x == 0) npart[(int64_t)k * gridDim.x + blockIdx.x] = sq;
+    }
+}
+
+// Modified Gram-Schmidt of W[k] against V_0..V_j in one launch (n <= 4,096): one
+// block per column keeps its rows of W in registers and walks the basis, the next
+// vector's loads in flight during the block reduction of the current one.  The
+// three short launches per vector it replaces (300 vectors over the first 24
+// steps) took 2.3-2.8 us each plus their gaps; now 12.9 us a step on average at 893 unknowns.
+constexpr int kMgsThreads = 512;
+template <int RPT>
+__global__ void __launch_bounds__(kMgsThreads) mgs_column(int n, int j, const int32_t *__restrict__ act,
+                                                          double *const *__restrict__ slabs, double *__restrict__ W,
+                                                          double2 *__restrict__ Hcol, int hstride,
+                                                          double *__restrict__ npart) {
+    __shared__ double2 red[2][kMgsThreads / 32];
+    const int k = blockIdx.x, c = act[k];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double *w = W + (int64_t)k * 2 * n;
+    double wr[RPT], wi[RPT], vr[RPT], vi[RPT];
+    auto load = [&](const double *src, double *re, double *im) {
 #pragma unroll
-        for (int u = 0; u < RW; ++u) {
-            const double vr = (double)v[rr[u]], vi = (double)v[n + rr[u]];
-            ar[u] += vr * hh.x - vi * hh.y;
-            ai[u] += vr * hh.y + vi * hh.x;
+        for (int q = 0; q < RPT; ++q) {
+            const int r = threadIdx.x + q * kMgsThreads;
+            re[q] = r < n ? src[r] : 0.0;
+            im[q] = r < n ? src[n + r] : 0.0;
+        }
+    };
+    load(w, wr, wi);
+    load(slabs[0] + (int64_t)c * 2 * n, vr, vi);
+    for (int i = 0; i <= j; ++i) {
+        double re = 0.0, im = 0.0;                        // conj(v) . w
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+            re += vr[q] * wr[q] + vi[q] * wi[q];
+            im += vr[q] * wi[q] - vi[q] * wr[q];
+        }
+        double nr[RPT], ni[RPT];
+        if (i < j) load(slabs[i + 1] + (int64_t)c * 2 * n, nr, ni);
+        re = warp_sum(re);
+        im = warp_sum(im);
+        if (lane == 0) red[i & 1][warp] = make_double2(re, im);
+        __syncthreads();
+        double2 h = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int t = 0; t < kMgsThreads / 32; ++t) {
+            h.x += red[i & 1][t].x;
+            h.y += red[i & 1][t].y;
+        }
+        if (threadIdx.x == 0) Hcol[(int64_t)c * hstride + i] = h;
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+            wr[q] -= vr[q] * h.x - vi[q] * h.y;
+            wi[q] -= vr[q] * h.y + vi[q] * h.x;
+            if (i < j) {
+                vr[q] = nr[q];
+                vi[q] = ni[q];
+            }
         }
     }
-    double *y = Y + (int64_t)(by_col ? c : k) * 2 * n;
+    double sq = 0.0, dummy = 0.0;
 #pragma unroll
-    for (int u = 0; u < RW; ++u) {
-        if (!in[u]) continue;
-        y[rr[u]] += sign * ar[u];
-        y[n + rr[u]] += sign * ai[u];
+    for (int q = 0; q < RPT; ++q) {
+        const int r = threadIdx.x + q * kMgsThreads;
+        if (r < n) {
+            w[r] = wr[q];
+            w[n + r] = wi[q];
+            sq += wr[q] * wr[q] + wi[q] * wi[q];
+        }
     }
+    block_sum2(sq, dummy);
+    if (threadIdx.x == 0) npart[k] = sq;
 }
 
 // ||W[k]||_2 (dznrm2): partial sums of squares per chunk.
@@ -316,23 +425,6 @@ __global__ void norm_finish(int nchunk, int count, const double *__restrict__ pa
     double s = 0.0;
     for (int b = 0; b < nchunk; ++b) s += part[(int64_t)k * nchunk + b];
     out[k] = sqrt(s);
-}
-
-// v_{j+1}[c] = W[k] / h_{j+1,j} (left zero when the norm is zero, as the
-// reference leaves the zero-filled column untouched); H(j+1, j) = norm.
-template <typename VT>
-__global__ void normalize(int n, const int32_t *__restrict__ act, const double *__restrict__ nrm,
-                          const double *__restrict__ W, VT *__restrict__ slab_next,
-                          double2 *__restrict__ Hcol, int hstride, int jrow) {
-    int k = blockIdx.y, c = act[k];
-    double s = nrm[k];
-    double inv = s != 0.0 ? 1.0 / s : 0.0;
-    const double *w = W + (int64_t)k * 2 * n;
-    VT *v = slab_next + (int64_t)c * 2 * n;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < 2LL * n;
-         r += (int64_t)gridDim.x * blockDim.x)
-        v[r] = (VT)(s != 0.0 ? w[r] * inv : 0.0);
-    if (blockIdx.x == 0 && threadIdx.x == 0) Hcol[(int64_t)c * hstride + jrow] = make_double2(s, 0.0);
 }
 
 // v_1 = b / ||b||; g_1 = ||b||.
@@ -370,7 +462,7 @@ __device__ __forceinline__ double2 shfl_up2(double2 v, int o) {
     return make_double2(__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o));
 }
 
-// Givens update of column j, one warp per active column.
+// Givens update of column j by one warp (norm = H(j+1, j)).
 // Hcols[j] points to the slab of H column j ([C][hstride] complex).
 //
 // The j earlier rotations form a chain: with a_0 = h_0 the i-th rotation gives
@@ -382,22 +474,15 @@ __device__ __forceinline__ double2 shfl_up2(double2 v, int o) {
 // as stable as the chain.  The result depends on j alone, not on the batch.
 // Latency bound; per launch, before -> after: 81 -> 6.1 us at 61 columns and 130
 // steps on average, 94 -> 8.5 us at 4 columns and 360 steps.
-constexpr int kGivensWarps = 2;
-
-__global__ void __launch_bounds__(32 * kGivensWarps) givens(int count, int j, const int32_t *__restrict__ act,
-                                                            double2 *const *__restrict__ Hcols, int hstride,
-                                                            double *__restrict__ cs, double2 *__restrict__ sn,
-                                                            double2 *__restrict__ g, int gstride, int cstride,
-                                                            double *__restrict__ resid) {
-    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (k >= count) return;
-    const int c = act[k];
+__device__ void givens(int k, int c, int lane, int j, double norm, double2 *const *__restrict__ Hcols, int hstride,
+                       double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g, int gstride,
+                       int cstride, double *__restrict__ resid) {
     double2 *h = Hcols[j] + (int64_t)c * hstride;
     double *csc = cs + (int64_t)c * cstride;
     double2 *snc = sn + (int64_t)c * cstride;
     double2 *gc = g + (int64_t)c * gstride;
     double2 a = h[0];                        // chain value entering the tile (same in every lane)
-    double2 cb = h[j + 1], g0 = gc[j], g1 = gc[j + 1];
+    double2 cb = make_double2(norm, 0.0), g0 = gc[j], g1 = gc[j + 1];
     double ci = lane < j ? csc[lane] : 1.0;
     double2 si = lane < j ? snc[lane] : make_double2(0.0, 0.0);
     double2 hn = lane < j ? h[lane + 1] : make_double2(0.0, 0.0);
@@ -457,6 +542,50 @@ __global__ void __launch_bounds__(32 * kGivensWarps) givens(int count, int j, co
     h[j] = ca;
     h[j + 1] = make_double2(0.0, 0.0);
     resid[k] = cabs_(g1);
+}
+
+// The end of an Arnoldi step: h_{j+1,j} = ||W[k]|| from the partial sums of squares,
+// v_{j+1}[c] = W[k] / h_{j+1,j} (zero when the norm is zero, as the reference leaves
+// the zero-filled column untouched), the Givens update of H's column j (one warp of
+// a column's first block), and the input X[k] = P v_{j+1} of the next product.
+// One launch in place of norm sum, scaling, Givens, gather and preconditioner.
+template <typename VT>
+__global__ void __launch_bounds__(256) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
+                                                        const double *__restrict__ npart,
+                                                        const double *__restrict__ W, VT *__restrict__ slab_next,
+                                                        const double *__restrict__ P, double *__restrict__ X,
+                                                        double2 *const *__restrict__ Hcols, int hstride,
+                                                        double *__restrict__ cs, double2 *__restrict__ sn,
+                                                        double2 *__restrict__ g, int gstride, int cstride,
+                                                        double *__restrict__ resid) {
+    __shared__ double total;
+    const int k = blockIdx.y, c = act[k];
+    double s = 0.0, dummy = 0.0;
+    for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += npart[(int64_t)k * nparts + b];
+    block_sum2(s, dummy);
+    if (threadIdx.x == 0) total = sqrt(s);
+    __syncthreads();
+    s = total;
+    const double inv = s != 0.0 ? 1.0 / s : 0.0;
+    const double *w = W + (int64_t)k * 2 * n;
+    VT *v = slab_next + (int64_t)c * 2 * n;
+    const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
+    double *x = X + (int64_t)k * 2 * n;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const VT vr = (VT)(s != 0.0 ? w[r] * inv : 0.0), vi = (VT)(s != 0.0 ? w[n + r] * inv : 0.0);
+        v[r] = vr;
+        v[n + r] = vi;
+        double re = (double)vr, im = (double)vi;
+        if (p) {
+            const double pr = p[r], pi = p[n + r], t = pr * re - pi * im;
+            im = pr * im + pi * re;
+            re = t;
+        }
+        x[r] = re;
+        x[n + r] = im;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 32)
+        givens(k, c, threadIdx.x, j, s, Hcols, hstride, cs, sn, g, gstride, cstride, resid);
 }
 
 // y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
@@ -576,18 +705,34 @@ __global__ void scale_cols(int n, const int32_t *__restrict__ idx, const double 
 
 int grid_rows(int64_t n2) { return (int)std::min<int64_t>(n_blocks(n2, 256), 1024); }
 
+// Groups of threads of combine() (see there).
+int combine_groups(int n, int ni) { return n <= 16384 && ni >= 16 ? 4 : 1; }
+int combine_blocks(int n, int ni) { return n_blocks(n, kThreads / combine_groups(n, ni)); }
+
 // combine() over at most kCombine basis vectors per launch (shared-memory bound).
+// ndot > 0: h holds chunk partials (FIN), for ni <= kCombine.  npart as in combine().
 constexpr int kCombine = 1024;
 template <typename VT>
 int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const int32_t *act,
-                        VT *const *slabs, const double2 *h, double sign, double *Y, int by_col) {
+                        VT *const *slabs, const double2 *h, double sign, double *Y, int by_col,
+                        int ndot = 0, double *npart = nullptr, double2 *Hcol = nullptr, int hstride = 0,
+                        int accumulate = 0) {
     int64_t launches = 0;
+    const int G = combine_groups(n, ni);
     for (int c0 = 0; c0 < ni; c0 += kCombine) {
         int cn = std::min(kCombine, ni - c0);
         // h is [count][ni]; pass the row stride through a shifted view per chunk
-        combine<VT><<<dim3(n_blocks(n, kThreads * kCombineRows), count), kThreads,
-                      cn * (sizeof(double2) + sizeof(VT *)), st>>>(
-            n, i0 + c0, cn, ni, c0, act, slabs, h, sign, Y, by_col);
+        const dim3 grid(n_blocks(n, kThreads / G), count);
+        const size_t smem = cn * (sizeof(double2) + sizeof(VT *));
+        double *np = c0 + cn == ni ? npart : nullptr;
+#define PLX_COMBINE(GG, FIN)                                                                                      \
+    combine<VT, GG, FIN><<<grid, kThreads, smem, st>>>(n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, \
+                                                       np, Hcol, hstride, accumulate)
+        if (G == 4 && ndot) PLX_COMBINE(4, true);
+        else if (G == 4) PLX_COMBINE(4, false);
+        else if (ndot) PLX_COMBINE(1, true);
+        else PLX_COMBINE(1, false);
+#undef PLX_COMBINE
         ++launches;
     }
     return launches;
@@ -631,8 +776,6 @@ class GmresRun final : public GmresStepper {
         if ((size_t)(m_ + 1) * sizeof(double2) > 200 * 1024) throw Error(PLX_ERR_ARG, "GMRES dimension above 12800");
         once_per_device(reinterpret_cast<const void *>(tri_solve), ctx_->device, [] {
             PLX_CHECK_CUDA(cudaFuncSetAttribute(tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         });
         hstride_ = m_ + 1;   // rows of an H column (0..m)
         d_act_.alloc(ctx_, C_);
@@ -641,7 +784,8 @@ class GmresRun final : public GmresStepper {
         Xa_.alloc(ctx_, (size_t)C_ * 2 * n);
         Wa_.alloc(ctx_, (size_t)C_ * 2 * n);
         work_.alloc(ctx_, (size_t)C_ * 2 * n);
-        nrm_part_.alloc(ctx_, (size_t)C_ * nchunk_);
+        // norm partials: per kRows rows, or per block of combine()
+        nrm_part_.alloc(ctx_, (size_t)C_ * std::max(nchunk_, n_blocks(n, kThreads / 4)));
         nrm_.alloc(ctx_, C_);
         cs_.alloc(ctx_, (size_t)C_ * m_);
         sn_.alloc(ctx_, (size_t)C_ * m_);
@@ -695,10 +839,9 @@ class GmresRun final : public GmresStepper {
     OpInput pre() override {
         const int n = g_->n_var;
         const int na = (int)act_.size();
-        gather_cols<VT><<<dim3(grid_rows(2LL * n), na), 256, 0, st_>>>(n, d_act_.p, h_slabs_[j_], Xa_.p);
-        ctx_->launches++;
-        if (jac_) {
-            scale_cols<<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, Pinv_.p, Xa_.p, 0);
+        if (!x_ready_) {
+            gather_cols<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, h_slabs_[j_],
+                                                                     jac_ ? Pinv_.p : nullptr, Xa_.p);
             ctx_->launches++;
         }
         return OpInput{g_, OpBatch{na, d_freq_act_.p}, Xa_.p, Wa_.p, work_.p, rq_.contraction};
@@ -720,32 +863,46 @@ class GmresRun final : public GmresStepper {
         PLX_CHECK_CUDA(cudaMemsetAsync(hcols_[j].p, 0, (size_t)C_ * hstride_ * 16, st_));
         size_t need = (size_t)na * ndot_ * (j + 1);
         if (part_.n < need) part_.alloc(ctx_, std::max(need, part_.n * 2));
-        auto project = [&](int i0, int i1, int accumulate) {
-            int ni = i1 - i0;
-            if (ni >= 8)
-                dots_wide<VT><<<dim3(ndot_, na), kThreads, 0, st_>>>(n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p, part_.p);
-            else
+        int nparts = 0;
+        // W -= V V^H W over basis vectors i0..i1-1, the coefficients into (or added to) H's
+        // column j; the last projection of the step leaves the norm partials
+        auto project = [&](int i0, int i1, int accumulate, bool last) {
+            const int ni = i1 - i0;
+            if (ni >= 8) {
+                const int nz = std::max(1, std::min(n_blocks(ni, kThreads / 32), n_blocks(592, ndot_ * na)));
+                dots_wide<VT><<<dim3(ndot_, na, nz), kThreads, 0, st_>>>(n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p,
+                                                                         part_.p);
+            } else {
                 dots_partial<VT><<<dim3(ndot_, na), kThreads, 0, st_>>>(n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p,
                                                                         part_.p);
-            dots_finish<<<dim3(n_blocks(ni, 128), na), 128, 0, st_>>>(ndot_, ni, i0, d_act_.p, part_.p, hbuf_.p,
-                                                                       hcols_[j].p, hstride_, accumulate);
-            ctx_->launches += 2 + combine_chunked(st_, n, i0, ni, na, d_act_.p, d_slabs_.p, hbuf_.p, -1.0, Wa_.p, 0);
+            }
+            ctx_->launches++;
+            const bool fin = ndot_ <= kCombineFin && ni <= kCombine;
+            if (!fin) {
+                dots_finish<<<dim3(n_blocks(ni, 128), na), 128, 0, st_>>>(ndot_, ni, i0, d_act_.p, part_.p, hbuf_.p,
+                                                                           hcols_[j].p, hstride_, accumulate);
+                ctx_->launches++;
+            }
+            if (last) nparts = combine_blocks(n, ni);
+            ctx_->launches += combine_chunked(st_, n, i0, ni, na, d_act_.p, d_slabs_.p, fin ? part_.p : hbuf_.p, -1.0,
+                                              Wa_.p, 0, fin ? ndot_ : 0, last ? nrm_part_.p : nullptr, hcols_[j].p,
+                                              hstride_, accumulate);
         };
         prof_begin(ctx_);
         if (j + 1 < 25 && !rq_.inner) {
-            for (int i = 0; i <= j; ++i) project(i, i + 1, 0);        // modified Gram-Schmidt
+            if (!mgs_fused(na, j, nparts))
+                for (int i = 0; i <= j; ++i) project(i, i + 1, 0, i == j);   // modified Gram-Schmidt
         } else {
-            project(0, j + 1, 0);                                     // classical GS ...
-            if (!rq_.single_pass) project(0, j + 1, 1);               // ... and re-orthogonalise
+            project(0, j + 1, 0, rq_.single_pass);                    // classical GS ...
+            if (!rq_.single_pass) project(0, j + 1, 1, true);         // ... and re-orthogonalise
         }
-        batch_norms(g_, na, Wa_.p, nrm_part_, nrm_);
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
         prof_begin(ctx_);
-        normalize<VT><<<dim3(grid_rows(2LL * n), na), 256, 0, st_>>>(n, d_act_.p, nrm_.p, Wa_.p, slabs_[j + 1].p,
-                                                                    hcols_[j].p, hstride_, j + 1);
-        givens<<<n_blocks(na, kGivensWarps), 32 * kGivensWarps, 0, st_>>>(na, j, d_act_.p, d_hcols_.p, hstride_, cs_.p, sn_.p, gv_.p,
-                                                  hstride_, m_, nrm_.p);
-        ctx_->launches += 2;
+        normalize_givens<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(
+            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, d_hcols_.p,
+            hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, nrm_.p);
+        ctx_->launches++;
+        x_ready_ = true;
         prof_end(ctx_, PROF_LSQ, 0.0, 0.0);
         PLX_CHECK_CUDA(cudaGetLastError());
         PLX_CHECK_CUDA(cudaMemcpyAsync(resid_.data(), nrm_.p, na * 8, cudaMemcpyDeviceToHost, st_));
@@ -780,6 +937,7 @@ class GmresRun final : public GmresStepper {
                     (rq_.tols.empty() ? rq_.tol : rq_.tols[c]))
                     res_.status[c] = PLX_ERR_NOT_CONVERGED;   // inner dimension used up (not an error)
         } else if (!trig.empty()) {
+            x_ready_ = false;                 // the true residual's product uses the input buffer
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
             tri_solve<<<nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
@@ -815,6 +973,7 @@ class GmresRun final : public GmresStepper {
             if (!done[c]) keep.push_back(c);
         if (keep.size() != act_.size()) {
             act_.swap(keep);
+            x_ready_ = false;                 // compact positions have changed
             if (!act_.empty()) upload_active();
         }
         ++j_;
@@ -827,6 +986,25 @@ class GmresRun final : public GmresStepper {
     }
 
   private:
+    // modified Gram-Schmidt in one launch where a block holds a column (the FP64 basis)
+    bool mgs_fused(int na, int j, int &nparts) {
+        if constexpr (std::is_same<VT, double>::value) {
+            const int n = g_->n_var;
+            if (n > 8 * kMgsThreads) return false;
+#define PLX_MGS(R) mgs_column<R><<<na, kMgsThreads, 0, st_>>>(n, j, d_act_.p, d_slabs_.p, Wa_.p, hcols_[j].p, hstride_, \
+                                                             nrm_part_.p)
+            if (n <= kMgsThreads) PLX_MGS(1);
+            else if (n <= 2 * kMgsThreads) PLX_MGS(2);
+            else if (n <= 4 * kMgsThreads) PLX_MGS(4);
+            else PLX_MGS(8);
+#undef PLX_MGS
+            ctx_->launches++;
+            nparts = 1;
+            return true;
+        }
+        return false;
+    }
+
     void upload_active() {
         std::vector<int32_t> fa(act_.size());
         for (size_t k = 0; k < act_.size(); ++k) fa[k] = rq_.freq[act_[k]];
@@ -843,6 +1021,7 @@ class GmresRun final : public GmresStepper {
     GmresResult &res_;
     int C_ = 0, m_ = 0, j_ = 0, nchunk_ = 0, ndot_ = 0, hstride_ = 0;
     bool jac_ = false;
+    bool x_ready_ = false;      // Xa holds the next product's input
     std::vector<int32_t> act_;
     std::vector<double> resid_;
     DevArray<int32_t> d_act_, d_freq_act_, d_cols_;

@@ -45,3 +45,22 @@ def test_residual_after_a_given_number_of_steps(ctx, steps):
     np.testing.assert_array_equal(tr, trace[:m])
     r = np.linalg.norm(b - op.matvec(1, x))
     assert abs(r - tr[-1]) <= 1e-6 * tr[-1]
+
+
+@pytest.mark.parametrize('steps', [1, 26, 40])
+def test_residual_above_the_fused_gram_schmidt(ctx, steps):
+    """4,693 unknowns: modified Gram-Schmidt vector by vector, norm partials over many blocks.
+    The same identity; the explicit residual is formed with the oracle's operator."""
+    p0 = configs.na_sphere(radius=35.0, n_freq=2, method='iterative')
+    text = p0.to_keyword_text()
+    p, s = Problem.from_keyword_text(text), model.System.from_keywords(keywords.read_keyword_text(text))
+    rng = np.random.default_rng(steps)
+    b = rng.standard_normal(p.n_var) + 1j * rng.standard_normal(p.n_var)
+    with Solver(p, ctx=ctx, store_t=True) as sv:
+        _, n, trace = sv.gmres(1, b, tol=3e-2 * np.linalg.norm(b), restart=500)
+        assert n >= 40
+        tol = trace[steps - 1] * (1.0 + 1e-6)
+        x, m, tr = sv.gmres(1, b, tol=tol, restart=500)
+    assert m == int(np.argmax(trace < tol)) + 1
+    r = np.linalg.norm(b - model.Operator(s).matvec(1, x))
+    assert abs(r - tr[-1]) <= 1e-6 * tr[-1]
