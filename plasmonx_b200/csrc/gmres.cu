@@ -18,6 +18,8 @@
 // FP64, and the refinement's FP64 residual absorbs the storage rounding.
 // Columns that converge leave the active list; the operator and the Arnoldi
 // kernels only touch active columns.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -65,12 +67,25 @@ __device__ __forceinline__ void block_sum2(double &a, double &b) {
     }
 }
 
+// The product's input split into BF16 high and low parts where it is formed (the
+// tensor-core contraction's column rows), in place of a pass that reads it again.
+__device__ __forceinline__ void split_column(const TcColumns &sp, int k, int r, double re, double im) {
+    const float a = (float)re, b = (float)im;
+    const __nv_bfloat16 ah = __float2bfloat16_rn(a), bh = __float2bfloat16_rn(b);
+    auto *hi = reinterpret_cast<__nv_bfloat16 *>(sp.hi) + 2 * (int64_t)k * sp.ld + r;
+    auto *lo = reinterpret_cast<__nv_bfloat16 *>(sp.lo) + 2 * (int64_t)k * sp.ld + r;
+    hi[0] = ah;
+    hi[sp.ld] = bh;
+    lo[0] = __float2bfloat16_rn(a - __bfloat162float(ah));
+    lo[sp.ld] = __float2bfloat16_rn(b - __bfloat162float(bh));
+}
+
 // X[k] = P[c] v elementwise for column c = act[k] of slab j (P = 1 when null): the
 // input of a step's product.  Only for the first step and when columns have left
 // the batch; otherwise `normalize_givens` has written it with the basis vector.
 template <typename VT>
 __global__ void gather_cols(int n, const int32_t *__restrict__ act, const VT *__restrict__ slab,
-                            const double *__restrict__ P, double *__restrict__ X) {
+                            const double *__restrict__ P, double *__restrict__ X, TcColumns sp) {
     const int k = blockIdx.y, c = act[k];
     const VT *src = slab + (int64_t)c * 2 * n;
     const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
@@ -84,6 +99,7 @@ __global__ void gather_cols(int n, const int32_t *__restrict__ act, const VT *__
         }
         dst[r] = re;
         dst[n + r] = im;
+        if (sp.hi) split_column(sp, k, r, re, im);
     }
 }
 
@@ -548,13 +564,14 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *cons
 // v_{j+1}[c] = W[k] / h_{j+1,j} (zero when the norm is zero, as the reference leaves
 // the zero-filled column untouched), the Givens update of H's column j (one warp of
 // a column's first block), and the input X[k] = P v_{j+1} of the next product.
-// One launch in place of norm sum, scaling, Givens, gather and preconditioner.
+// One launch in place of norm sum, scaling, Givens, gather, preconditioner and the
+// tensor-core split.
 template <typename VT>
 __global__ void __launch_bounds__(256) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
                                                         const double *__restrict__ npart,
                                                         const double *__restrict__ W, VT *__restrict__ slab_next,
                                                         const double *__restrict__ P, double *__restrict__ X,
-                                                        double2 *const *__restrict__ Hcols, int hstride,
+                                                        TcColumns sp, double2 *const *__restrict__ Hcols, int hstride,
                                                         double *__restrict__ cs, double2 *__restrict__ sn,
                                                         double2 *__restrict__ g, int gstride, int cstride,
                                                         double *__restrict__ resid) {
@@ -583,6 +600,7 @@ __global__ void __launch_bounds__(256) normalize_givens(int n, int j, const int3
         }
         x[r] = re;
         x[n + r] = im;
+        if (sp.hi) split_column(sp, k, r, re, im);
     }
     if (blockIdx.x == 0 && threadIdx.x < 32)
         givens(k, c, threadIdx.x, j, s, Hcols, hstride, cs, sn, g, gstride, cstride, resid);
@@ -799,6 +817,7 @@ class GmresRun final : public GmresStepper {
         h_slabs_.assign(m_ + 1, nullptr);
         h_hcols_.assign(m_, nullptr);
         PLX_CHECK_CUDA(cudaMemsetAsync(d_X_, 0, (size_t)C_ * 2 * n * 8, st_));
+        if (rq_.contraction == Contraction::TC3 || rq_.contraction == Contraction::TC1) split_ = tc_presplit(g_, C_);
         jac_ = rq_.jacobi && rq_.inner;
         if (jac_) {
             DevArray<int32_t> d_fall;
@@ -841,10 +860,10 @@ class GmresRun final : public GmresStepper {
         const int na = (int)act_.size();
         if (!x_ready_) {
             gather_cols<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, h_slabs_[j_],
-                                                                     jac_ ? Pinv_.p : nullptr, Xa_.p);
+                                                                     jac_ ? Pinv_.p : nullptr, Xa_.p, split_);
             ctx_->launches++;
         }
-        return OpInput{g_, OpBatch{na, d_freq_act_.p}, Xa_.p, Wa_.p, work_.p, rq_.contraction};
+        return OpInput{g_, OpBatch{na, d_freq_act_.p}, Xa_.p, Wa_.p, work_.p, rq_.contraction, split_.hi != nullptr};
     }
 
     // the Arnoldi step on W, the least-squares update and the convergence test
@@ -899,7 +918,7 @@ class GmresRun final : public GmresStepper {
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
         prof_begin(ctx_);
         normalize_givens<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(
-            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, d_hcols_.p,
+            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_hcols_.p,
             hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, nrm_.p);
         ctx_->launches++;
         x_ready_ = true;
@@ -1021,6 +1040,7 @@ class GmresRun final : public GmresStepper {
     GmresResult &res_;
     int C_ = 0, m_ = 0, j_ = 0, nchunk_ = 0, ndot_ = 0, hstride_ = 0;
     bool jac_ = false;
+    TcColumns split_{nullptr, nullptr, 0};   // tensor-core runs: the split rows of the next input
     bool x_ready_ = false;      // Xa holds the next product's input
     std::vector<int32_t> act_;
     std::vector<double> resid_;
@@ -1052,7 +1072,7 @@ void gmres_batched(plx_geom *g, const GmresRequest &rq, const double *d_B, doubl
     auto run = make_gmres(g, rq, d_B, d_X, res);
     while (run->wants_product()) {
         OpInput in = run->pre();
-        apply_operator(in.g, in.b, in.X, in.Y, in.work, in.how);
+        apply_operator(in.g, in.b, in.X, in.Y, in.work, in.how, in.presplit);
         run->post();
     }
     run->end();

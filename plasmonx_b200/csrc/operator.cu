@@ -443,36 +443,6 @@ __global__ void dipole_rows(int N, int nt, int nv, int count, const int32_t *__r
     Y[(int64_t)c * 2 * nv + nv + r] = sc[nv + r] + zre * xi + zim * xr;
 }
 
-// Rows after a contraction with the folded A0 = blockdiag(K - P, I) T (one atom
-// type): only the diagonal D(w) is left, y = s + D(w) x, with -z(w) on the
-// charge rows and sum_t f_t,i / alpha_t(w) on the dipole rows.
-__global__ void folded_rows(int N, int nt, int nv, int64_t ldS, int count, const int32_t *__restrict__ freq,
-                            const int32_t *__restrict__ type, const Cplx *__restrict__ dq,
-                            const double *__restrict__ frac, const Cplx *__restrict__ inv_alpha,
-                            const double *__restrict__ S, const double *__restrict__ X,
-                            double *__restrict__ Y) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (r >= nv || c >= count) return;
-    const int f = freq[c];
-    Cplx d = {0.0, 0.0};
-    if (r < N) {
-        d = dq[type[r] + nt * f];
-    } else {
-        const int i = (r - N) / 3;
-        for (int t = 0; t < nt; ++t) {
-            const double fr = frac[t + (int64_t)nt * i];
-            const Cplx a = inv_alpha[t + nt * f];
-            d.re += fr * a.re;
-            d.im += fr * a.im;
-        }
-    }
-    const int64_t base = (int64_t)c * 2 * nv, sb = (int64_t)c * 2 * ldS;
-    const double xr = X[base + r], xi = X[base + nv + r];
-    Y[base + r] = S[sb + r] + d.re * xr - d.im * xi;
-    Y[base + nv + r] = S[sb + ldS + r] + d.re * xi + d.im * xr;
-}
-
 // Alloy correction after the folded contraction: for every interface row i,
 //   y_i += sum_{j of another type} 1/2 (w_tj/w_ti(w) - 1) K_ji (s_j - s_i),
 // s = T x of the interface atoms (rows n + position in J of the output).
@@ -793,44 +763,46 @@ static double *folded_output(plx_geom *g, const OpBatch &b, double *work) {
     return g->d_fold_work.p;
 }
 
-// Y = S + D(w) X after the folded contraction S = A0 X (and the interface
-// correction of alloys).
-static void folded_finish(plx_geom *g, const OpBatch &b, const double *S, const double *X, double *Y) {
+// The interface correction of alloys after a folded contraction that has left
+// Y = A0 X + D(w) X and the interface atoms' T x in S.
+static void folded_finish(plx_geom *g, const OpBatch &b, const double *S, double *Y) {
+    if (g->n_xrows == 0) return;
     plx_ctx *ctx = g->ctx;
-    const int64_t M = g->fold_rows;
     prof_begin(ctx);
-    folded_rows<<<dim3(n_blocks(g->n_var, 256), b.count), 256, 0, ctx->stream>>>(
-        g->n_atoms, g->n_types, g->n_var, M, b.count, b.d_freq, g->d_type.p, g->d_dq.p, g->d_frac.p,
-        g->d_inv_alpha.p, S, X, Y);
+    iface_rows<<<dim3(n_blocks(g->n_xrows, 128), b.count), 128, 0, ctx->stream>>>(
+        g->n_xrows, b.count, g->n_types, g->n_var, g->fold_rows, b.d_freq, g->d_type.p, g->d_xrow.p, g->d_xipos.p,
+        g->d_xrowptr.p, g->d_xcol.p, g->d_xtj.p, g->d_xkt.p, g->d_wratio.p, S, Y);
     ctx->launches++;
-    if (g->n_xrows > 0) {
-        iface_rows<<<dim3(n_blocks(g->n_xrows, 128), b.count), 128, 0, ctx->stream>>>(
-            g->n_xrows, b.count, g->n_types, g->n_var, M, b.d_freq, g->d_type.p, g->d_xrow.p, g->d_xipos.p,
-            g->d_xrowptr.p, g->d_xcol.p, g->d_xtj.p, g->d_xkt.p, g->d_wratio.p, S, Y);
-        ctx->launches++;
-    }
     PLX_CHECK_CUDA(cudaGetLastError());
     prof_end(ctx, PROF_ROWS, 0.0, 0.0);
 }
 
 static double tc_bytes(plx_geom *g, Contraction how, int count) {
     const double nn = (double)g->n_var;
-    return (how == Contraction::TC3 ? 4.0 : 2.0) * (double)g->fold_rows * (double)g->ldk + 2.0 * 8.0 * nn * 2.0 * count;
+    const double rows = tc_folds_operator(g) ? (double)g->fold_rows : nn;
+    return (how == Contraction::TC3 ? 4.0 : 2.0) * rows * (double)g->ldk + 2.0 * 8.0 * nn * 2.0 * count;
+}
+
+// A tensor-core application: one contraction with the folded matrix (BEM: with D)
+// whose output rows already carry the diagonal, Y = A0 X + D(w) X.
+static TcItem tc_item(plx_geom *g, const OpBatch &b, const double *X, double *Y, double *work, Contraction how,
+                      bool presplit) {
+    const bool folds = tc_folds_operator(g);
+    return TcItem{g,     b.count, X, folds ? folded_output(g, b, work) : work, how == Contraction::TC3 ? 3 : 1, folds,
+                  b.d_freq, Y,    presplit};
 }
 
 void apply_operator(plx_geom *g, const OpBatch &b, const double *X, double *Y, double *work,
-                    Contraction how) {
+                    Contraction how, bool presplit) {
     if (b.count == 0) return;
-    if ((how == Contraction::TC3 || how == Contraction::TC1) && tc_folds_operator(g)) {
-        // A(w) X = A0 X + D(w) X: one tensor-core contraction with the folded
-        // matrix and a diagonal pass (no conductance rows per application)
+    if (how == Contraction::TC3 || how == Contraction::TC1) {
         plx_ctx *ctx = g->ctx;
         const double nn = (double)g->n_var;
-        double *S = folded_output(g, b, work);
+        const TcItem it = tc_item(g, b, X, Y, work, how, presplit);
         prof_begin(ctx);
-        tc_contract(g, b.count, X, S, how == Contraction::TC3 ? 3 : 1, true);
+        tc_contract_group({it});
         prof_end(ctx, PROF_TC, 2.0 * nn * nn * 2.0 * b.count, tc_bytes(g, how, b.count));
-        folded_finish(g, b, S, X, Y);
+        if (it.folded) folded_finish(g, b, it.S, Y);
         return;
     }
     contract_t(g, b.count, X, work, how);
@@ -857,17 +829,15 @@ void apply_operator_group(const std::vector<OpInput> &items) {
         if (ok) grp.push_back(i);
     }
     if (grp.size() < 2) {
-        for (const OpInput &it : items) apply_operator(it.g, it.b, it.X, it.Y, it.work, it.how);
+        for (const OpInput &it : items) apply_operator(it.g, it.b, it.X, it.Y, it.work, it.how, it.presplit);
         return;
     }
     plx_ctx *ctx = items[grp[0]].g->ctx;
     std::vector<TcItem> ti;
-    std::vector<double *> S;
     double flops = 0.0, bytes = 0.0;
     for (size_t k : grp) {
         const OpInput &it = items[k];
-        S.push_back(folded_output(it.g, it.b, it.work));
-        ti.push_back(TcItem{it.g, it.b.count, it.X, S.back(), it.how == Contraction::TC3 ? 3 : 1, true});
+        ti.push_back(tc_item(it.g, it.b, it.X, it.Y, it.work, it.how, it.presplit));
         const double nn = (double)it.g->n_var;
         flops += 2.0 * nn * nn * 2.0 * it.b.count;
         bytes += tc_bytes(it.g, it.how, it.b.count);
@@ -877,12 +847,12 @@ void apply_operator_group(const std::vector<OpInput> &items) {
     prof_end(ctx, PROF_TC, flops, bytes);
     for (size_t j = 0; j < grp.size(); ++j) {
         const OpInput &it = items[grp[j]];
-        folded_finish(it.g, it.b, S[j], it.X, it.Y);
+        folded_finish(it.g, it.b, ti[j].S, it.Y);
     }
     for (size_t i = 0; i < items.size(); ++i)
         if (std::find(grp.begin(), grp.end(), i) == grp.end()) {
             const OpInput &it = items[i];
-            apply_operator(it.g, it.b, it.X, it.Y, it.work, it.how);
+            apply_operator(it.g, it.b, it.X, it.Y, it.work, it.how, it.presplit);
         }
 }
 

@@ -174,8 +174,8 @@ struct plx_geom {
     plx::DevArray<int32_t> d_xcol, d_xtj;         // position of j in J, type of j
     plx::DevArray<double> d_xkt;                  // K_ji
     plx::DevArray<double> d_fold_work;            // [R][fold_rows] output of the folded contraction
-    // FP32 partial sums of the k-pieces of the tensor-core contraction's split
-    // tiles ([piece][column][256 rows])
+    // FP32 partial sums of the tensor-core contraction's split tiles
+    // ([slot][column][256 rows])
     plx::DevArray<float> d_tcpart;
     plx::DevArray<int> d_tc_err;
     // diagonal of blockdiag(Kop, I) T on the charge rows, frequency independent parts:
@@ -223,7 +223,7 @@ void upload_frequency_tables(plx_geom *g);
 //   Y = A(w_c) X for a batch: X, Y are [count][2][n_var] split-complex, device.
 //   work must hold 2*count*n_var doubles.
 void apply_operator(plx_geom *g, const OpBatch &b, const double *X, double *Y, double *work,
-                    Contraction how);
+                    Contraction how, bool presplit = false);
 //   S = T X (no K, no diagonal), S and X as above.
 void contract_t(plx_geom *g, int count, const double *X, double *S, Contraction how);
 //   S = X T for rows X [R][n] and a row-major n x n matrix in FP64
@@ -242,10 +242,22 @@ struct TcItem {
     plx_geom *g;
     int count;
     const double *X;
-    double *S;
+    double *S;                // [R][M] sums; with Y only the rows beyond n are written
     int nprod;
     bool folded;
+    const int32_t *d_freq;    // with Y: frequency of each column
+    double *Y;                // non-null: Y = S + D(w) X in place of S for the first n rows
+    bool presplit;            // the columns are in the buffers of tc_presplit already
 };
+// Split (BF16 high / low) rows of the columns, [2 count][ld]: where a producer of the
+// columns may write them itself (presplit).  Builds the operand if needed; valid until
+// the next contraction of the geometry without presplit.
+struct TcColumns {
+    uint16_t *hi, *lo;
+    int64_t ld;
+};
+TcColumns tc_presplit(plx_geom *g, int count);
+TcColumns tc_column_buffers(plx_geom *g, int count);
 void tc_contract_group(const std::vector<TcItem> &items);
 // true when apply_operator contracts with the folded A0 on the tensor cores:
 // every atomistic geometry (T stored or generated; alloys with the interface
@@ -317,6 +329,7 @@ struct OpInput {
     double *Y;
     double *work;
     Contraction how;
+    bool presplit;      // X is in the geometry's split column buffers already (tc_presplit)
 };
 // A batched GMRES advanced one Arnoldi step at a time (make_gmres has run the
 // set-up): while wants_product(): pre() returns the batch to multiply, the

@@ -389,7 +389,7 @@ void solve_refined(plx_geom *g, const RefineRequest &rq, const double *d_B, doub
         if (!os.begin()) break;
         OpInput need{};
         while (os.advance(&need)) {
-            apply_operator(need.g, need.b, need.X, need.Y, need.work, need.how);
+            apply_operator(need.g, need.b, need.X, need.Y, need.work, need.how, need.presplit);
             os.product_done();
         }
     }

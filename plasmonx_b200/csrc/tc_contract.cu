@@ -13,14 +13,14 @@
 //   D = TMEM accumulators 128 x BN (FP32), lane = row m, column = c
 // One CTA computes a 256 x BN tile of S as two 128-row accumulators (TMEM
 // columns [0, BN) and [BN, 2 BN)) that share every B tile, which halves the
-// B traffic from L2 per row of T; 4 warps: thread 0 issues the TMA
-// loads, thread 32 issues the MMAs, all 128 threads drain TMEM in the
-// epilogue.  Operand tiles are 32 elements (64 bytes) deep along k and are
+// B traffic from L2 per row of T.  Six warps: warps 0-3 drain TMEM in the
+// epilogue, one thread of warp 4 issues the loads and one of warp 5 the MMAs.
+// Operand tiles are 32 elements (64 bytes) deep along k and are
 // loaded by TMA with the 64-byte swizzle that the UMMA descriptors describe;
 // the small stages allow 4-6 of them in flight.
 // Every wait on an mbarrier is bounded.  The pipeline waits use the context's
 // limit (plx_set_wait_limit); a CTA whose wait runs out records an error code
-// and gives up, in this order: the MMA issuer still commits `done`, which
+// and gives up, in this order: the MMA issuer still commits `drained`, which
 // arrives only when every MMA it has issued has finished; all threads wait for
 // it, so no MMA reads shared memory or writes tensor memory after that point;
 // the producer then waits for the loads it has issued to land, so no copy
@@ -62,6 +62,10 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
@@ -148,33 +152,151 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
 // Work of one launch: the output tiles (256 rows x bn columns, column tile
 // fastest so that the tiles sharing one row block of an operand run side by
 // side and its second read comes from L2) of one or several groups -- a group
-// is one contraction S = A X of one geometry.  A group's first `full` tiles are
-// computed whole, one CTA each, and stored as FP64 into S; each of its
-// remaining tiles is split over k into q pieces of kper k-tiles, one CTA each,
-// which store FP32 partial sums into P (piece j at P + j * 256 * bn,
-// [column][row]); reduce_pieces adds a tile's pieces in order.  With the
-// pieces filling the last wave, every SM gets the same work (whole tiles plus
-// one piece) instead of a last wave that leaves SMs idle.  Several groups in one
-// launch run whole tiles only, the groups ordered by decreasing k length, so
-// that the hardware's in-order dispatch of CTAs to free SMs balances them.
+// is one contraction S = A X of one geometry -- in one list, the groups ordered
+// by decreasing k length.  The first `full` tiles (whole waves of the chip) are
+// computed whole, one CTA each.  The k-tiles of the remaining tiles, end to end,
+// are dealt to the CTAs of the last wave in equal runs of `run` k-tiles (at least
+// kMinRun): a run covers the end of one tile, perhaps whole small tiles, and the
+// beginning of another.  A tile that lies in one run is stored like a whole one;
+// the others leave FP32 partial sums ([column][row], slot = tile + CTA index, which
+// no two of them share), added in k order by reduce_pieces.
+//
+// The operand is streamed once whatever the split, so the launch is bound by HBM
+// (by L2 for operands that fit it) as long as every SM has the same share.  Splitting
+// each remaining tile into sms / remaining equal pieces left 38 SMs of 148 idle at 55
+// tiles (13,528 unknowns: 156 us a launch, now 121 us) and 24 at 31 tiles (7,844
+// unknowns: 51.7 -> 47 us); grouped launches ran whole tiles only, 30 CTAs for six
+// geometries of 143 to 2,700 unknowns (25.9 -> 11 us).
 constexpr int kMaxGroups = 6;
+constexpr int kMinRun = 8;          // k-tiles: below, a piece's prologue and partial sums cost more than it saves
+constexpr int kThreadsTc = 192;
+
+// The rest of an operator row after the contraction, applied where its sums are
+// complete: Y = S + D(w) X for the first n rows (D(w): -z(w) of the atom's type on
+// charge rows, sum_t f_t,i / alpha_t(w) on dipole rows; the BEM's z(w) with N = n,
+// nt = 1, type = null).  Rows beyond n go to S as without it.
+struct TcRows {
+    int n, N, nt;
+    const int32_t *freq, *type;
+    const Cplx *dq;
+    const double *frac;
+    const Cplx *inv_alpha;
+    const double *X;
+    double *Y;                  // null: no rows, S alone
+};
 struct TcGroup {
     int M, R, bn, ktiles;       // rows, real columns, column tile, k-tiles (32 deep)
-    int unit0;                  // first CTA of the group
-    int full, q, kper, ctiles;  // schedule (see above)
+    int ctiles;                 // column tiles
+    int tile0;                  // index of the group's first tile in the launch's list
+    int unit0;                  // k-tiles of the split tiles before the group
     const uint8_t *ah, *al;     // A high / low, tile-ordered and pre-swizzled (16 KB per stage tile)
     double *S;                  // [R][M] FP64
-    float *P;                   // pieces of the split tiles
     int *err;                   // the geometry's error word (first bounded wait that ran out)
+    TcRows rows;
 };
 struct TcLaunch {
-    CUtensorMap map[kMaxGroups][4];   // [2], [3]: X high, X low ([0], [1] unused: A goes by bulk copy)
+    CUtensorMap map[kMaxGroups][2];   // X high, X low (A goes by bulk copy)
     TcGroup grp[kMaxGroups];
-    int ngroups;
+    int ngroups, tiles;
+    int full;                   // tiles computed whole, one CTA each
+    int run, units;             // k-tiles a CTA of the split tiles takes, and their number
+    float *P;                   // partial sums, slots of 256 x bn_max
     int stages;                 // pipeline depth
     int bn_max;                 // shared-memory / tensor-memory sizing
     uint32_t wait_limit;
 };
+
+// A piece of work of a CTA: k-tiles [kt0, kt0 + nk) of a group's tile.
+struct TcSeg {
+    int gi, tile, kt0, nk, slot;     // slot < 0: the whole tile
+};
+
+// Group of tile t of the launch's list.
+__device__ __forceinline__ int group_of_tile(const TcLaunch &p, int t) {
+    int g = 0;
+    while (g + 1 < p.ngroups && t >= p.grp[g + 1].tile0) ++g;
+    return g;
+}
+
+// First split tile of a group (index within the group).
+__device__ __forceinline__ int first_split(const TcLaunch &p, int g) { return max(0, p.full - p.grp[g].tile0); }
+
+// The segments of a CTA in order: call with u = start of its range, advances u.
+__device__ __forceinline__ TcSeg next_segment(const TcLaunch &p, int cta, int &u, int uend) {
+    TcSeg s;
+    if (cta < p.full) {
+        s.gi = group_of_tile(p, cta);
+        s.tile = cta - p.grp[s.gi].tile0;
+        s.kt0 = 0;
+        s.nk = p.grp[s.gi].ktiles;
+        s.slot = -1;
+        u = uend;
+        return s;
+    }
+    int g = 0;
+    while (g + 1 < p.ngroups && u >= p.grp[g + 1].unit0) ++g;
+    const int kt = p.grp[g].ktiles, rem = u - p.grp[g].unit0, local = rem / kt;
+    s.gi = g;
+    s.tile = first_split(p, g) + local;
+    s.kt0 = rem - local * kt;
+    s.nk = min(kt - s.kt0, uend - u);
+    s.slot = s.nk == kt ? -1 : p.grp[g].tile0 + s.tile - p.full + (cta - p.full);
+    u += s.nk;
+    return s;
+}
+
+// Stores the complete sums s of real columns c .. c + 2 NP - 1 (NP complex columns,
+// those inside the batch) at row r.  All its loads go out before the first store: one
+// column after the other, each behind the previous one's store, took 50 us of a
+// 713 us launch at 48 columns.
+template <int NP>
+__device__ __forceinline__ void store_columns(const TcGroup &G, int r, int c, const double (&s)[2 * NP]) {
+    const TcRows &q = G.rows;
+    if (!(q.Y && r < q.n)) {
+#pragma unroll
+        for (int k = 0; k < 2 * NP; ++k)
+            if (c + k < G.R) G.S[(int64_t)(c + k) * G.M + r] = s[k];
+        return;
+    }
+    Cplx d[NP];
+    double x[2 * NP];
+    int f[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        const bool in = c + 2 * k < G.R;
+        f[k] = in ? __ldg(q.freq + (c >> 1) + k) : 0;
+        const int64_t o = (int64_t)(c + 2 * k) * q.n + r;
+        x[2 * k] = in ? __ldg(q.X + o) : 0.0;
+        x[2 * k + 1] = in ? __ldg(q.X + o + q.n) : 0.0;
+        d[k] = {0.0, 0.0};
+    }
+    if (r < q.N) {
+        const double2 *dq = reinterpret_cast<const double2 *>(q.dq) + (q.type ? __ldg(q.type + r) : 0);
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const double2 v = __ldg(dq + q.nt * f[k]);
+            d[k] = {v.x, v.y};
+        }
+    } else {
+        const double *frac = q.frac + (int64_t)q.nt * ((r - q.N) / 3);
+        for (int t = 0; t < q.nt; ++t) {
+            const double fr = __ldg(frac + t);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const double2 v = __ldg(reinterpret_cast<const double2 *>(q.inv_alpha) + t + q.nt * f[k]);
+                d[k].re += fr * v.x;
+                d[k].im += fr * v.y;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+        if (c + 2 * k < G.R) {
+            const int64_t o = (int64_t)(c + 2 * k) * q.n + r;
+            q.Y[o] = s[2 * k] + d[k].re * x[2 * k] - d[k].im * x[2 * k + 1];
+            q.Y[o + q.n] = s[2 * k + 1] + d[k].re * x[2 * k + 1] + d[k].im * x[2 * k];
+        }
+}
 
 // Bytes of one pipeline stage: the A and X tiles its products read -- high and
 // low parts for three products, the high parts alone for one (whose stages are
@@ -184,52 +306,44 @@ __host__ __device__ constexpr int tc_stage_bytes(int bn, int nprod) {
 }
 
 template <int NPROD>
-__global__ void __launch_bounds__(128, 1) tc_contract_kernel(const __grid_constant__ TcLaunch p) {
-    // this CTA's group and unit: a whole tile, or one k-piece of a remaining tile
-    int gi = 0;
-    while (gi + 1 < p.ngroups && (int)blockIdx.x >= p.grp[gi + 1].unit0) ++gi;
-    const TcGroup &G = p.grp[gi];
-    const int u = (int)blockIdx.x - G.unit0;
-    int tile, kt0, nk, piece = -1;
-    if (u < G.full) {
-        tile = u;
-        kt0 = 0;
-        nk = G.ktiles;
-    } else {
-        piece = u - G.full;
-        tile = G.full + piece / G.q;
-        kt0 = (piece % G.q) * G.kper;
-        nk = min(G.ktiles, kt0 + G.kper) - kt0;
-    }
-    const int bn = G.bn, M = G.M, R = G.R, ktiles = G.ktiles;
-    const int bnp = (bn + 31) & ~31;     // TMEM columns of one accumulator (32-aligned)
+__global__ void __launch_bounds__(kThreadsTc, 1) tc_contract_kernel(const __grid_constant__ TcLaunch p) {
+    const int cta = (int)blockIdx.x;
+    const int u0 = cta < p.full ? 0 : (cta - p.full) * p.run;
+    const int uend = cta < p.full ? 1 : min(p.units, u0 + p.run);
     const int STAGES = p.stages;
     const int kStage = tc_stage_bytes(p.bn_max, NPROD);
     const int kA = kBM * kBK * 2;
-    const int mtile = tile / G.ctiles;
-    int *err = G.err;
     const uint32_t wait_limit = p.wait_limit;
-    // two accumulators of bn columns each (rows m0.. and m0 + 128..), at TMEM
-    // columns 0 and bnp; bn_max is a multiple of 32
-    const uint32_t tmem_cols = 2 * p.bn_max <= 64 ? 64 : (2 * p.bn_max <= 128 ? 128 : (2 * p.bn_max <= 256 ? 256 : 512));
+    // an accumulator set is two accumulators (rows m0.. and m0 + 128..) of bn_max columns
+    // (a multiple of 32); two sets where they fit the 512 TMEM columns, so that a
+    // segment's products start while the previous one is stored
+    const int set_cols = 2 * p.bn_max;
+    const int nbuf = 2 * set_cols <= 512 ? 2 : 1;
+    const int need_cols = nbuf * set_cols;
+    const uint32_t tmem_cols = need_cols <= 64 ? 64 : (need_cols <= 128 ? 128 : (need_cols <= 256 ? 256 : 512));
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(base + STAGES * kStage);
     uint64_t *empty = full + STAGES;
-    uint64_t *done = empty + STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+    uint64_t *done = empty + STAGES;          // [2]: a set's sums are complete
+    uint64_t *freed = done + 2;               // [2]: a set has been read out
+    uint64_t *drained = freed + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *err = p.grp[0].err;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (tile % G.ctiles) * bn;
-    const int m0 = mtile * kBM;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(done, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&done[s], 1);
+            mbar_init(&freed[s], 128);
+        }
+        mbar_init(drained, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -244,143 +358,201 @@ __global__ void __launch_bounds__(128, 1) tc_contract_kernel(const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    auto stage_ptr = [&](int s, int which) -> uint8_t * {
-        // which: 0 A high, 1 A low, 2 X high, 3 X low (the low parts only for NPROD > 1)
-        constexpr int parts = NPROD > 1 ? 2 : 1;
-        uint8_t *st = base + s * kStage;
-        return which < 2 ? st + which * kA : st + parts * kA + (which - 2) * (p.bn_max * kBK * 2);
-    };
+    // a stage holds A high (A low), X high (X low); the low parts only for NPROD > 1.  The
+    // issuing threads keep stage, phase and addresses as running values: their loop is the
+    // launch's limit at few columns, and recomputing them (a division by the number of
+    // stages among it) cost 640 cycles a k-tile against 32-64 per product (41,892
+    // unknowns, 42 columns: one product 675 -> 509 us, three 1,077 -> 990 us, 6.9-7.1 TB/s)
+    constexpr int kParts = NPROD > 1 ? 2 : 1;
+    const int kX = kParts * kA, kXl = p.bn_max * kBK * 2;
 
-    int issued = 0;     // loads issued by the producer (thread 0)
-    if (threadIdx.x == 0) {
+    int issued = 0;     // loads issued by the producer
+    if (threadIdx.x == 128) {
         // ---------------- TMA producer ----------------
-        const CUtensorMap *mp = p.map[gi];
-        // one product (NPROD = 1) reads only the high parts: half the operand bytes
-        const uint32_t tx = (uint32_t)(NPROD > 1 ? 2 * kA + 2 * bn * kBK * 2 : kA + bn * kBK * 2);
-        for (int kt = 0; kt < nk; ++kt) {
-            const int s = kt % STAGES;
-            if (kt >= STAGES) {
-                if (!mbar_wait(&empty[s], ((kt / STAGES) - 1) & 1, wait_limit, abort_flag, err, 1) || *abort_flag) {
+        int u = u0, s = 0;
+        uint32_t ph = 1;                      // a stage's first use finds its barrier free
+        uint8_t *st = base;
+        bool ok = true;
+        while (u < uend && ok) {
+            const TcSeg sg = next_segment(p, cta, u, uend);
+            const TcGroup &G = p.grp[sg.gi];
+            const CUtensorMap *mp = p.map[sg.gi];
+            const int bn = G.bn, mtile = sg.tile / G.ctiles, n0 = (sg.tile % G.ctiles) * bn;
+            // one product (NPROD = 1) reads only the high parts: half the operand bytes
+            const uint32_t tx = (uint32_t)(NPROD > 1 ? 2 * kA + 2 * bn * kBK * 2 : kA + bn * kBK * 2);
+            const size_t a0 = (size_t)(mtile * (int64_t)G.ktiles + sg.kt0) * kA;   // tile-ordered A
+            const uint8_t *ah = G.ah + a0, *al = G.al + a0;
+            int kx = sg.kt0 * kBK;
+            for (int kt = 0; kt < sg.nk; ++kt) {
+                if (!mbar_wait(&empty[s], ph, wait_limit, abort_flag, err, 1)) {
                     *abort_flag = 1;
+                    ok = false;
                     break;
                 }
+                uint64_t *bar = &full[s];
+                mbar_expect_tx(bar, tx);
+                bulk_load(st, ah, kA, bar);
+                if (NPROD > 1) bulk_load(st + kA, al, kA, bar);
+                tma_load_2d(&mp[0], bar, st + kX, kx, n0);
+                if (NPROD > 1) tma_load_2d(&mp[1], bar, st + kX + kXl, kx, n0);
+                ah += kA;
+                al += kA;
+                kx += kBK;
+                ++issued;
+                st += kStage;
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                    st = base;
+                }
             }
-            mbar_expect_tx(&full[s], tx);
-            const int kx = (kt0 + kt) * kBK;
-            const size_t aoff = (size_t)(mtile * ktiles + kt0 + kt) * kA;   // tile-ordered A
-            bulk_load(stage_ptr(s, 0), G.ah + aoff, kA, &full[s]);
-            if (NPROD > 1) bulk_load(stage_ptr(s, 1), G.al + aoff, kA, &full[s]);
-            tma_load_2d(&mp[2], &full[s], stage_ptr(s, 2), kx, n0);
-            if (NPROD > 1) tma_load_2d(&mp[3], &full[s], stage_ptr(s, 3), kx, n0);
-            issued = kt + 1;
         }
-    } else if (threadIdx.x == 32) {
+    } else if (threadIdx.x == 160) {
         // ---------------- MMA issuer ----------------
-        const uint32_t idesc = umma_idesc_bf16(kUM, bn);
         constexpr uint64_t kHalf = (uint64_t)(kUM * kBK * 2) >> 4;   // second 128 rows of an A tile
-        for (int kt = 0; kt < nk; ++kt) {
-            const int s = kt % STAGES;
-            if (!mbar_wait(&full[s], (kt / STAGES) & 1, wait_limit, abort_flag, err, 2) || *abort_flag) {
+        // stage 0's descriptors; a stage, a part and a k step add to the address field
+        const uint64_t d0 = umma_desc_sw64(base);
+        const uint64_t dStage = (uint64_t)kStage >> 4, dLow = (uint64_t)kA >> 4, dX = (uint64_t)kX >> 4,
+                       dXl = (uint64_t)kXl >> 4;
+        int u = u0, s = 0;
+        uint32_t ph = 0;
+        uint64_t da = d0;
+        bool ok = true;
+        for (int seg = 0; u < uend && ok; ++seg) {
+            const TcSeg sg = next_segment(p, cta, u, uend);
+            const int buf = seg % nbuf;
+            const uint32_t idesc = umma_idesc_bf16(kUM, p.grp[sg.gi].bn);
+            if (seg >= nbuf && !mbar_wait(&freed[buf], ((seg / nbuf) - 1) & 1, wait_limit, abort_flag, err, 6)) {
                 *abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t dTh = umma_desc_sw64(stage_ptr(s, 0));
-            const uint64_t dTl = umma_desc_sw64(stage_ptr(s, 1));
-            const uint64_t dXh = umma_desc_sw64(stage_ptr(s, 2));
-            const uint64_t dXl = umma_desc_sw64(stage_ptr(s, 3));
+            const uint32_t t0 = tmem + (uint32_t)(buf * set_cols), t1 = t0 + (uint32_t)p.bn_max;
+            for (int kt = 0; kt < sg.nk; ++kt) {
+                if (!mbar_wait(&full[s], ph, wait_limit, abort_flag, err, 2)) {
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
-                // advance 16 elements = 32 bytes = 2 descriptor units along k
-                const uint64_t off = (uint64_t)(kk * kUmmaK * 2) >> 4;
-                const uint32_t acc0 = (kt > 0 || kk > 0) ? 1u : 0u;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint32_t td = tmem + (uint32_t)(h * bnp);
-                    const uint64_t ho = h * kHalf;
-                    umma_bf16(td, dTh + ho + off, dXh + off, idesc, acc0);
+                for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
+                    // advance 16 elements = 32 bytes = 2 descriptor units along k
+                    const uint64_t a = da + ((uint64_t)(kk * kUmmaK * 2) >> 4), x = a + dX;
+                    const uint32_t acc0 = (kt > 0 || kk > 0) ? 1u : 0u;
+                    umma_bf16(t0, a, x, idesc, acc0);
+                    umma_bf16(t1, a + kHalf, x, idesc, acc0);
                     if (NPROD > 1) {
-                        umma_bf16(td, dTh + ho + off, dXl + off, idesc, 1u);
-                        umma_bf16(td, dTl + ho + off, dXh + off, idesc, 1u);
+                        umma_bf16(t0, a, x + dXl, idesc, 1u);
+                        umma_bf16(t1, a + kHalf, x + dXl, idesc, 1u);
+                        umma_bf16(t0, a + dLow, x, idesc, 1u);
+                        umma_bf16(t1, a + dLow + kHalf, x, idesc, 1u);
                     }
                 }
+                umma_commit(&empty[s]);
+                da += dStage;
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                    da = d0;
+                }
             }
-            umma_commit(&empty[s]);
+            if (ok) umma_commit(&done[buf]);
         }
         // always: arrives once every MMA issued above has completed (also after
         // an abort, so that nothing below frees memory an MMA still uses)
-        umma_commit(done);
+        umma_commit(drained);
+    } else if (warp < 4) {
+        // ---------------- epilogue: TMEM -> result, or the piece's partial (FP32) ----------------
+        int u = u0;
+        for (int seg = 0; u < uend; ++seg) {
+            const TcSeg sg = next_segment(p, cta, u, uend);
+            const TcGroup &G = p.grp[sg.gi];
+            const int bn = G.bn, buf = seg % nbuf;
+            const int m0 = sg.tile / G.ctiles * kBM, n0 = (sg.tile % G.ctiles) * bn;
+            // one lane polls; the warp stays together, the loads below are warp-wide
+            bool ok = true;
+            if (lane == 0) ok = mbar_wait(&done[buf], (seg / nbuf) & 1, wait_limit, abort_flag, err, 3) && !*abort_flag;
+            if (!__all_sync(0xffffffffu, ok)) {
+                *abort_flag = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int row = m0 + h * kUM + warp * 32 + lane;
+#pragma unroll 1
+                for (int c0 = 0; c0 < bn; c0 += 16) {
+                    uint32_t v[16];
+                    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * set_cols + h * p.bn_max + c0);
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                          "=r"(v[14]), "=r"(v[15])
+                        : "r"(taddr));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (sg.slot >= 0) {
+                        // partial of a split tile: [column][256 rows] FP32, every element written
+                        float *pp = p.P + (int64_t)sg.slot * kBM * p.bn_max + (h * kUM + warp * 32 + lane);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) pp[(int64_t)(c0 + j) * kBM] = __uint_as_float(v[j]);
+                    } else if (row < G.M) {
+                        double s[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) s[j] = (double)__uint_as_float(v[j]);
+                        store_columns<8>(G, row, n0 + c0, s);
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(&freed[buf]);
+        }
     }
     __syncwarp();
-
-    // ---------------- epilogue: TMEM -> S (FP64) or the piece's partial (FP32) ----------------
-    bool fin = mbar_wait(done, 0, wait_limit, nullptr, err, 3);
-    if (!fin) {
-        *abort_flag = 1;
-        fin = mbar_wait(done, 0, kDrainLimit, nullptr, err, 4);
-    }
-    // uniform over the CTA; a thread that raised the flag counts it itself
-    const bool have = !__syncthreads_or(*abort_flag != 0 || !fin);
-    if (!have && threadIdx.x == 0) {
+    __syncthreads();
+    // every MMA issued has finished before shared and tensor memory go
+    if (!mbar_wait(drained, 0, kDrainLimit, nullptr, err, 4)) *abort_flag = 1;
+    if (threadIdx.x == 128 && *abort_flag) {
         // let the loads already issued land before the CTA can exit: the last
         // phase of each stage (earlier phases completed before it was re-armed)
         for (int kt = issued > STAGES ? issued - STAGES : 0; kt < issued; ++kt)
             mbar_wait(&full[kt % STAGES], (kt / STAGES) & 1, kDrainLimit, nullptr, err, 5);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (have) {
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        const int row = m0 + h * kUM + warp * 32 + lane;
-#pragma unroll 1
-        for (int c0 = 0; c0 < bn; c0 += 32) {
-            uint32_t v[32];
-            const int nc = min(32, bn - c0);           // 32, or 16 for the last chunk
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * bnp + c0);
-            if (nc == 32) {
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                    "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                      "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                      "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-                      "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                      "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr));
-            } else {
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                      "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                      "=r"(v[14]), "=r"(v[15])
-                    : "r"(taddr));
-#pragma unroll
-                for (int j = 16; j < 32; ++j) v[j] = 0u;
-            }
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (piece >= 0) {
-                // partial of a split tile: [column][256 rows] FP32, every element written
-                float *pp = G.P + (int64_t)piece * kBM * bn + (h * kUM + warp * 32 + lane);
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < nc) pp[(int64_t)(c0 + j) * kBM] = __uint_as_float(v[j]);
-            } else if (row < M) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int c = n0 + c0 + j;
-                    if (j < nc && c < R) G.S[(int64_t)c * M + row] = (double)__uint_as_float(v[j]);
-                }
-            }
-        }
-      }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
     }
+}
+
+// Split tiles: the sum of a tile's FP32 pieces in k order (FP64 sums), stored like a
+// whole tile.  One block per (split tile, eight columns), a thread per row: all its
+// loads are independent (32 columns a block and thread: 14 us at 7,844 unknowns and
+// 124 pieces, now 6.6 us with the diagonal rows that took 4.1 us in a launch of
+// their own).
+constexpr int kRedCols = 8;
+__global__ void __launch_bounds__(kBM) reduce_pieces(const __grid_constant__ TcLaunch p) {
+    const int t = p.full + blockIdx.x;                       // index in the launch's list
+    const int g = group_of_tile(p, t);
+    const TcGroup &G = p.grp[g];
+    const int tile = t - G.tile0;
+    const int k0 = G.unit0 + (tile - first_split(p, g)) * G.ktiles;      // its k-tiles [k0, k0 + ktiles)
+    const int f0 = k0 / p.run, f1 = (k0 + G.ktiles - 1) / p.run;         // CTAs that hold them
+    if (f0 == f1) return;                                    // stored by its one CTA
+    const int m0 = tile / G.ctiles * kBM, n0 = (tile % G.ctiles) * G.bn;
+    const int r = threadIdx.x, c0 = blockIdx.y * kRedCols;
+    if (m0 + r >= G.M || c0 >= G.bn) return;
+    double a[kRedCols];
+#pragma unroll
+    for (int j = 0; j < kRedCols; ++j) a[j] = 0.0;
+    for (int c = f0; c <= f1; ++c) {
+        const float *pp = p.P + ((int64_t)(blockIdx.x + c) * p.bn_max + c0) * kBM + r;
+#pragma unroll
+        for (int j = 0; j < kRedCols; ++j) a[j] += (double)pp[(int64_t)j * kBM];
+    }
+    store_columns<kRedCols / 2>(G, m0 + r, n0 + c0, a);
 }
 
 // The A operand (T, A0 or D^T split in BF16 high/low) is stored in the order
@@ -506,17 +678,14 @@ __global__ void fold_split(int N, int n, int64_t ld, int64_t ktiles, int hetero,
     split_store(a, a_tiled(r, k, ktiles), hi, lo);
 }
 
-// FP64 -> (BF16 high, BF16 low) split of a row-major [rows][cols] array into a
-// zero-padded [rows_pad][ld] pair.
-__global__ void split_bf16(int rows, int cols, int64_t ld_in, const double *__restrict__ in, int rows_pad,
-                           int64_t ld_out, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
-    int64_t total = (int64_t)rows_pad * ld_out;
+// FP64 -> (BF16 high, BF16 low) split of row-major rows [rows][n] into rows of ld
+// elements, whose padding stays zero.
+__global__ void split_bf16(int rows, int n, const double *__restrict__ in, int64_t ld, __nv_bfloat16 *__restrict__ hi,
+                           __nv_bfloat16 *__restrict__ lo) {
+    const int64_t total = (int64_t)rows * n;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = e / ld_out, c = e % ld_out;
-        float x = (r < rows && c < cols) ? (float)in[r * ld_in + c] : 0.0f;
-        __nv_bfloat16 h = __float2bfloat16_rn(x);
-        hi[e] = h;
-        lo[e] = __float2bfloat16_rn(x - __bfloat162float(h));
+        const int64_t r = e / n;
+        split_store(in[e], r * ld + (e - r * n), hi, lo);
     }
 }
 
@@ -551,49 +720,33 @@ CUtensorMap make_map(const void *ptr, uint64_t inner, uint64_t outer, uint64_t l
     return m;
 }
 
-// Remaining tiles of a group: S = the sum of a tile's q FP32 pieces in piece
-// order (FP64 sums), for the rows and columns inside the matrix.  One block per
-// (tile, 32-column group); threads over the tile's 256 rows.
-__global__ void reduce_pieces(int M, int R, int bn, int full, int ctiles, int q, const float *__restrict__ P,
-                              double *__restrict__ S) {
-    const int t = blockIdx.x;                       // remaining tile index
-    const int tile = full + t;
-    const int m0 = (tile / ctiles) * kBM, n0 = (tile % ctiles) * bn;
-    const int r = threadIdx.x;                      // 0..255
-    if (m0 + r >= M) return;
-    for (int c = blockIdx.y * 32; c < min(bn, blockIdx.y * 32 + 32); ++c) {
-        if (n0 + c >= R) break;
-        double a = 0.0;
-        for (int p = 0; p < q; ++p) a += (double)P[((int64_t)(t * q + p) * bn + c) * kBM + r];
-        S[(int64_t)(n0 + c) * M + m0 + r] = a;
-    }
-}
-
 int sm_count(int device) {
     int v = 0;
     PLX_CHECK_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device));
     return v > 0 ? v : 1;
 }
 
-// Schedule of one group's `tiles` output tiles of `ktiles` k-tiles on `sms` SMs
-// (one CTA per SM): whole tiles in full waves; the r = tiles mod sms tiles of
-// the last wave are split into q = sms / r pieces (at least 8 k-tiles each)
-// when that lets the pieces fill the wave -- otherwise (r close to sms, or no
-// split possible) they run whole too.  Returns the group's number of CTAs.
-int make_schedule(TcGroup &gp, int tiles, int sms, bool split) {
-    gp.full = tiles;
-    gp.q = 1;
-    gp.kper = gp.ktiles;
-    const int r = tiles % sms;
-    if (!split || r == 0 || (double)r / sms >= 0.9) return tiles;
-    int q = std::min(sms / r, gp.ktiles / 8);
-    if (q < 2) return tiles;
-    const int kper = (gp.ktiles + q - 1) / q;
-    q = (gp.ktiles + kper - 1) / kper;              // no empty piece
-    gp.full = tiles - r;
-    gp.q = q;
-    gp.kper = kper;
-    return gp.full + r * q;
+// Schedule of the launch's tiles on `sms` SMs (one CTA per SM, see TcLaunch): whole
+// waves of whole tiles, and the last wave's k-tiles in equal runs -- unless its tiles
+// fill at least 0.9 of the chip (splitting would cost more in partial sums than the
+// idle SMs) or would be split below kMinRun k-tiles a CTA.  Sets full, run, units and
+// the groups' unit0; returns the number of CTAs.
+int make_schedule(TcLaunch &L, int sms) {
+    const int r = L.tiles % sms;
+    L.full = r >= 0.9 * sms ? L.tiles : L.tiles - r;
+    L.units = 0;
+    for (int g = 0; g < L.ngroups; ++g) {
+        TcGroup &gp = L.grp[g];
+        const int end = g + 1 < L.ngroups ? L.grp[g + 1].tile0 : L.tiles;
+        gp.unit0 = L.units;
+        L.units += std::max(0, end - std::max(gp.tile0, L.full)) * gp.ktiles;
+    }
+    if (L.units == 0) {
+        L.run = 1;
+        return L.full;
+    }
+    L.run = std::max(kMinRun, (L.units + sms - 1) / sms);
+    return L.full + (L.units + L.run - 1) / L.run;
 }
 
 }  // namespace
@@ -803,8 +956,7 @@ void tc_contract_group(const std::vector<TcItem> &items) {
                 for (const TcItem &it : items) tc_contract_group({it});
                 return;
             }
-    const bool single = items.size() == 1;
-    // longest k first: the hardware hands CTAs to free SMs in launch order
+    // longest k first: whole tiles go to the SMs in launch order
     std::vector<int> order(items.size());
     for (size_t i = 0; i < items.size(); ++i) order[i] = (int)i;
     std::stable_sort(order.begin(), order.end(),
@@ -813,12 +965,8 @@ void tc_contract_group(const std::vector<TcItem> &items) {
     std::memset(&L, 0, sizeof(L));
     L.ngroups = (int)items.size();
     L.wait_limit = ctx->wait_limit;
-    int units = 0, bn_max = 32;
+    int bn_max = 32;
     const int sms = sm_count(ctx->device);
-    struct Post {
-        int gi, rem;
-    };
-    std::vector<Post> post;
     for (int k = 0; k < L.ngroups; ++k) {
         const TcItem &it = items[order[k]];
         plx_geom *g = it.g;
@@ -836,17 +984,15 @@ void tc_contract_group(const std::vector<TcItem> &items) {
         const int ntile = (R + 255) / 256;
         const int bn = ((R + ntile - 1) / ntile + 15) / 16 * 16;
         const int Rpad = ntile * bn;
-        const size_t need = (size_t)Rpad * ld;
-        if (g->d_Xh.n < need) {
-            g->d_Xh.alloc(ctx, need);
-            g->d_Xl.alloc(ctx, need);
+        if (!it.presplit) {
+            tc_column_buffers(g, it.count);
+            split_bf16<<<std::min<int64_t>(4096, n_blocks((int64_t)R * n, 256)), 256, 0, ctx->stream>>>(
+                R, n, it.X, ld, reinterpret_cast<__nv_bfloat16 *>(g->d_Xh.p),
+                reinterpret_cast<__nv_bfloat16 *>(g->d_Xl.p));
+            ctx->launches++;
         }
-        split_bf16<<<std::min<int64_t>(4096, n_blocks((int64_t)Rpad * ld, 256)), 256, 0, ctx->stream>>>(
-            R, n, n, it.X, Rpad, ld, reinterpret_cast<__nv_bfloat16 *>(g->d_Xh.p),
-            reinterpret_cast<__nv_bfloat16 *>(g->d_Xl.p));
-        ctx->launches++;
-        L.map[k][2] = make_map(g->d_Xh.p, ld, Rpad, ld, bn);
-        L.map[k][3] = make_map(g->d_Xl.p, ld, Rpad, ld, bn);
+        L.map[k][0] = make_map(g->d_Xh.p, ld, Rpad, ld, bn);
+        L.map[k][1] = make_map(g->d_Xl.p, ld, Rpad, ld, bn);
         TcGroup &gp = L.grp[k];
         // A in tile order, one contiguous pre-swizzled 16 KB block per stage tile
         gp.ah = reinterpret_cast<const uint8_t *>(it.folded ? g->d_Ah.p : g->d_Th.p);
@@ -856,42 +1002,76 @@ void tc_contract_group(const std::vector<TcItem> &items) {
         gp.bn = bn;
         gp.ktiles = (int)(ld / kBK);
         gp.ctiles = ntile;
-        gp.unit0 = units;
+        gp.tile0 = L.tiles;
         gp.S = it.S;
-        const int mtiles = (M + kBM - 1) / kBM;
-        units += make_schedule(gp, mtiles * ntile, sms, single);
-        const int rem = mtiles * ntile - gp.full;
-        if (rem > 0) {
-            const size_t pn = (size_t)rem * gp.q * kBM * bn;
-            if (g->d_tcpart.n < pn) g->d_tcpart.alloc(ctx, pn);
-            gp.P = g->d_tcpart.p;
-            post.push_back({k, rem});
+        if (it.Y) {
+            const bool bem = is_bem(g);
+            gp.rows = TcRows{n,
+                             bem ? n : g->n_atoms,
+                             g->n_types,
+                             it.d_freq,
+                             bem ? nullptr : g->d_type.p,
+                             g->d_dq.p,
+                             g->d_frac.p,
+                             g->d_inv_alpha.p,
+                             it.X,
+                             it.Y};
         }
+        L.tiles += (M + kBM - 1) / kBM * ntile;
         bn_max = std::max(bn_max, (bn + 31) / 32 * 32);
         if (!g->d_tc_err.p) throw Error(PLX_ERR_CUDA, "tensor-core error word missing");
         gp.err = g->d_tc_err.p;
     }
     L.bn_max = bn_max;
+    const int ctas = make_schedule(L, sms);
+    const int split = L.tiles - L.full;
+    if (split > 0) {
+        plx_geom *g0 = items[order[0]].g;
+        const size_t pn = (size_t)(split + ctas - L.full) * kBM * bn_max;
+        if (g0->d_tcpart.n < pn) g0->d_tcpart.alloc(ctx, pn);
+        L.P = g0->d_tcpart.p;
+    }
     L.stages = std::min(8, kSmemBudget / tc_stage_bytes(bn_max, nprod));
     const int smem = L.stages * tc_stage_bytes(bn_max, nprod) + 1024 /* align */ + 256 /* barriers */;
     auto kern = nprod == 1 ? tc_contract_kernel<1> : tc_contract_kernel<3>;
     once_per_device(reinterpret_cast<const void *>(kern), ctx->device, [&] {
         PLX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     });
-    kern<<<units, 128, smem, ctx->stream>>>(L);
+    kern<<<ctas, kThreadsTc, smem, ctx->stream>>>(L);
     ctx->launches++;
     PLX_CHECK_CUDA(cudaGetLastError());
-    for (const Post &q : post) {
-        const TcGroup &gp = L.grp[q.gi];
-        reduce_pieces<<<dim3(q.rem, (gp.bn + 31) / 32), kBM, 0, ctx->stream>>>(gp.M, gp.R, gp.bn, gp.full, gp.ctiles, gp.q,
-                                                                      gp.P, gp.S);
+    if (split > 0) {
+        reduce_pieces<<<dim3(split, n_blocks(bn_max, kRedCols)), kBM, 0, ctx->stream>>>(L);
         ctx->launches++;
     }
     PLX_CHECK_CUDA(cudaGetLastError());
 }
 
+TcColumns tc_column_buffers(plx_geom *g, int count) {
+    // rows for every column tiling of up to `count` columns (a tile pads to 16 columns,
+    // at most R / 256 + 1 tiles); the padding along k stays zero, rows past the batch
+    // feed columns of the product that are not stored
+    const size_t rows = 2 * (size_t)count + 16 * ((2 * (size_t)count + 255) / 256);
+    const size_t need = rows * g->ldk;
+    if (g->d_Xh.n < need) {
+        g->d_Xh.alloc(g->ctx, need);
+        g->d_Xl.alloc(g->ctx, need);
+        PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Xh.p, 0, need * 2, g->ctx->stream));
+        PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Xl.p, 0, need * 2, g->ctx->stream));
+    }
+    return TcColumns{g->d_Xh.p, g->d_Xl.p, g->ldk};
+}
+
+TcColumns tc_presplit(plx_geom *g, int count) {
+    if (tc_folds_operator(g))
+        build_a_split(g);
+    else
+        build_t_split(g);
+    return tc_column_buffers(g, count);
+}
+
 void tc_contract(plx_geom *g, int count, const double *X, double *S, int nprod, bool folded) {
-    tc_contract_group({TcItem{g, count, X, S, nprod, folded}});
+    tc_contract_group({TcItem{g, count, X, S, nprod, folded, nullptr, nullptr, false}});
 }
 
 int tc_error(plx_geom *g) {
