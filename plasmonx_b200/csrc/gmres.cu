@@ -252,30 +252,15 @@ __global__ void dots_finish(int nchunk, int ni, int i0, const int32_t *__restric
 // W[k] -= sum_{ii} V_{i0+ii}[c] h[k][ii]   (sign = -1), or X[c] += ... (sign = +1,
 // target indexed by column instead of compact position when by_col != 0).
 //
-// A block owns 256 / G rows of one column; its G groups of threads take every G-th
-// basis vector each (loads of a batch of them in flight together) and the groups'
-// sums are added in order.  G = 4 up to 16,384 unknowns, where one thread per row
-// leaves the chip idle whenever few columns are active (2,800 unknowns, 4 columns:
-// 44 CTAs, 36 us a launch, now 10.3 us; 893 unknowns, 61 columns 27 -> 15 us), and
-// 1 above, where a thread per row suffices.  G depends on n and ni alone, so a
-// column's sums do not depend on its batch.
-//
 // FIN: `h` holds the projections' chunk partials [k][ndot][ni], which every block
 // sums itself (up to four chunks: a launch less); the first block of a column also
-// adds them to H.  npart (optional): the sum of squares of the block's new rows.
+// adds them to H.
 constexpr int kCombineFin = 4;
-template <typename VT, int G, bool FIN>
-__global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int hld, int hoff,
-                                                    const int32_t *__restrict__ act,
-                                                    VT *const *__restrict__ slabs,
-                                                    const double2 *__restrict__ h, int ndot, double sign,
-                                                    double *__restrict__ Y, int by_col, double *__restrict__ npart,
-                                                    double2 *__restrict__ Hcol, int hstride, int accumulate) {
-    constexpr int RB = kThreads / G;
-    extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
-    __shared__ double2 red[G > 1 ? kThreads : 1];
-    const VT **col = reinterpret_cast<const VT **>(sh + ni);
-    const int k = blockIdx.y, c = act[k];
+template <typename VT, bool FIN>
+__device__ __forceinline__ void combine_setup(int n, int i0, int ni, int hld, int hoff, int k, int c,
+                                              VT *const *__restrict__ slabs, const double2 *__restrict__ h, int ndot,
+                                              double2 *__restrict__ Hcol, int hstride, int accumulate, double2 *sh,
+                                              const VT **col) {
     for (int t = threadIdx.x; t < ni; t += blockDim.x) {
         double2 v;
         if (FIN) {
@@ -296,6 +281,101 @@ __global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int h
         col[t] = slabs[i0 + t] + (int64_t)c * 2 * n;
     }
     __syncthreads();
+}
+
+// Real and imaginary part of v h, and of conj(v) w, with the roundings the sums of the
+// plain form have always had (one product rounded, the other fused): near the attainable
+// accuracy its stopping test turns on the last bits of the iterate, so kernels that
+// replace one another keep them, whatever the compiler would contract.  `whole`: the
+// vector is one of the leading groups of eight, whose imaginary parts fuse vi h.x.
+__device__ __forceinline__ double2 prod(double vr, double vi, double2 h, bool whole) {
+    return make_double2(fma(vr, h.x, -__dmul_rn(vi, h.y)), whole ? fma(vi, h.x, __dmul_rn(vr, h.y))
+                                                                 : fma(vr, h.y, __dmul_rn(vi, h.x)));
+}
+__device__ __forceinline__ double2 conj_prod(double vr, double vi, double wr, double wi) {
+    return make_double2(fma(vr, wr, __dmul_rn(vi, wi)), fma(vr, wi, -__dmul_rn(vi, wr)));
+}
+
+// The FP64 basis (the plain form): every row is one chain over ii in ascending order.
+// A block owns 32 rows: all 256 threads load 32 vectors of them and leave their
+// products in shared memory, the next 32 vectors in flight, and two warps (re, im; a
+// lane a row) add them in order; a thread per row and all its loads left 44 CTAs at 2,800 unknowns and 4 columns (36 us a launch, now 12.6 us; 893
+// unknowns, 61 columns 27 -> 19 us).
+constexpr int kChainRows = 32, kChainVec = 32;
+template <bool FIN>
+__global__ void __launch_bounds__(kThreads) combine_chain(int n, int i0, int ni, int hld, int hoff,
+                                                          const int32_t *__restrict__ act,
+                                                          double *const *__restrict__ slabs,
+                                                          const double2 *__restrict__ h, int ndot, double sign,
+                                                          double *__restrict__ Y, int by_col,
+                                                          double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
+    __shared__ double ps[2][kChainVec][2][kChainRows];
+    const double **col = reinterpret_cast<const double **>(sh + ni);
+    const int k = blockIdx.y, c = act[k];
+    combine_setup<double, FIN>(n, i0, ni, hld, hoff, k, c, slabs, h, ndot, Hcol, hstride, accumulate, sh, col);
+    const int row = threadIdx.x % kChainRows, grp = threadIdx.x / kChainRows;
+    const int r = blockIdx.x * kChainRows + row;
+    const int rr = min(r, n - 1);                         // a valid row; its sum is not stored
+    constexpr int G = kThreads / kChainRows, L = kChainVec / G;          // 8 groups, 4 vectors a thread
+    double vr[L], vi[L];
+    auto load = [&](int ii) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int t = ii + grp * L + q;
+            vr[q] = t < ni ? col[t][rr] : 0.0;
+            vi[q] = t < ni ? col[t][n + rr] : 0.0;
+        }
+    };
+    double sum = 0.0;                                     // groups 0 and 1: re, im of the row
+    load(0);
+    int buf = 0;
+    for (int ii = 0; ii < ni; ii += kChainVec, buf ^= 1) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int t = ii + grp * L + q;
+            const double2 p = prod(vr[q], vi[q], t < ni ? sh[t] : make_double2(0.0, 0.0), t < (ni & ~7));
+            ps[buf][grp * L + q][0][row] = p.x;
+            ps[buf][grp * L + q][1][row] = p.y;
+        }
+        if (ii + kChainVec < ni) load(ii + kChainVec);
+        __syncthreads();
+        const int m = min(kChainVec, ni - ii);
+        if (grp < 2) {
+            if (m == kChainVec) {
+#pragma unroll
+                for (int q = 0; q < kChainVec; ++q) sum += ps[buf][q][grp][row];
+            } else {
+                for (int q = 0; q < m; ++q) sum += ps[buf][q][grp][row];
+            }
+        }
+    }
+    if (r >= n || grp >= 2) return;
+    double *y = Y + (int64_t)(by_col ? c : k) * 2 * n + grp * n;
+    y[r] += sign * sum;
+}
+
+// The FP32 basis of an inner solve: a block owns 256 / G rows of one column; its G
+// groups of threads take every G-th basis vector each (loads of a batch of them in
+// flight together) and the groups' sums are added in order.  G = 4 up to 16,384
+// unknowns, where one thread per row leaves the chip idle whenever few columns are
+// active, and 1 above, where a thread per row suffices.  G depends on n and ni alone,
+// so a column's sums do not depend on its batch.  npart (optional): the sum of squares
+// of the block's new rows.  13,528 unknowns, up to 21 columns and 256 vectors: 40 ->
+// 22 us a launch on average.
+template <int G, bool FIN>
+__global__ void __launch_bounds__(kThreads) combine_inner(int n, int i0, int ni, int hld, int hoff,
+                                                          const int32_t *__restrict__ act,
+                                                          float *const *__restrict__ slabs,
+                                                          const double2 *__restrict__ h, int ndot, double sign,
+                                                          double *__restrict__ Y, int by_col, double *__restrict__ npart,
+                                                          double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    constexpr int RB = kThreads / G;
+    extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
+    __shared__ double2 red[G > 1 ? kThreads : 1];
+    const float **col = reinterpret_cast<const float **>(sh + ni);
+    const int k = blockIdx.y, c = act[k];
+    combine_setup<float, FIN>(n, i0, ni, hld, hoff, k, c, slabs, h, ndot, Hcol, hstride, accumulate, sh, col);
     const int row = threadIdx.x % RB, grp = threadIdx.x / RB;
     const int r = blockIdx.x * RB + row;
     const bool in = r < n;
@@ -304,7 +384,7 @@ __global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int h
     constexpr int kBatch = 8;                             // basis vectors whose loads are in flight together
     int ii = grp;
     for (; ii + (kBatch - 1) * G < ni; ii += kBatch * G) {
-        VT vr[kBatch], vi[kBatch];
+        float vr[kBatch], vi[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; ++q) {
             vr[q] = col[ii + q * G][rr];
@@ -318,7 +398,7 @@ __global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int h
         }
     }
     for (; ii < ni; ii += G) {
-        const VT *v = col[ii];
+        const float *v = col[ii];
         const double2 hh = sh[ii];
         const double vr = (double)v[rr], vi = (double)v[n + rr];
         ar += vr * hh.x - vi * hh.y;
@@ -352,24 +432,28 @@ __global__ void __launch_bounds__(kThreads) combine(int n, int i0, int ni, int h
 
 // Modified Gram-Schmidt of W[k] against V_0..V_j in one launch (n <= 4,096): one
 // block per column keeps its rows of W in registers and walks the basis, the next
-// vector's loads in flight during the block reduction of the current one.  The
-// three short launches per vector it replaces (300 vectors over the first 24
-// steps) took 2.3-2.8 us each plus their gaps; now 12.9 us a step on average at 893 unknowns.
-constexpr int kMgsThreads = 512;
-template <int RPT>
-__global__ void __launch_bounds__(kMgsThreads) mgs_column(int n, int j, const int32_t *__restrict__ act,
-                                                          double *const *__restrict__ slabs, double *__restrict__ W,
-                                                          double2 *__restrict__ Hcol, int hstride,
-                                                          double *__restrict__ npart) {
-    __shared__ double2 red[2][kMgsThreads / 32];
+// vector's loads in flight during the block reduction of the current one.  256
+// threads take kDotRows rows, as in dots_partial, and the sums run in its order
+// (a thread's rows, the warp's lanes, the warps, the chunks), so both give the same
+// bits.  The three short launches per vector it replaces (300 vectors over the first
+// 24 steps) took 2.3-2.8 us each plus their gaps; now 11.7 us a step on average at 893
+// unknowns.
+template <int CHUNKS>
+__global__ void __launch_bounds__(CHUNKS * kThreads) mgs_column(int n, int j, const int32_t *__restrict__ act,
+                                                                double *const *__restrict__ slabs,
+                                                                double *__restrict__ W, double2 *__restrict__ Hcol,
+                                                                int hstride) {
+    constexpr int kWarps = kThreads / 32;
+    __shared__ double2 red[2][CHUNKS][kWarps];
     const int k = blockIdx.x, c = act[k];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunk = threadIdx.x / kThreads, tid = threadIdx.x % kThreads;
+    const int warp = tid >> 5, lane = tid & 31, r0 = chunk * kDotRows + tid;
     double *w = W + (int64_t)k * 2 * n;
-    double wr[RPT], wi[RPT], vr[RPT], vi[RPT];
+    double wr[kDotPT], wi[kDotPT], vr[kDotPT], vi[kDotPT];
     auto load = [&](const double *src, double *re, double *im) {
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-            const int r = threadIdx.x + q * kMgsThreads;
+        for (int q = 0; q < kDotPT; ++q) {
+            const int r = r0 + q * kThreads;
             re[q] = r < n ? src[r] : 0.0;
             im[q] = r < n ? src[n + r] : 0.0;
         }
@@ -377,60 +461,71 @@ __global__ void __launch_bounds__(kMgsThreads) mgs_column(int n, int j, const in
     load(w, wr, wi);
     load(slabs[0] + (int64_t)c * 2 * n, vr, vi);
     for (int i = 0; i <= j; ++i) {
-        double re = 0.0, im = 0.0;                        // conj(v) . w
+        double re = 0.0, im = 0.0;
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-            re += vr[q] * wr[q] + vi[q] * wi[q];
-            im += vr[q] * wi[q] - vi[q] * wr[q];
+        for (int q = 0; q < kDotPT; ++q) {
+            const double2 p = conj_prod(vr[q], vi[q], wr[q], wi[q]);
+            re += p.x;
+            im += p.y;
         }
-        double nr[RPT], ni[RPT];
+        double nr[kDotPT], ni[kDotPT];
         if (i < j) load(slabs[i + 1] + (int64_t)c * 2 * n, nr, ni);
         re = warp_sum(re);
         im = warp_sum(im);
-        if (lane == 0) red[i & 1][warp] = make_double2(re, im);
+        if (lane == 0) red[i & 1][chunk][warp] = make_double2(re, im);
         __syncthreads();
+        double2 p = make_double2(0.0, 0.0);               // lane q: chunk q's sum over its warps
+        if (lane < CHUNKS)
+#pragma unroll
+            for (int t = 0; t < kWarps; ++t) {
+                p.x += red[i & 1][lane][t].x;
+                p.y += red[i & 1][lane][t].y;
+            }
         double2 h = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int t = 0; t < kMgsThreads / 32; ++t) {
-            h.x += red[i & 1][t].x;
-            h.y += red[i & 1][t].y;
+        for (int q = 0; q < CHUNKS; ++q) {
+            h.x += __shfl_sync(0xffffffffu, p.x, q);
+            h.y += __shfl_sync(0xffffffffu, p.y, q);
         }
         if (threadIdx.x == 0) Hcol[(int64_t)c * hstride + i] = h;
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-            wr[q] -= vr[q] * h.x - vi[q] * h.y;
-            wi[q] -= vr[q] * h.y + vi[q] * h.x;
+        for (int q = 0; q < kDotPT; ++q) {
+            const double2 p = prod(vr[q], vi[q], h, false);
+            wr[q] -= p.x;
+            wi[q] -= p.y;
             if (i < j) {
                 vr[q] = nr[q];
                 vi[q] = ni[q];
             }
         }
     }
-    double sq = 0.0, dummy = 0.0;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-        const int r = threadIdx.x + q * kMgsThreads;
+    for (int q = 0; q < kDotPT; ++q) {
+        const int r = r0 + q * kThreads;
         if (r < n) {
             w[r] = wr[q];
             w[n + r] = wi[q];
-            sq += wr[q] * wr[q] + wi[q] * wi[q];
         }
     }
-    block_sum2(sq, dummy);
-    if (threadIdx.x == 0) npart[k] = sq;
 }
 
 // ||W[k]||_2 (dznrm2): partial sums of squares per chunk.
-__global__ void norm_partial(int n, const double *__restrict__ W, double *__restrict__ part) {
-    int k = blockIdx.y;
-    const double *w = W + (int64_t)k * 2 * n;
-    int r0 = blockIdx.x * kRows, rn = min(kRows, n - r0);
+// Sum of squares of one chunk by a block of kThreads; valid in thread 0.
+__device__ __forceinline__ double norm_chunk(int n, const double *__restrict__ w, int chunk) {
+    int r0 = chunk * kRows, rn = min(kRows, n - r0);
     double s = 0.0, dummy = 0.0;
-    for (int t = threadIdx.x; t < rn; t += blockDim.x) {
+    for (int t = threadIdx.x; t < rn; t += kThreads) {
         double a = w[r0 + t], b = w[n + r0 + t];
         s += a * a + b * b;
     }
     block_sum2(s, dummy);
+    return s;
+}
+
+__global__ void __launch_bounds__(kThreads) norm_partial(int n, const double *__restrict__ W,
+                                                         double *__restrict__ part) {
+    const int k = blockIdx.y;
+    const double s = norm_chunk(n, W + (int64_t)k * 2 * n, blockIdx.x);
     if (threadIdx.x == 0) part[(int64_t)k * gridDim.x + blockIdx.x] = s;
 }
 
@@ -463,10 +558,12 @@ __global__ void start_vectors(int n, const int32_t *__restrict__ act, const doub
 
 __device__ __forceinline__ double cabs_(double2 a) { return hypot(a.x, a.y); }
 
+// x' = c x + s y, y' = c y - conj(s) x, with fixed roundings (see prod).
 __device__ __forceinline__ void zrot_(double2 &x, double2 &y, double c, double2 s) {
-    double2 nx = make_double2(c * x.x + (s.x * y.x - s.y * y.y), c * x.y + (s.x * y.y + s.y * y.x));
-    // y' = c y - conj(s) x
-    double2 ny = make_double2(c * y.x - (s.x * x.x + s.y * x.y), c * y.y - (s.x * x.y - s.y * x.x));
+    const double2 nx = make_double2(fma(c, x.x, fma(s.x, y.x, -__dmul_rn(s.y, y.y))),
+                                    fma(c, x.y, fma(s.x, y.y, __dmul_rn(s.y, y.x))));
+    const double2 ny = make_double2(fma(c, y.x, fma(-s.x, x.x, -__dmul_rn(s.y, x.y))),
+                                    fma(c, y.y, fma(-s.x, x.y, __dmul_rn(s.y, x.x))));
     x = nx;
     y = ny;
 }
@@ -483,16 +580,21 @@ __device__ __forceinline__ double2 shfl_up2(double2 v, int o) {
 //
 // The j earlier rotations form a chain: with a_0 = h_0 the i-th rotation gives
 // h_i' = c_i a_i + s_i h_{i+1} and passes on a_{i+1} = c_i h_{i+1} - conj(s_i) a_i.
-// One thread walking it pays a dependent global load and ~6 FP64 latencies per
-// rotation (2.1 us per 16 rotations).  The chain is a composition of maps
-// a -> p a + q, so a warp takes 32 rotations at a time (coalesced loads) and
-// composes them with a 5-step scan; |p| <= 1 throughout, so the composition is
-// as stable as the chain.  The result depends on j alone, not on the batch.
-// Latency bound; per launch, before -> after: 81 -> 6.1 us at 61 columns and 130
-// steps on average, 94 -> 8.5 us at 4 columns and 360 steps.
+// One thread walking it in global memory paid a dependent load per rotation (81 us
+// at 130 rotations, 94 us at 360).  A warp loads 32 rotations at a time, coalesced and
+// a tile ahead.  SCAN (inner solves): the chain is a composition of maps a -> p a + q,
+// composed with a 5-step scan; |p| <= 1 throughout, so that is as stable as the
+// chain.  Otherwise (the plain form) every lane walks the chain in its order with
+// the tile's values from shared memory, which keeps the chain's bits.
+// The result depends on j alone, not on the batch.
+struct Rotation {
+    double2 s, h;
+    double c;
+};
+template <bool SCAN>
 __device__ void givens(int k, int c, int lane, int j, double norm, double2 *const *__restrict__ Hcols, int hstride,
                        double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g, int gstride,
-                       int cstride, double *__restrict__ resid) {
+                       int cstride, double *__restrict__ resid, Rotation *rot) {
     double2 *h = Hcols[j] + (int64_t)c * hstride;
     double *csc = cs + (int64_t)c * cstride;
     double2 *snc = sn + (int64_t)c * cstride;
@@ -504,29 +606,46 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *cons
     double2 hn = lane < j ? h[lane + 1] : make_double2(0.0, 0.0);
     for (int i0 = 0; i0 < j; i0 += 32) {
         const int i = i0 + lane, in = i + 32;
-        // the next tile's loads, in flight during this tile's scan
+        // the next tile's loads, in flight during this tile's chain
         const double cin = in < j ? csc[in] : 1.0;
         const double2 sin_ = in < j ? snc[in] : make_double2(0.0, 0.0);
         const double2 hnn = in < j ? h[in + 1] : make_double2(0.0, 0.0);
-        double2 p = i < j ? make_double2(-si.x, si.y) : make_double2(1.0, 0.0);      // -conj(s)
-        double2 q = i < j ? make_double2(ci * hn.x, ci * hn.y) : make_double2(0.0, 0.0);
+        if (SCAN) {
+            double2 p = i < j ? make_double2(-si.x, si.y) : make_double2(1.0, 0.0);      // -conj(s)
+            double2 q = i < j ? make_double2(ci * hn.x, ci * hn.y) : make_double2(0.0, 0.0);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double2 pp = shfl_up2(p, o), qq = shfl_up2(q, o);
-            if (lane >= o) {
-                const double2 t = cmul(p, qq);
-                q.x += t.x;
-                q.y += t.y;
-                p = cmul(p, pp);
+            for (int o = 1; o < 32; o <<= 1) {
+                const double2 pp = shfl_up2(p, o), qq = shfl_up2(q, o);
+                if (lane >= o) {
+                    const double2 t = cmul(p, qq);
+                    q.x += t.x;
+                    q.y += t.y;
+                    p = cmul(p, pp);
+                }
             }
+            const double2 t = cmul(p, a);
+            const double2 out = make_double2(t.x + q.x, t.y + q.y);      // a after this lane's rotation
+            double2 ai = shfl_up2(out, 1);                               // a before it
+            if (lane == 0) ai = a;
+            if (i < j)
+                h[i] = make_double2(ci * ai.x + (si.x * hn.x - si.y * hn.y), ci * ai.y + (si.x * hn.y + si.y * hn.x));
+            a = shfl2(out, 31);
+        } else {
+            __syncwarp();
+            rot[lane] = Rotation{si, hn, ci};
+            __syncwarp();
+            const int m = min(32, j - i0);
+            double2 mine = make_double2(0.0, 0.0);
+#pragma unroll 8
+            for (int t = 0; t < m; ++t) {
+                const Rotation r = rot[t];
+                double2 x = a, y = r.h;
+                zrot_(x, y, r.c, r.s);
+                if (lane == t) mine = x;
+                a = y;
+            }
+            if (i < j) h[i] = mine;
         }
-        const double2 t = cmul(p, a);
-        const double2 out = make_double2(t.x + q.x, t.y + q.y);      // a after this lane's rotation
-        double2 ai = shfl_up2(out, 1);                               // a before it
-        if (lane == 0) ai = a;
-        if (i < j)
-            h[i] = make_double2(ci * ai.x + (si.x * hn.x - si.y * hn.y), ci * ai.y + (si.x * hn.y + si.y * hn.x));
-        a = shfl2(out, 31);
         ci = cin;
         si = sin_;
         hn = hnn;
@@ -560,31 +679,47 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *cons
     resid[k] = cabs_(g1);
 }
 
-// The end of an Arnoldi step: h_{j+1,j} = ||W[k]|| from the partial sums of squares,
-// v_{j+1}[c] = W[k] / h_{j+1,j} (zero when the norm is zero, as the reference leaves
-// the zero-filled column untouched), the Givens update of H's column j (one warp of
-// a column's first block), and the input X[k] = P v_{j+1} of the next product.
-// One launch in place of norm sum, scaling, Givens, gather, preconditioner and the
-// tensor-core split.
+// The end of an Arnoldi step: h_{j+1,j} = ||W[k]||, v_{j+1}[c] = W[k] / h_{j+1,j} (zero
+// when the norm is zero, as the reference leaves the zero-filled column untouched),
+// the Givens update of H's column j (one warp of a column's first block), and the
+// input X[k] = P v_{j+1} of the next product, split for the tensor cores.  One launch
+// in place of norm, scaling, Givens, gather, preconditioner and split.
+//
+// The norm: nparts partial sums of squares npart -- added by the block in the inner
+// solves (VT float), in their order in the plain form -- or with nparts = 0 the chunks
+// of W themselves (up to kNormChunks, in norm_partial's order).
+constexpr int kNormChunks = 2;
 template <typename VT>
-__global__ void __launch_bounds__(256) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
-                                                        const double *__restrict__ npart,
-                                                        const double *__restrict__ W, VT *__restrict__ slab_next,
-                                                        const double *__restrict__ P, double *__restrict__ X,
-                                                        TcColumns sp, double2 *const *__restrict__ Hcols, int hstride,
-                                                        double *__restrict__ cs, double2 *__restrict__ sn,
-                                                        double2 *__restrict__ g, int gstride, int cstride,
-                                                        double *__restrict__ resid) {
+__global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
+                                                             const double *__restrict__ npart,
+                                                             const double *__restrict__ W, VT *__restrict__ slab_next,
+                                                             const double *__restrict__ P, double *__restrict__ X,
+                                                             TcColumns sp, double2 *const *__restrict__ Hcols,
+                                                             int hstride, double *__restrict__ cs,
+                                                             double2 *__restrict__ sn, double2 *__restrict__ g,
+                                                             int gstride, int cstride, double *__restrict__ resid) {
+    constexpr bool kInner = sizeof(VT) == 4;
     __shared__ double total;
+    __shared__ Rotation rot[kInner ? 1 : 32];
     const int k = blockIdx.y, c = act[k];
-    double s = 0.0, dummy = 0.0;
-    for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += npart[(int64_t)k * nparts + b];
-    block_sum2(s, dummy);
+    const double *w = W + (int64_t)k * 2 * n;
+    double s = 0.0;
+    if (kInner) {
+        double dummy = 0.0;
+        for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += npart[(int64_t)k * nparts + b];
+        block_sum2(s, dummy);
+    } else if (nparts == 0) {
+        for (int q = 0; q * kRows < n; ++q) {
+            const double p = norm_chunk(n, w, q);
+            s += p;
+        }
+    } else if (threadIdx.x == 0) {
+        for (int b = 0; b < nparts; ++b) s += npart[(int64_t)k * nparts + b];
+    }
     if (threadIdx.x == 0) total = sqrt(s);
     __syncthreads();
     s = total;
     const double inv = s != 0.0 ? 1.0 / s : 0.0;
-    const double *w = W + (int64_t)k * 2 * n;
     VT *v = slab_next + (int64_t)c * 2 * n;
     const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
     double *x = X + (int64_t)k * 2 * n;
@@ -603,19 +738,26 @@ __global__ void __launch_bounds__(256) normalize_givens(int n, int j, const int3
         if (sp.hi) split_column(sp, k, r, re, im);
     }
     if (blockIdx.x == 0 && threadIdx.x < 32)
-        givens(k, c, threadIdx.x, j, s, Hcols, hstride, cs, sn, g, gstride, cstride, resid);
+        givens<kInner>(k, c, threadIdx.x, j, s, Hcols, hstride, cs, sn, g, gstride, cstride, resid, rot);
 }
 
 // y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
 // per triggered column, y stored compactly [k][j+1].  Back substitution in
 // blocks of 32 columns: the 32 x 32 triangle is staged in shared memory and
 // solved by one warp in registers, then the whole block subtracts the 32
-// solved unknowns from the rows above (each row in descending column order,
-// as the unblocked substitution does) while it stages the next triangle.  One
+// solved unknowns from the rows above (each row in descending column order and
+// with the roundings of the unblocked substitution) while it stages the next triangle.  One
 // warp reading the columns of R from global memory, one dependent load per
 // unknown, took 326 us at 61-130 unknowns and 1,125 us at 700; now 100 and
 // 333 us (latency bound: ~32 dependent multiplications a block).
 constexpr int kTriB = 32;
+
+// n / d rounded once from id = 1 / d rounded once (Markstein's theorem: the remainder
+// of the first estimate is exact and its correction rounds correctly).
+__device__ __forceinline__ double quotient(double n, double d, double id) {
+    const double q = n * id;
+    return fma(fma(-q, d, n), id, q);
+}
 
 __global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t *__restrict__ act,
                                                  double2 *const *__restrict__ Hcols, int hstride,
@@ -644,13 +786,14 @@ __global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t
             const int l = threadIdx.x;
             double2 v = l < nb ? ys[b0 + l] : make_double2(0.0, 0.0);
             const double2 r = l < nb ? tri[l][l] : make_double2(1.0, 0.0);
-            const double d = r.x * r.x + r.y * r.y;
-            const double2 ri = make_double2(r.x / d, -r.y / d);
+            const double d = fma(r.x, r.x, __dmul_rn(r.y, r.y)), id = 1.0 / d;
             for (int i = nb - 1; i >= 0; --i) {
-                const double2 yi = shfl2(cmul(v, ri), i);
+                const double2 yi = shfl2(make_double2(quotient(fma(v.x, r.x, __dmul_rn(v.y, r.y)), d, id),
+                                                      quotient(fma(v.y, r.x, -__dmul_rn(v.x, r.y)), d, id)),
+                                         i);
                 if (l == i) v = yi;
                 if (l < i) {
-                    const double2 p = cmul(tri[i][l], yi);
+                    const double2 p = prod(tri[i][l].x, tri[i][l].y, yi, false);
                     v.x -= p.x;
                     v.y -= p.y;
                 }
@@ -669,7 +812,7 @@ __global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         if (i0 - 1 - q >= 0) {
-                            const double2 p = cmul(r[q], ys[b0 + i0 - 1 - q]);
+                            const double2 p = prod(r[q].x, r[q].y, ys[b0 + i0 - 1 - q], false);
                             v.x -= p.x;
                             v.y -= p.y;
                         }
@@ -723,12 +866,13 @@ __global__ void scale_cols(int n, const int32_t *__restrict__ idx, const double 
 
 int grid_rows(int64_t n2) { return (int)std::min<int64_t>(n_blocks(n2, 256), 1024); }
 
-// Groups of threads of combine() (see there).
+// Groups of threads of combine_inner() (see there).
 int combine_groups(int n, int ni) { return n <= 16384 && ni >= 16 ? 4 : 1; }
 int combine_blocks(int n, int ni) { return n_blocks(n, kThreads / combine_groups(n, ni)); }
 
-// combine() over at most kCombine basis vectors per launch (shared-memory bound).
-// ndot > 0: h holds chunk partials (FIN), for ni <= kCombine.  npart as in combine().
+// The basis combination over at most kCombine basis vectors per launch
+// (shared-memory bound).  ndot > 0: h holds chunk partials (FIN), for ni <= kCombine.
+// npart: norm partials of the last launch (FP32 basis).
 constexpr int kCombine = 1024;
 template <typename VT>
 int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const int32_t *act,
@@ -736,21 +880,27 @@ int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const
                         int ndot = 0, double *npart = nullptr, double2 *Hcol = nullptr, int hstride = 0,
                         int accumulate = 0) {
     int64_t launches = 0;
-    const int G = combine_groups(n, ni);
     for (int c0 = 0; c0 < ni; c0 += kCombine) {
         int cn = std::min(kCombine, ni - c0);
         // h is [count][ni]; pass the row stride through a shifted view per chunk
-        const dim3 grid(n_blocks(n, kThreads / G), count);
         const size_t smem = cn * (sizeof(double2) + sizeof(VT *));
-        double *np = c0 + cn == ni ? npart : nullptr;
-#define PLX_COMBINE(GG, FIN)                                                                                      \
-    combine<VT, GG, FIN><<<grid, kThreads, smem, st>>>(n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, \
-                                                       np, Hcol, hstride, accumulate)
-        if (G == 4 && ndot) PLX_COMBINE(4, true);
-        else if (G == 4) PLX_COMBINE(4, false);
-        else if (ndot) PLX_COMBINE(1, true);
-        else PLX_COMBINE(1, false);
+        if constexpr (std::is_same<VT, double>::value) {
+            const dim3 grid(n_blocks(n, kChainRows), count);
+            (ndot ? combine_chain<true> : combine_chain<false>)<<<grid, kThreads, smem, st>>>(
+                n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, Hcol, hstride, accumulate);
+        } else {
+            const int G = combine_groups(n, ni);
+            const dim3 grid(n_blocks(n, kThreads / G), count);
+            double *np = c0 + cn == ni ? npart : nullptr;
+#define PLX_COMBINE(GG, FIN)                                                                                    \
+    combine_inner<GG, FIN><<<grid, kThreads, smem, st>>>(n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, \
+                                                         np, Hcol, hstride, accumulate)
+            if (G == 4 && ndot) PLX_COMBINE(4, true);
+            else if (G == 4) PLX_COMBINE(4, false);
+            else if (ndot) PLX_COMBINE(1, true);
+            else PLX_COMBINE(1, false);
 #undef PLX_COMBINE
+        }
         ++launches;
     }
     return launches;
@@ -794,6 +944,8 @@ class GmresRun final : public GmresStepper {
         if ((size_t)(m_ + 1) * sizeof(double2) > 200 * 1024) throw Error(PLX_ERR_ARG, "GMRES dimension above 12800");
         once_per_device(reinterpret_cast<const void *>(tri_solve), ctx_->device, [] {
             PLX_CHECK_CUDA(cudaFuncSetAttribute(tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024));
+            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024));
         });
         hstride_ = m_ + 1;   // rows of an H column (0..m)
         d_act_.alloc(ctx_, C_);
@@ -884,7 +1036,7 @@ class GmresRun final : public GmresStepper {
         if (part_.n < need) part_.alloc(ctx_, std::max(need, part_.n * 2));
         int nparts = 0;
         // W -= V V^H W over basis vectors i0..i1-1, the coefficients into (or added to) H's
-        // column j; the last projection of the step leaves the norm partials
+        // column j; with an FP32 basis the last projection leaves the norm partials
         auto project = [&](int i0, int i1, int accumulate, bool last) {
             const int ni = i1 - i0;
             if (ni >= 8) {
@@ -909,11 +1061,19 @@ class GmresRun final : public GmresStepper {
         };
         prof_begin(ctx_);
         if (j + 1 < 25 && !rq_.inner) {
-            if (!mgs_fused(na, j, nparts))
-                for (int i = 0; i <= j; ++i) project(i, i + 1, 0, i == j);   // modified Gram-Schmidt
+            if (!mgs_fused(na, j))
+                for (int i = 0; i <= j; ++i) project(i, i + 1, 0, false);    // modified Gram-Schmidt
         } else {
             project(0, j + 1, 0, rq_.single_pass);                    // classical GS ...
             if (!rq_.single_pass) project(0, j + 1, 1, true);         // ... and re-orthogonalise
+        }
+        if (std::is_same<VT, double>::value) {
+            nparts = 0;
+            if (nchunk_ > kNormChunks) {
+                norm_partial<<<dim3(nchunk_, na), kThreads, 0, st_>>>(n, Wa_.p, nrm_part_.p);
+                ctx_->launches++;
+                nparts = nchunk_;
+            }
         }
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
         prof_begin(ctx_);
@@ -1006,19 +1166,16 @@ class GmresRun final : public GmresStepper {
 
   private:
     // modified Gram-Schmidt in one launch where a block holds a column (the FP64 basis)
-    bool mgs_fused(int na, int j, int &nparts) {
+    bool mgs_fused(int na, int j) {
         if constexpr (std::is_same<VT, double>::value) {
             const int n = g_->n_var;
-            if (n > 8 * kMgsThreads) return false;
-#define PLX_MGS(R) mgs_column<R><<<na, kMgsThreads, 0, st_>>>(n, j, d_act_.p, d_slabs_.p, Wa_.p, hcols_[j].p, hstride_, \
-                                                             nrm_part_.p)
-            if (n <= kMgsThreads) PLX_MGS(1);
-            else if (n <= 2 * kMgsThreads) PLX_MGS(2);
-            else if (n <= 4 * kMgsThreads) PLX_MGS(4);
-            else PLX_MGS(8);
+            if (n > 4 * kDotRows) return false;
+#define PLX_MGS(Q) mgs_column<Q><<<na, Q * kThreads, 0, st_>>>(n, j, d_act_.p, d_slabs_.p, Wa_.p, hcols_[j].p, hstride_)
+            if (n <= kDotRows) PLX_MGS(1);
+            else if (n <= 2 * kDotRows) PLX_MGS(2);
+            else PLX_MGS(4);
 #undef PLX_MGS
             ctx_->launches++;
-            nparts = 1;
             return true;
         }
         return false;
