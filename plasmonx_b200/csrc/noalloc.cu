@@ -50,11 +50,6 @@ double *scratch_for_device(int dev) {
     return g_scratch_ptr[dev];
 }
 
-template <int R>
-void launch_partial(dim3 grid, cudaStream_t st, int n, int kchunk, const double *X, const double *T, double *part) {
-    plx::skinny_partial<R><<<grid, plx::kSkinnyCols, 0, st>>>(n, kchunk, X, T, part);
-}
-
 }  // namespace
 
 extern "C" plx_status plx_contract_noalloc(plx_geom *g, int32_t count, const double *d_X, double *d_S) {
@@ -76,14 +71,7 @@ extern "C" plx_status plx_contract_noalloc(plx_geom *g, int32_t count, const dou
                                               std::to_string(kNoAllocScratchDoubles));
         double *part = scratch_for_device(ctx->device);
         cudaStream_t st = ctx->stream;
-        dim3 grid(plx::n_blocks(n, plx::kSkinnyCols), ks);
-        switch (count) {
-#define PLX_NA(RR) \
-    case RR: launch_partial<RR>(grid, st, n, kchunk, d_X, g->d_T.p, part); break;
-            PLX_NA(1) PLX_NA(2) PLX_NA(3) PLX_NA(4) PLX_NA(5) PLX_NA(6) PLX_NA(7) PLX_NA(8)
-            PLX_NA(9) PLX_NA(10) PLX_NA(11) PLX_NA(12) PLX_NA(13) PLX_NA(14) PLX_NA(15) PLX_NA(16)
-#undef PLX_NA
-        }
+        plx::launch_product_partial(st, count, n, ks, kchunk, d_X, g->d_T.p, part);
         plx::skinny_reduce<<<plx::n_blocks((int64_t)count * n, 256), 256, 0, st>>>(n, count, ks, part, d_S);
         ctx->launches += 2;
         PLX_CHECK_CUDA(cudaGetLastError());

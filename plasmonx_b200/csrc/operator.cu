@@ -18,97 +18,6 @@ namespace plx {
 namespace {
 
 // ---------------------------------------------------------------------------
-// S^T = X^T T, tiled (R > 16): 64 x 128 output tiles, 8 x 8 per thread (four
-// FMAs per shared-memory load, which keeps the FP64 pipe rather than shared
-// memory the limit), the next k-slab prefetched into registers while the
-// current one is multiplied.  Split over K in the SAME chunks as
-// skinny_partial and reduced by skinny_reduce, and every output element is
-// accumulated by one FMA chain in k order from zero, exactly as
-// skinny_partial does, so a column's result does not depend on the number of
-// columns in the batch.
-// ---------------------------------------------------------------------------
-constexpr int BM = 64, BN = 128, BK = 8, kTiledThreads = 128;
-
-__global__ void __launch_bounds__(kTiledThreads) tiled_partial(int R, int n, int kchunk,
-                                                               const double *__restrict__ Xt,
-                                                               const double *__restrict__ T,
-                                                               double *__restrict__ part) {
-    __shared__ double As[2][BM][BK + 1];
-    __shared__ double Bs[2][BK][BN];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;          // 16 x 8 threads
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-    const int kbeg = blockIdx.z * kchunk, kend = min(n, kbeg + kchunk);
-    constexpr int LA = BM * BK / kTiledThreads, LB = BK * BN / kTiledThreads;   // 4, 8
-    double ra[LA], rb[LB];
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < LA; ++q) {
-            const int e = threadIdx.x + q * kTiledThreads, r = e / BK, k = e % BK;
-            const int gr = row0 + r, gk = k0 + k;
-            ra[q] = (gr < R && gk < kend) ? Xt[(int64_t)gr * n + gk] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int e = threadIdx.x + q * kTiledThreads, k = e / BN, c = e % BN;
-            const int gk = k0 + k, gc = col0 + c;
-            rb[q] = (gk < kend && gc < n) ? T[(int64_t)gk * n + gc] : 0.0;
-        }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < LA; ++q) {
-            const int e = threadIdx.x + q * kTiledThreads;
-            As[buf][e / BK][e % BK] = ra[q];
-        }
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int e = threadIdx.x + q * kTiledThreads;
-            Bs[buf][e / BN][e % BN] = rb[q];
-        }
-    };
-    double acc[8][8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int v = 0; v < 8; ++v) acc[u][v] = 0.0;
-    if (kbeg < kend) {
-        load(kbeg);
-        store(0);
-    }
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        const bool more = k0 + BK < kend;
-        if (more) load(k0 + BK);
-        const int kn = min(BK, kend - k0);
-        for (int k = 0; k < kn; ++k) {
-            double a[8], b[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = As[buf][ty * 8 + u][k];
-#pragma unroll
-            for (int v = 0; v < 8; ++v) b[v] = Bs[buf][k][tx + 16 * v];
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-#pragma unroll
-                for (int v = 0; v < 8; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
-        }
-        if (more) store(buf ^ 1);
-        __syncthreads();
-        buf ^= 1;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int gr = row0 + ty * 8 + u;
-        if (gr >= R) continue;
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-            const int gc = col0 + tx + 16 * v;
-            if (gc < n) part[((int64_t)blockIdx.z * R + gr) * n + gc] = acc[u][v];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // S = T X generated on the fly (matrix-free), at most CB columns per launch:
 // one or several warps per target atom, the lanes over the source atoms.
 //
@@ -208,17 +117,24 @@ __global__ void __launch_bounds__(32 * kOtfWarps) otf_contract(int N, int wt, in
 }
 
 // ---------------------------------------------------------------------------
-// The same for many columns: the tiled product above with its T slab generated
-// in shared memory, split over source atoms and reduced by skinny_reduce.  Rows
+// The same for many columns: S^T = X^T T with T generated in shared memory 16
+// unknowns at a time, split over source atoms and reduced by skinny_reduce.  Rows
 // and columns run atom by atom (an atom's charge, then its three dipole
 // components), so a thread evaluates one pair of atoms and writes its 4 x 4
 // block: the slab's erf and exp are evaluated once per pair instead of once per
 // element.  BM rows of X^T a block (16, 32, 48 or 64): the fewest that hold the
-// batch, so that 42 rows do not run as 64.  Every output is one FMA chain over
-// the unknowns of a chunk in order, whatever BM.
-// Measured at 13,528 unknowns and 42 rows: 5,085 us element by element in 64
-// rows, now 1,429 us (average of four launches).
+// batch, so that 42 rows do not run as 64.  The products are FP64 matrix
+// instructions, each of the four warps 32 columns.  Every kFlush slabs (256 unknowns)
+// the sums move to a second set in shared memory: chains of thousands of terms cost
+// accuracy (a smooth vector on 23,400 unknowns: 6.3e-15 of the norm in one chain a
+// chunk, 4.4e-15 in the thread-per-atom form, now 0.7e-15).  The order of an element's
+// sum does not depend on BM.
+// Measured at 13,528 unknowns and 42 rows: 5,085 us element by element in 64 rows,
+// 1,429 us a pair at a time with FMAs, now 1,083 us (average of four launches).
 // ---------------------------------------------------------------------------
+constexpr int BN = 128, kTiledThreads = 128;
+constexpr int kFlush = 16;
+
 template <int BM, bool FMU>
 __global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n, int jchunk, int N, int nt,
                                                                    const double *__restrict__ pos,
@@ -230,17 +146,31 @@ __global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n,
     constexpr int NC = FMU ? 4 : 1;
     constexpr int KA = 16 / NC;                // source atoms a slab (16 unknowns)
     constexpr int CA = BN / NC;                // target atoms a block
-    constexpr int RM = BM / 8;                 // rows a thread
-    __shared__ double As[BM][16 + 1];
-    __shared__ double Bs[16][BN];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    constexpr int MT = BM / 8, NT = BN / 32;   // 8 x 8 tiles of a warp
+    __shared__ double As[BM][16 + 4];          // the paddings spread a fragment over the banks
+    __shared__ double Bs[16][BN + 4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kk = lane & 3, g = lane >> 2;
     const int row0 = blockIdx.y * BM, i0 = blockIdx.x * CA;
     const int jbeg = blockIdx.z * jchunk, jend = min(N, jbeg + jchunk);
-    double acc[RM][8];
+    double acc[MT][NT][2];
 #pragma unroll
-    for (int u = 0; u < RM; ++u)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int v = 0; v < 8; ++v) acc[u][v] = 0.0;
+        for (int t = 0; t < NT; ++t) acc[m][t][0] = acc[m][t][1] = 0.0;
+    extern __shared__ double upper[];          // [MT * NT * 2][threads]: the second set
+    for (int e = 0; e < MT * NT * 2; ++e) upper[e * kTiledThreads + threadIdx.x] = 0.0;
+    auto flush = [&]() {
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    upper[((m * NT + t) * 2 + v) * kTiledThreads + threadIdx.x] += acc[m][t][v];
+                    acc[m][t][v] = 0.0;
+                }
+    };
+    int slab = 0;
     for (int j0 = jbeg; j0 < jend; j0 += KA) {
         __syncthreads();
         for (int e = threadIdx.x; e < BM * 16; e += kTiledThreads) {
@@ -276,7 +206,7 @@ __global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n,
             }
             // element [source component][target component]
             double2 *b = reinterpret_cast<double2 *>(&Bs[(NC * jl) % 16][(NC * il) % BN]);
-            constexpr int ld = BN / 2;
+            constexpr int ld = (BN + 4) / 2;
             b[0] = make_double2(t.qq, t.mq[0]);
             b[1] = make_double2(t.mq[1], t.mq[2]);
             b[ld] = make_double2(t.qm[0], t.mm[0]);
@@ -287,30 +217,34 @@ __global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n,
             b[3 * ld + 1] = make_double2(t.mm[4], t.mm[5]);
         }
         __syncthreads();
-        const int kn = min(16, NC * (jend - j0));
-#pragma unroll 4
-        for (int k = 0; k < kn; ++k) {
-            double a[RM], b[8];
 #pragma unroll
-            for (int u = 0; u < RM; ++u) a[u] = As[ty * RM + u][k];
+        for (int k = 0; k < 16; k += 4) {      // unknowns past the chunk are zeros
+            double a[MT], b[NT];
 #pragma unroll
-            for (int v = 0; v < 8; ++v) b[v] = Bs[k][tx + 16 * v];
+            for (int m = 0; m < MT; ++m) a[m] = As[8 * m + g][k + kk];
 #pragma unroll
-            for (int u = 0; u < RM; ++u)
+            for (int t = 0; t < NT; ++t) b[t] = Bs[k + kk][32 * warp + 8 * t + g];
 #pragma unroll
-                for (int v = 0; v < 8; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) dmma(acc[m][t], a[m], b[t]);
         }
+        if (++slab % kFlush == 0) flush();
     }
+    flush();
 #pragma unroll
-    for (int u = 0; u < RM; ++u) {
-        const int gr = row0 + ty * RM + u;
+    for (int m = 0; m < MT; ++m) {
+        const int gr = row0 + 8 * m + g;
         if (gr >= R) continue;
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-            const int c = tx + 16 * v, i = i0 + c / NC, comp = c % NC;
-            if (i < N)
-                part[((int64_t)blockIdx.z * R + gr) * n + (comp == 0 ? i : N + 3 * i + comp - 1)] = acc[u][v];
-        }
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int c = 32 * warp + 8 * t + 2 * kk + v, i = i0 + c / NC, comp = c % NC;
+                if (i < N)
+                    part[((int64_t)blockIdx.z * R + gr) * n + (comp == 0 ? i : N + 3 * i + comp - 1)] =
+                        upper[((m * NT + t) * 2 + v) * kTiledThreads + threadIdx.x];
+            }
     }
 }
 
@@ -642,30 +576,17 @@ void contract_t(plx_geom *g, int count, const double *X, double *S, Contraction 
 }
 
 // S = X T for R rows X [R][n] and a row-major n x n FP64 matrix (S^T = T^T X^T):
-// the split-K products above, the partial sums in `scratch` (grown on demand).
-// A row's result does not depend on R within R <= 16 or above it.
+// the split-K products of skinny.cuh, the partial sums in `scratch` (grown on demand).
+// A row's result does not depend on R.
 void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const double *X, const double *T, double *S) {
-    // K split: depends on n only (not on the batch), see tiled_partial
-    const int cb = n_blocks(n, kSkinnyCols);
+    // K split: depends on n only (not on the batch)
     int ks, kchunk;
     skinny_split(n, ks, kchunk);
     size_t need = (size_t)ks * R * n;
     if (scratch.n < need) scratch.alloc(ctx, need);
     double *part = scratch.p;
     cudaStream_t st = ctx->stream;
-    if (R <= 16) {
-        dim3 grid(cb, ks);
-        switch (R) {
-#define PLX_SK(RR) \
-    case RR: skinny_partial<RR><<<grid, kSkinnyCols, 0, st>>>(n, kchunk, X, T, part); break;
-            PLX_SK(2) PLX_SK(4) PLX_SK(6) PLX_SK(8) PLX_SK(10) PLX_SK(12) PLX_SK(14) PLX_SK(16)
-#undef PLX_SK
-            default: throw Error(PLX_ERR_ARG, "bad skinny row count");
-        }
-    } else {
-        dim3 grid(n_blocks(n, BN), n_blocks(R, BM), ks);
-        tiled_partial<<<grid, kTiledThreads, 0, st>>>(R, n, kchunk, X, T, part);
-    }
+    launch_product_partial(st, R, n, ks, kchunk, X, T, part);
     skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, ks, part, S);
     ctx->launches += 2;
     PLX_CHECK_CUDA(cudaGetLastError());
@@ -691,19 +612,26 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
             if (g->d_part.n < need) g->d_part.alloc(ctx, need);
             const int bm = R <= 16 ? 16 : R <= 32 ? 32 : (R <= 48 ? 48 : 64);
             const dim3 grid(tiles, n_blocks(R, bm), js);
-#define PLX_OTF(BMV, F)                                                                                             \
-    otf_tiled_partial<BMV, F><<<grid, kTiledThreads, 0, st>>>(R, n, jchunk, N, g->n_types, g->d_pos.p, g->d_par.p, \
-                                                              g->d_type.p, g->d_widths.p, X, g->d_part.p)
+#define PLX_OTF(BMV, F)                                                                                            \
+    {                                                                                                             \
+        auto kern = otf_tiled_partial<BMV, F>;                                                                    \
+        const size_t smem = (size_t)BMV * BN * sizeof(double);                                                    \
+        once_per_device(reinterpret_cast<const void *>(kern), ctx->device, [&] {                                  \
+            PLX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));   \
+        });                                                                                                       \
+        kern<<<grid, kTiledThreads, smem, st>>>(R, n, jchunk, N, g->n_types, g->d_pos.p, g->d_par.p, g->d_type.p, \
+                                                g->d_widths.p, X, g->d_part.p);                                   \
+    }
             if (fmu) {
-                if (bm == 16) PLX_OTF(16, true);
-                else if (bm == 32) PLX_OTF(32, true);
-                else if (bm == 48) PLX_OTF(48, true);
-                else PLX_OTF(64, true);
+                if (bm == 16) PLX_OTF(16, true)
+                else if (bm == 32) PLX_OTF(32, true)
+                else if (bm == 48) PLX_OTF(48, true)
+                else PLX_OTF(64, true)
             } else {
-                if (bm == 16) PLX_OTF(16, false);
-                else if (bm == 32) PLX_OTF(32, false);
-                else if (bm == 48) PLX_OTF(48, false);
-                else PLX_OTF(64, false);
+                if (bm == 16) PLX_OTF(16, false)
+                else if (bm == 32) PLX_OTF(32, false)
+                else if (bm == 48) PLX_OTF(48, false)
+                else PLX_OTF(64, false)
             }
 #undef PLX_OTF
             skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, js, g->d_part.p, S);
