@@ -232,6 +232,14 @@ void rhs_batch(plx_geom *g, const OpBatch &b, const int32_t *d_pol, double *Bout
 //   1 / diag(A(w_c)) for every column, [count][2][n] split complex.
 void diagonal_inverse(plx_geom *g, const OpBatch &b, double *Pinv);
 
+// fold.cu: the charge rows of A0 = (K - P) T (alloys: 1/2 (K + K^T) in place of K), T
+// stored or generated, into the tensor-core operand
+struct FoldTarget {
+    uint16_t *hi, *lo;
+    int64_t ktiles;
+};
+void fold_charge_rows(plx_geom *g, const FoldTarget &out);
+
 // tc_contract.cu: S = T X with BF16-split operands on the tensor cores
 // (nprod 3: Th Xh + Th Xl + Tl Xh; nprod 1: Th Xh).  X, S: [count][2][n] FP64.
 void build_t_split(plx_geom *g);

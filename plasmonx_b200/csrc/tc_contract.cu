@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "operand.cuh"
 #include "pair_tiles.cuh"
 #include "plx_internal.h"
 
@@ -43,9 +44,7 @@ namespace plx {
 
 namespace {
 
-constexpr int kUM = 128;          // rows per tcgen05.mma (TMEM lanes)
-constexpr int kBM = 2 * kUM;      // rows of T per CTA: two accumulators share every B tile
-constexpr int kBK = 32;           // k per stage (64 bytes of BF16: the 64-byte swizzle atom)
+constexpr int kUM = kBM / 2;      // rows per tcgen05.mma (TMEM lanes): two accumulators share every B tile
 constexpr int kLdAlign = 64;      // k padding of the split operands (zeros)
 constexpr int kUmmaK = 16;        // k per tcgen05.mma (kind::f16)
 constexpr uint32_t kDrainLimit = 1u << 22;  // clean-up waits after an abort (seconds at most)
@@ -555,28 +554,6 @@ __global__ void __launch_bounds__(kBM) reduce_pieces(const __grid_constant__ TcL
     store_columns<kRedCols / 2>(G, m0 + r, n0 + c0, a);
 }
 
-// The A operand (T, A0 or D^T split in BF16 high/low) is stored in the order
-// the kernel reads it: [m-tile of 256 rows][k-slab of 32][256 rows][32 k], so
-// every stage's tile (256 x 32) is one contiguous 16 KB block of HBM, and within
-// the tile already in the shared-memory image the UMMA descriptors read: the
-// 64-byte swizzle, in which the 16-byte chunk c of row r sits at chunk
-// c ^ ((r >> 1) & 3) of its 64-byte row.  A stage's A tile is then one plain
-// bulk copy.  Rows beyond n and k beyond n are zero.
-__device__ __forceinline__ int64_t a_tile_pos(int64_t rr, int64_t kk) {
-    return rr * kBK + ((((kk >> 3) ^ ((rr >> 1) & 3)) << 3) | (kk & 7));
-}
-__device__ __forceinline__ int64_t a_tiled(int64_t r, int64_t k, int64_t ktiles) {
-    return ((r / kBM) * ktiles + k / kBK) * (int64_t)(kBM * kBK) + a_tile_pos(r % kBM, k % kBK);
-}
-
-__device__ __forceinline__ void split_store(double a, int64_t idx, __nv_bfloat16 *__restrict__ hi,
-                                            __nv_bfloat16 *__restrict__ lo) {
-    float x = (float)a;
-    __nv_bfloat16 h = __float2bfloat16_rn(x);
-    hi[idx] = h;
-    lo[idx] = __float2bfloat16_rn(x - __bfloat162float(h));
-}
-
 // Row-major n x n FP64 matrix -> tiled BF16 pair; the output is walked in its
 // own (contiguous) order.
 __global__ void split_tiled(int n, int64_t ktiles, int64_t total, const double *__restrict__ in,
@@ -625,57 +602,57 @@ __global__ void split_tiled_gen(int N, int n, int fmu, int64_t ktiles, const dou
     }
 }
 
-// Folded operator rows, split like T.  For a charge row i < N
-//   A0[i][k] = sum_e c_e (T[j_e][k] - T[i][k])      (CSR order, FP64)
-// with c_e = K_ij for one atom type (the charge rows of (K - P) T,
-// update_y_q of matrix_module.f90:1011-1098, applied to T itself) and
-// c_e = 1/2 (K_ij + K_ji) for alloys (the w-independent part of
-// 1/2 (K + (w_j/w_i) K^T)); for a dipole row A0[r][k] = T[r][k]; the rows
-// appended after n are the charge rows of T of the interface atoms.  T comes
-// from the stored matrix or, without one, from the pair formulas.  One block
-// per (row, column chunk); rows vary fastest over the grid, so the blocks
-// running together share their neighbours' rows of T in L2.
-// T rows [t_row0, ...) held in T (stored matrix: t_row0 = 0; a generated
-// window of charge rows otherwise), or generated from the pair formulas.
-__device__ __forceinline__ double t_value(const double *__restrict__ T, int64_t t_row0, int N, int n, int fmu,
-                                          const double *__restrict__ pos, const double *__restrict__ par, int64_t r,
-                                          int64_t k) {
-    return T ? T[(r - t_row0) * n + k] : plx_t_element(N, fmu != 0, pos, par, r, k);
+// Rows of the folded operand that are rows of T, split like T: the dipole rows r < n
+// and, after them, the charge rows of the interface atoms.  (The charge rows are folded
+// in fold.cu.)
+__global__ void copy_rows_split(int N, int n, int64_t ktiles, const double *__restrict__ T,
+                                const int32_t *__restrict__ iface_atom, __nv_bfloat16 *__restrict__ hi,
+                                __nv_bfloat16 *__restrict__ lo) {
+    const int64_t r = N + (int64_t)blockIdx.x;
+    const int64_t k = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int64_t src = r < n ? r : iface_atom[r - n];
+    split_store(T[src * n + k], a_tiled(r, k, ktiles), hi, lo);
 }
 
-// Charge rows [a0, a0 + gridDim.x) of T generated into a window buffer.
-__global__ void t_rows_gen(int N, int n, int fmu, int64_t a0, const double *__restrict__ pos,
-                           const double *__restrict__ par, double *__restrict__ Tw) {
-    const int64_t a = a0 + blockIdx.x;
-    const int64_t k = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
-    if (k < n) Tw[(int64_t)blockIdx.x * n + k] = plx_t_element(N, fmu != 0, pos, par, a, k);
-}
-
-__global__ void fold_split(int N, int n, int64_t ld, int64_t ktiles, int hetero, int fmu, int64_t r_begin,
-                           int64_t t_row0,
-                           const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-                           const double *__restrict__ kval, const double *__restrict__ ktval,
-                           const double *__restrict__ T, const double *__restrict__ pos,
-                           const double *__restrict__ par, const int32_t *__restrict__ iface_atom,
-                           __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
-    const int64_t r = r_begin + blockIdx.x;
-    const int64_t k = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
-    if (k >= ld) return;
-    double a = 0.0;
-    if (k < n) {
-        if (r < N) {
-            const double trk = t_value(T, t_row0, N, n, fmu, pos, par, r, k);
-            for (int e = rowptr[r]; e < rowptr[r + 1]; ++e) {
-                const double c = hetero ? 0.5 * (kval[e] + ktval[e]) : kval[e];
-                a = fma(c, t_value(T, t_row0, N, n, fmu, pos, par, col[e], k) - trk, a);
-            }
-        } else if (r < n) {
-            a = t_value(T, t_row0, N, n, fmu, pos, par, r, k);
-        } else {
-            a = t_value(T, t_row0, N, n, fmu, pos, par, iface_atom[r - n], k);
-        }
+// The same rows without a stored T, a thread per pair of atoms: the dipole rows of atom i
+// (or, beyond N, the charge row of interface atom i - N) against atom j, whose error
+// functions and exponential are evaluated once for the pair's 12 (4) elements.
+__global__ void pair_rows_split(int N, int n, int nt, int fmu, int64_t ktiles, const double *__restrict__ pos,
+                                const double *__restrict__ par, const int32_t *__restrict__ type,
+                                const PairWidths *__restrict__ widths, const int32_t *__restrict__ iface_atom,
+                                __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
+    const int j = blockIdx.y * blockDim.x + threadIdx.x;
+    if (j >= N) return;
+    const int u = fmu ? blockIdx.x : blockIdx.x + N;       // wFQ has no dipole rows
+    const bool face = u >= N;
+    const int i = face ? iface_atom[u - N] : u;
+    PairTile t;
+    t.qq = 0.0;
+    for (int k = 0; k < 3; ++k) t.qm[k] = t.mq[k] = 0.0;
+    for (int k = 0; k < 6; ++k) t.mm[k] = 0.0;
+    if (i == j) {
+        t.qq = par[2 * N + i];
+    } else {
+        const double dx = pos[i] - pos[j], dy = pos[N + i] - pos[N + j], dz = pos[2 * N + i] - pos[2 * N + j];
+        const int ti = type[i], tj = type[j];
+        if (fmu) plx_pair_tile_w(dx, dy, dz, widths[ti + nt * tj], ti == tj, t);
+        else t.qq = plx_pair_qq_w(dx, dy, dz, widths[ti + nt * tj]);
     }
-    split_store(a, a_tiled(r, k, ktiles), hi, lo);
+    auto put = [&](int64_t r, int64_t k, double v) { split_store(v, a_tiled(r, k, ktiles), hi, lo); };
+    if (face) {
+        const int64_t r = n + (u - N);
+        put(r, j, t.qq);
+        if (fmu)
+            for (int b = 0; b < 3; ++b) put(r, N + 3LL * j + b, t.qm[b]);
+        return;
+    }
+    const int mi[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+    for (int a = 0; a < 3; ++a) {
+        const int64_t r = N + 3LL * i + a;
+        put(r, j, t.mq[a]);
+        for (int b = 0; b < 3; ++b) put(r, N + 3LL * j + b, t.mm[mi[a][b]]);
+    }
 }
 
 // FP64 -> (BF16 high, BF16 low) split of row-major rows [rows][n] into rows of ld
@@ -862,67 +839,20 @@ static void build_a_split(plx_geom *g) {
     const int fmu = g->model == PLX_WFQFMU, N = g->n_atoms;
     auto *hi = reinterpret_cast<__nv_bfloat16 *>(g->d_Ah.p);
     auto *lo = reinterpret_cast<__nv_bfloat16 *>(g->d_Al.p);
-    const unsigned kchunks = (unsigned)((ld + 255) / 256);
     cudaStream_t st = g->ctx->stream;
-    if (g->has_T) {
-        fold_split<<<dim3((unsigned)M, kchunks), 256, 0, st>>>(
-            N, (int)n, ld, ktiles, hetero, fmu, 0, 0, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_T.p,
-            g->d_pos.p, g->d_par.p, g->d_iface_atom.p, hi, lo);
+    const FoldTarget out{g->d_Ah.p, g->d_Al.p, ktiles};
+    if (M > N && g->has_T) {
+        copy_rows_split<<<dim3((unsigned)(M - N), (unsigned)((n + 255) / 256)), 256, 0, st>>>(
+            N, (int)n, ktiles, g->d_T.p, g->d_iface_atom.p, hi, lo);
         g->ctx->launches++;
-    } else {
-        // matrix-free: dipole and interface rows generated element by element; the
-        // charge rows folded chunk by chunk from a window of generated T rows that
-        // covers the chunk's conductance neighbours (atoms are ordered in space, so
-        // a window is the chunk plus the neighbours' reach)
-        if (M > N) {
-            fold_split<<<dim3((unsigned)(M - N), kchunks), 256, 0, st>>>(
-                N, (int)n, ld, ktiles, hetero, fmu, N, 0, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p,
-                nullptr, g->d_pos.p, g->d_par.p, g->d_iface_atom.p, hi, lo);
-            g->ctx->launches++;
-        }
-        std::vector<int32_t> rowptr(N + 1), col((size_t)g->nnz);
-        PLX_CHECK_CUDA(cudaMemcpyAsync(rowptr.data(), g->d_rowptr.p, (N + 1) * 4, cudaMemcpyDeviceToHost, st));
-        if (g->nnz) PLX_CHECK_CUDA(cudaMemcpyAsync(col.data(), g->d_col.p, g->nnz * 4, cudaMemcpyDeviceToHost, st));
-        PLX_CHECK_CUDA(cudaStreamSynchronize(st));
-        const int64_t max_rows = std::max<int64_t>(64, (int64_t)(6.0e9 / (8.0 * (double)n)));   // <= ~6 GB window
-        DevArray<double> Tw;
-        Tw.alloc(g->ctx, (size_t)(max_rows * n));
-        int64_t r0 = 0;
-        while (r0 < N) {
-            // grow the chunk while its window fits
-            int64_t r1 = r0, lo_w = r0, hi_w = r0;
-            while (r1 < N) {
-                int64_t l = std::min<int64_t>(lo_w, r1), h = std::max<int64_t>(hi_w, r1);
-                for (int e = rowptr[r1]; e < rowptr[r1 + 1]; ++e) {
-                    l = std::min<int64_t>(l, col[e]);
-                    h = std::max<int64_t>(h, col[e]);
-                }
-                if (h - l + 1 > max_rows) break;
-                lo_w = l;
-                hi_w = h;
-                ++r1;
-            }
-            if (r1 == r0) {
-                // a single row reaching farther than the window: generate its T values in place
-                fold_split<<<dim3(1, kchunks), 256, 0, st>>>(N, (int)n, ld, ktiles, hetero, fmu, r0, 0, g->d_rowptr.p,
-                                                             g->d_col.p, g->d_kval.p, g->d_ktval.p, nullptr, g->d_pos.p,
-                                                             g->d_par.p, g->d_iface_atom.p, hi, lo);
-                g->ctx->launches++;
-                r0 = r0 + 1;
-                continue;
-            }
-            const int64_t W = hi_w - lo_w + 1;
-            t_rows_gen<<<dim3((unsigned)W, (unsigned)((n + 255) / 256)), 256, 0, st>>>(N, (int)n, fmu, lo_w, g->d_pos.p,
-                                                                                       g->d_par.p, Tw.p);
-            fold_split<<<dim3((unsigned)(r1 - r0), kchunks), 256, 0, st>>>(
-                N, (int)n, ld, ktiles, hetero, fmu, r0, lo_w, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p,
-                Tw.p, g->d_pos.p, g->d_par.p, g->d_iface_atom.p, hi, lo);
-            g->ctx->launches += 2;
-            PLX_CHECK_CUDA(cudaGetLastError());
-            r0 = r1;
-        }
-        PLX_CHECK_CUDA(cudaStreamSynchronize(st));
+    } else if (M > N) {
+        const unsigned units = (unsigned)((fmu ? N : 0) + (M - n));
+        pair_rows_split<<<dim3(units, (unsigned)((N + 127) / 128)), 128, 0, st>>>(
+            N, (int)n, g->n_types, fmu, ktiles, g->d_pos.p, g->d_par.p, g->d_type.p, g->d_widths.p, g->d_iface_atom.p, hi,
+            lo);
+        g->ctx->launches++;
     }
+    fold_charge_rows(g, out);
     PLX_CHECK_CUDA(cudaGetLastError());
     if (!g->d_tc_err.p) {
         g->d_tc_err.alloc(g->ctx, 1);
