@@ -43,6 +43,40 @@ void plx::dev_free(plx_ctx *ctx, void *p, size_t bytes) {
     ctx->in_use -= bytes;
 }
 
+void plx::PinnedArray::alloc(plx_ctx *c, size_t count) {
+    release();
+    ctx = c;
+    if (count == 0) return;
+    if (count <= kPinnedKeep) {
+        std::lock_guard<std::mutex> lock(c->pinned_mutex);
+        for (size_t i = c->pinned.size(); i-- > 0;)
+            if (c->pinned[i].second >= count) {
+                p = c->pinned[i].first;
+                n = c->pinned[i].second;
+                c->pinned.erase(c->pinned.begin() + (ptrdiff_t)i);
+                return;
+            }
+        count = (count + 511) / 512 * 512;
+    }
+    PLX_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), count * sizeof(double), cudaHostAllocDefault));
+    n = count;
+}
+
+// Kernels of the context's stream may still be about to write the block: its next
+// user's kernels come after them on that stream, and cudaFreeHost waits for them.
+void plx::PinnedArray::release() {
+    if (!p) return;
+    bool keep = false;
+    if (n <= kPinnedKeep) {
+        std::lock_guard<std::mutex> lock(ctx->pinned_mutex);
+        keep = ctx->pinned.size() < kPinnedBlocks;
+        if (keep) ctx->pinned.emplace_back(p, n);
+    }
+    if (!keep) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+}
+
 namespace {
 
 template <typename F>
@@ -141,6 +175,7 @@ plx_ctx *plx_ctx_create(int32_t device, uint64_t hbm_budget_bytes) {
     if (!ctx) return nullptr;
     ctx->device = device;
     plx_status s = guarded(ctx, [&] {
+        ctx->pinned.reserve(kPinnedBlocks);
         PLX_CHECK_CUDA(cudaSetDevice(device));
         PLX_CHECK_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         PLX_CHECK_CUDA(cudaEventCreate(&ctx->ev0));
@@ -165,6 +200,7 @@ void plx_ctx_destroy(plx_ctx *ctx) {
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
+    for (auto &b : ctx->pinned) cudaFreeHost(b.first);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     // the pool keeps freed blocks for reuse; a closed context's blocks go back to
     // the device, so that what it held is free for other contexts and processes

@@ -21,7 +21,9 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstring>
 #include <memory>
 #include <type_traits>
 
@@ -529,21 +531,24 @@ __global__ void __launch_bounds__(kThreads) norm_partial(int n, const double *__
     if (threadIdx.x == 0) part[(int64_t)k * gridDim.x + blockIdx.x] = s;
 }
 
+// `host`: the same norms in the run's pinned block
 __global__ void norm_finish(int nchunk, int count, const double *__restrict__ part,
-                            double *__restrict__ out) {
+                            double *__restrict__ out, double *__restrict__ host) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     double s = 0.0;
     for (int b = 0; b < nchunk; ++b) s += part[(int64_t)k * nchunk + b];
     out[k] = sqrt(s);
+    host[k] = sqrt(s);
 }
 
-// v_1 = b / ||b||; g_1 = ||b||.
+// v_1 = b / ||b||; g_1 = ||b||; the slab's address into the table.
 template <typename VT>
 __global__ void start_vectors(int n, const int32_t *__restrict__ act, const double *__restrict__ nrm,
-                              const double *__restrict__ B, VT *__restrict__ slab0,
+                              const double *__restrict__ B, VT *__restrict__ slab0, VT **__restrict__ slabs,
                               double2 *__restrict__ g, int gstride) {
     int k = blockIdx.y, c = act[k];
+    if (blockIdx.x == 0 && k == 0 && threadIdx.x == 0) slabs[0] = slab0;
     double s = nrm[k];
     const double *b = B + (int64_t)c * 2 * n;
     VT *v = slab0 + (int64_t)c * 2 * n;
@@ -576,7 +581,7 @@ __device__ __forceinline__ double2 shfl_up2(double2 v, int o) {
 }
 
 // Givens update of column j by one warp (norm = H(j+1, j)).
-// Hcols[j] points to the slab of H column j ([C][hstride] complex).
+// Hcol is the slab of H column j ([C][hstride] complex).
 //
 // The j earlier rotations form a chain: with a_0 = h_0 the i-th rotation gives
 // h_i' = c_i a_i + s_i h_{i+1} and passes on a_{i+1} = c_i h_{i+1} - conj(s_i) a_i.
@@ -592,10 +597,10 @@ struct Rotation {
     double c;
 };
 template <bool SCAN>
-__device__ void givens(int k, int c, int lane, int j, double norm, double2 *const *__restrict__ Hcols, int hstride,
+__device__ void givens(int k, int c, int lane, int j, double norm, double2 *__restrict__ Hcol, int hstride,
                        double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g, int gstride,
                        int cstride, double *__restrict__ resid, Rotation *rot) {
-    double2 *h = Hcols[j] + (int64_t)c * hstride;
+    double2 *h = Hcol + (int64_t)c * hstride;
     double *csc = cs + (int64_t)c * cstride;
     double2 *snc = sn + (int64_t)c * cstride;
     double2 *gc = g + (int64_t)c * gstride;
@@ -688,13 +693,19 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *cons
 // The norm: nparts partial sums of squares npart -- added by the block in the inner
 // solves (VT float), in their order in the plain form -- or with nparts = 0 the chunks
 // of W themselves (up to kNormChunks, in norm_partial's order).
+//
+// The launch also enters the new slab and H column in the address tables, which the
+// kernels of the next steps read, and leaves the residual estimates in pinned host
+// memory: three 8-byte copies in, one back and a clearing of the H column (every row
+// that is read has been written) cost a step about 20 us of gaps between the kernels.
 constexpr int kNormChunks = 2;
 template <typename VT>
 __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
                                                              const double *__restrict__ npart,
                                                              const double *__restrict__ W, VT *__restrict__ slab_next,
                                                              const double *__restrict__ P, double *__restrict__ X,
-                                                             TcColumns sp, double2 *const *__restrict__ Hcols,
+                                                             TcColumns sp, VT **__restrict__ slabs,
+                                                             double2 **__restrict__ Hcols, double2 *__restrict__ Hcol,
                                                              int hstride, double *__restrict__ cs,
                                                              double2 *__restrict__ sn, double2 *__restrict__ g,
                                                              int gstride, int cstride, double *__restrict__ resid) {
@@ -702,6 +713,10 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
     __shared__ double total;
     __shared__ Rotation rot[kInner ? 1 : 32];
     const int k = blockIdx.y, c = act[k];
+    if (blockIdx.x == 0 && k == 0 && threadIdx.x == 0) {
+        slabs[j + 1] = slab_next;
+        Hcols[j] = Hcol;
+    }
     const double *w = W + (int64_t)k * 2 * n;
     double s = 0.0;
     if (kInner) {
@@ -738,7 +753,7 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
         if (sp.hi) split_column(sp, k, r, re, im);
     }
     if (blockIdx.x == 0 && threadIdx.x < 32)
-        givens<kInner>(k, c, threadIdx.x, j, s, Hcols, hstride, cs, sn, g, gstride, cstride, resid, rot);
+        givens<kInner>(k, c, threadIdx.x, j, s, Hcol, hstride, cs, sn, g, gstride, cstride, resid, rot);
 }
 
 // y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
@@ -910,12 +925,12 @@ int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const
 
 // Norms ||v[k]|| of a compact batch (used for ||b|| and the true residual).
 static void batch_norms(plx_geom *g, int count, const double *V, DevArray<double> &part,
-                        DevArray<double> &out) {
+                        DevArray<double> &out, double *host) {
     plx_ctx *ctx = g->ctx;
     const int n = g->n_var;
     int nchunk = n_blocks(n, kRows);
     norm_partial<<<dim3(nchunk, count), kThreads, 0, ctx->stream>>>(n, V, part.p);
-    norm_finish<<<n_blocks(count, 128), 128, 0, ctx->stream>>>(nchunk, count, part.p, out.p);
+    norm_finish<<<n_blocks(count, 128), 128, 0, ctx->stream>>>(nchunk, count, part.p, out.p, host);
     ctx->launches += 2;
 }
 
@@ -923,7 +938,7 @@ static void batch_norms(plx_geom *g, int count, const double *V, DevArray<double
 // operator application of every step can be shared with other solves (a
 // grouped tensor-core launch over several geometries): begin(), then while
 // wants_product(): pre() -> the caller forms W = A X of the returned batch ->
-// post(); then end().  gmres_batched runs it with its own operator.
+// post() -> settle(); then end().  gmres_batched runs it with its own operator.
 template <typename VT>
 class GmresRun final : public GmresStepper {
   public:
@@ -966,8 +981,7 @@ class GmresRun final : public GmresStepper {
         std::vector<DevArray<double2>>(m_).swap(hcols_);
         d_slabs_.alloc(ctx_, m_ + 1);
         d_hcols_.alloc(ctx_, m_);
-        h_slabs_.assign(m_ + 1, nullptr);
-        h_hcols_.assign(m_, nullptr);
+        host_.alloc(ctx_, (size_t)2 * C_);
         PLX_CHECK_CUDA(cudaMemsetAsync(d_X_, 0, (size_t)C_ * 2 * n * 8, st_));
         if (rq_.contraction == Contraction::TC3 || rq_.contraction == Contraction::TC1) split_ = tc_presplit(g_, C_);
         jac_ = rq_.jacobi && rq_.inner;
@@ -982,15 +996,13 @@ class GmresRun final : public GmresStepper {
         act_.resize(C_);
         for (int c = 0; c < C_; ++c) act_[c] = c;
         PLX_CHECK_CUDA(cudaMemcpyAsync(d_act_.p, act_.data(), C_ * 4, cudaMemcpyHostToDevice, st_));
-        batch_norms(g_, C_, d_B_, nrm_part_, nrm_);   // B is [C] in column order == compact order here
-        std::vector<double> bnorm(C_);
-        PLX_CHECK_CUDA(cudaMemcpyAsync(bnorm.data(), nrm_.p, C_ * 8, cudaMemcpyDeviceToHost, st_));
-        PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
+        batch_norms(g_, C_, d_B_, nrm_part_, nrm_, host_.p);   // B is [C] in column order == compact order here
         slabs_[0].alloc(ctx_, (size_t)C_ * 2 * n);
-        h_slabs_[0] = slabs_[0].p;
         start_vectors<VT><<<dim3(grid_rows(2LL * n), C_), 256, 0, st_>>>(n, d_act_.p, nrm_.p, d_B_, slabs_[0].p,
-                                                                      gv_.p, hstride_);
+                                                                      d_slabs_.p, gv_.p, hstride_);
         ctx_->launches++;
+        PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
+        const double *bnorm = host_.p;
         act_.clear();
         for (int c = 0; c < C_; ++c) {
             if (!std::isfinite(bnorm[c])) {
@@ -1000,7 +1012,6 @@ class GmresRun final : public GmresStepper {
             }
         }
         upload_active();
-        resid_.assign(C_, 0.0);
         j_ = 0;
     }
 
@@ -1011,27 +1022,20 @@ class GmresRun final : public GmresStepper {
         const int n = g_->n_var;
         const int na = (int)act_.size();
         if (!x_ready_) {
-            gather_cols<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, h_slabs_[j_],
+            gather_cols<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, slabs_[j_].p,
                                                                      jac_ ? Pinv_.p : nullptr, Xa_.p, split_);
             ctx_->launches++;
         }
         return OpInput{g_, OpBatch{na, d_freq_act_.p}, Xa_.p, Wa_.p, work_.p, rq_.contraction, split_.hi != nullptr};
     }
 
-    // the Arnoldi step on W, the least-squares update and the convergence test
+    // launches the Arnoldi step on W and the least-squares update
     void post() override {
         const int n = g_->n_var;
         const int j = j_;
         const int na = (int)act_.size();
         hcols_[j].alloc(ctx_, (size_t)C_ * hstride_);
-        h_hcols_[j] = hcols_[j].p;
         slabs_[j + 1].alloc(ctx_, (size_t)C_ * 2 * n);
-        h_slabs_[j + 1] = slabs_[j + 1].p;
-        PLX_CHECK_CUDA(cudaMemcpyAsync(d_slabs_.p + j + 1, &h_slabs_[j + 1], sizeof(VT *), cudaMemcpyHostToDevice, st_));
-        if (j == 0)
-            PLX_CHECK_CUDA(cudaMemcpyAsync(d_slabs_.p, &h_slabs_[0], sizeof(VT *), cudaMemcpyHostToDevice, st_));
-        PLX_CHECK_CUDA(cudaMemcpyAsync(d_hcols_.p + j, &h_hcols_[j], sizeof(double2 *), cudaMemcpyHostToDevice, st_));
-        PLX_CHECK_CUDA(cudaMemsetAsync(hcols_[j].p, 0, (size_t)C_ * hstride_ * 16, st_));
         size_t need = (size_t)na * ndot_ * (j + 1);
         if (part_.n < need) part_.alloc(ctx_, std::max(need, part_.n * 2));
         int nparts = 0;
@@ -1076,25 +1080,32 @@ class GmresRun final : public GmresStepper {
             }
         }
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
+        for (int k = 0; k < na; ++k) memcpy(host_.p + k, &kPending, 8);
         prof_begin(ctx_);
         normalize_givens<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(
-            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_hcols_.p,
-            hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, nrm_.p);
+            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p,
+            d_hcols_.p, hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, host_.p);
         ctx_->launches++;
         x_ready_ = true;
         prof_end(ctx_, PROF_LSQ, 0.0, 0.0);
         PLX_CHECK_CUDA(cudaGetLastError());
-        PLX_CHECK_CUDA(cudaMemcpyAsync(resid_.data(), nrm_.p, na * 8, cudaMemcpyDeviceToHost, st_));
-        PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
-        // --- convergence test -----------------------------------------------------
+    }
+
+    // waits for the step and tests its residuals
+    void settle() override {
+        const int n = g_->n_var;
+        const int j = j_;
+        const int na = (int)act_.size();
+        const double *resid = host_.p;
+        await_residuals(na);
         std::vector<int32_t> trig;
         for (int k = 0; k < na; ++k) {
             int c = act_[k];
             res_.steps[c] = j + 1;
-            if (rq_.record_trace) res_.trace[(size_t)c * m_ + j] = resid_[k];
+            if (rq_.record_trace) res_.trace[(size_t)c * m_ + j] = resid[k];
             const double tc = rq_.tols.empty() ? rq_.tol : rq_.tols[c];
-            if (!std::isfinite(resid_[k])) res_.status[c] = PLX_ERR_NAN;
-            else if (resid_[k] < tc || (rq_.inner && j == m_ - 1)) trig.push_back(c);
+            if (!std::isfinite(resid[k])) res_.status[c] = PLX_ERR_NAN;
+            else if (resid[k] < tc || (rq_.inner && j == m_ - 1)) trig.push_back(c);
         }
         std::vector<char> done(C_, 0);
         for (int c : act_)
@@ -1112,7 +1123,7 @@ class GmresRun final : public GmresStepper {
             }
             for (int c : trig) done[c] = 1;
             for (int c : trig)
-                if (resid_[std::find(act_.begin(), act_.end(), c) - act_.begin()] >=
+                if (resid[std::find(act_.begin(), act_.end(), c) - act_.begin()] >=
                     (rq_.tols.empty() ? rq_.tol : rq_.tols[c]))
                     res_.status[c] = PLX_ERR_NOT_CONVERGED;   // inner dimension used up (not an error)
         } else if (!trig.empty()) {
@@ -1136,9 +1147,8 @@ class GmresRun final : public GmresStepper {
                                : Contraction::FP64);
             residual<<<dim3(grid_rows(2LL * n), nt), 256, 0, st_>>>(n, d_cols_.p, d_B_, Wa_.p);
             ctx_->launches++;
-            batch_norms(g_, nt, Wa_.p, nrm_part_, nrm_);
-            std::vector<double> tres(nt);
-            PLX_CHECK_CUDA(cudaMemcpyAsync(tres.data(), nrm_.p, nt * 8, cudaMemcpyDeviceToHost, st_));
+            const double *tres = host_.p + C_;
+            batch_norms(g_, nt, Wa_.p, nrm_part_, nrm_, host_.p + C_);
             PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
             for (int t = 0; t < nt; ++t)
                 if (tres[t] < rq_.tol) done[trig[t]] = 1;
@@ -1181,12 +1191,33 @@ class GmresRun final : public GmresStepper {
         return false;
     }
 
+    // The residuals reach the host before the runtime reports the end of the kernel that
+    // wrote them: reading the words for up to about half a millisecond and then waiting
+    // for the stream brings the next product 4 us forward (12.2 -> 8 us after the step).
+    // A residual with the pending word's bits costs that wait, nothing else.
+    void await_residuals(int na) {
+        const volatile uint64_t *w = reinterpret_cast<const volatile uint64_t *>(host_.p);
+        int k = 0;
+        for (int polls = 0; k < na && polls < kPolls;) {
+            if (w[k] != kPending) ++k;
+            else {
+                ++polls;
+                __builtin_ia32_pause();
+            }
+        }
+        if (k < na) PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
+        std::atomic_thread_fence(std::memory_order_acquire);
+    }
+
     void upload_active() {
         std::vector<int32_t> fa(act_.size());
         for (size_t k = 0; k < act_.size(); ++k) fa[k] = rq_.freq[act_[k]];
         PLX_CHECK_CUDA(cudaMemcpyAsync(d_act_.p, act_.data(), act_.size() * 4, cudaMemcpyHostToDevice, st_));
         PLX_CHECK_CUDA(cudaMemcpyAsync(d_freq_act_.p, fa.data(), fa.size() * 4, cudaMemcpyHostToDevice, st_));
     }
+
+    static constexpr uint64_t kPending = 0xfff8a5c35a3c0001ull;      // a NaN that no kernel forms
+    static constexpr int kPolls = 1 << 14;
 
     plx_geom *g_;
     plx_ctx *ctx_;
@@ -1200,7 +1231,7 @@ class GmresRun final : public GmresStepper {
     TcColumns split_{nullptr, nullptr, 0};   // tensor-core runs: the split rows of the next input
     bool x_ready_ = false;      // Xa holds the next product's input
     std::vector<int32_t> act_;
-    std::vector<double> resid_;
+    PinnedArray host_;          // residual estimates [C], true residuals [C]
     DevArray<int32_t> d_act_, d_freq_act_, d_cols_;
     DevArray<double> Xa_, Wa_, work_, nrm_part_, nrm_, cs_, Pinv_;
     DevArray<double2> sn_, gv_, hbuf_, part_, ybuf_;
@@ -1208,8 +1239,6 @@ class GmresRun final : public GmresStepper {
     std::vector<DevArray<double2>> hcols_;
     DevArray<VT *> d_slabs_;
     DevArray<double2 *> d_hcols_;
-    std::vector<VT *> h_slabs_;
-    std::vector<double2 *> h_hcols_;
 };
 
 std::unique_ptr<GmresStepper> make_gmres(plx_geom *g, const GmresRequest &rq, const double *d_B, double *d_X,
@@ -1231,6 +1260,7 @@ void gmres_batched(plx_geom *g, const GmresRequest &rq, const double *d_B, doubl
         OpInput in = run->pre();
         apply_operator(in.g, in.b, in.X, in.Y, in.work, in.how, in.presplit);
         run->post();
+        run->settle();
     }
     run->end();
 }

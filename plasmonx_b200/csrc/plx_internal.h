@@ -75,6 +75,24 @@ struct DevArray {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+// Pinned host doubles that kernels of the context write and the host reads after
+// a synchronisation (zero copy).  Blocks of up to kPinnedKeep doubles go back to
+// the context's list (kPinnedBlocks at most), which its destruction frees: pinning
+// memory costs more than a small solve's step.
+struct PinnedArray {
+    plx_ctx *ctx = nullptr;
+    double *p = nullptr;
+    size_t n = 0;
+    PinnedArray() = default;
+    PinnedArray(const PinnedArray &) = delete;
+    PinnedArray &operator=(const PinnedArray &) = delete;
+    ~PinnedArray() { release(); }
+    void alloc(plx_ctx *c, size_t count);
+    void release();
+};
+constexpr size_t kPinnedKeep = 8192;      // 64 KB
+constexpr size_t kPinnedBlocks = 32;
+
 }  // namespace plx
 
 // Constants of an ordered atom-type pair (type of i, type of j), the table
@@ -99,6 +117,8 @@ struct plx_ctx {
     // they give up (plx_set_wait_limit)
     static constexpr uint32_t kDefaultWaitLimit = 1u << 22;
     uint32_t wait_limit = kDefaultWaitLimit;
+    std::mutex pinned_mutex;
+    std::vector<std::pair<double *, size_t>> pinned;   // free blocks of PinnedArray
     // contraction profiling (plx_profile_enable)
     bool profile = false;
     std::vector<cudaEvent_t> prof_events;   // pairs (start, stop), reused
@@ -341,13 +361,15 @@ struct OpInput {
 };
 // A batched GMRES advanced one Arnoldi step at a time (make_gmres has run the
 // set-up): while wants_product(): pre() returns the batch to multiply, the
-// caller writes its product to OpInput::Y, then post(); finally end().  B, X
-// and res must outlive the stepper.
+// caller writes its product to OpInput::Y, then post(), which queues the step,
+// and settle(), which waits for it; finally end().  B, X and res must outlive
+// the stepper.
 struct GmresStepper {
     virtual ~GmresStepper() = default;
     virtual bool wants_product() const = 0;
     virtual OpInput pre() = 0;
     virtual void post() = 0;
+    virtual void settle() = 0;
     virtual void end() = 0;
 };
 std::unique_ptr<GmresStepper> make_gmres(plx_geom *g, const GmresRequest &rq, const double *d_B, double *d_X,
@@ -417,7 +439,7 @@ struct RefineState {
 
 // One outer refinement step over a state's ACTIVE slots: begin() (false when
 // none is active), then while advance(&need): the caller computes the inner
-// operator product `need` and calls product_done(); advance() returning false
+// operator product `need` and calls product_done(), then settle(); advance() returning false
 // means the step (inner cycles, x += d, FP64 residual) is complete.
 class OuterStep {
   public:
@@ -426,6 +448,7 @@ class OuterStep {
     bool begin();
     bool advance(OpInput *need);
     void product_done();
+    void settle();
 
   private:
     RefineState &s_;

@@ -338,6 +338,8 @@ bool OuterStep::advance(OpInput *need) {
 
 void OuterStep::product_done() { run_->post(); }
 
+void OuterStep::settle() { run_->settle(); }
+
 // ---------------------------------------------------------------------------
 
 void refine_group_step(const std::vector<RefineState *> &states) {
@@ -360,7 +362,9 @@ void refine_group_step(const std::vector<RefineState *> &states) {
         }
         if (need.empty()) break;
         apply_operator_group(need);
+        // every state's step is queued before the first wait
         for (OuterStep *os : who) os->product_done();
+        for (OuterStep *os : who) os->settle();
     }
 }
 
@@ -391,6 +395,7 @@ void solve_refined(plx_geom *g, const RefineRequest &rq, const double *d_B, doub
         while (os.advance(&need)) {
             apply_operator(need.g, need.b, need.X, need.Y, need.work, need.how, need.presplit);
             os.product_done();
+            os.settle();
         }
     }
     for (int c = 0; c < C; ++c) {
