@@ -27,6 +27,7 @@
 #include <memory>
 #include <type_traits>
 
+#include "pdl.cuh"
 #include "plx_internal.h"
 
 namespace plx {
@@ -88,6 +89,7 @@ __device__ __forceinline__ void split_column(const TcColumns &sp, int k, int r, 
 template <typename VT>
 __global__ void gather_cols(int n, const int32_t *__restrict__ act, const VT *__restrict__ slab,
                             const double *__restrict__ P, double *__restrict__ X, TcColumns sp) {
+    pdl_sync();
     const int k = blockIdx.y, c = act[k];
     const VT *src = slab + (int64_t)c * 2 * n;
     const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
@@ -120,6 +122,7 @@ __global__ void __launch_bounds__(kThreads) dots_partial(int n, int i0, int i1,
                                                          VT *const *__restrict__ slabs,
                                                          const double *__restrict__ W,
                                                          double2 *__restrict__ part) {
+    pdl_sync();
     __shared__ double2 red[kThreads / 32][32];
     const int k = blockIdx.y, c = act[k];
     const int r0 = blockIdx.x * kDotRows;
@@ -179,6 +182,7 @@ __global__ void __launch_bounds__(kThreads) dots_wide(int n, int i0, int i1,
                                                       VT *const *__restrict__ slabs,
                                                       const double *__restrict__ W,
                                                       double2 *__restrict__ part) {
+    pdl_sync();
     __shared__ double wsh[2][kDotRows];
     const int k = blockIdx.y, c = act[k];
     const int r0 = blockIdx.x * kDotRows;
@@ -230,6 +234,7 @@ __global__ void __launch_bounds__(kThreads) dots_wide(int n, int i0, int i1,
 __global__ void dots_finish(int nchunk, int ni, int i0, const int32_t *__restrict__ act,
                             const double2 *__restrict__ part, double2 *__restrict__ h,
                             double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    pdl_sync();
     int k = blockIdx.y;
     int ii = blockIdx.x * blockDim.x + threadIdx.x;
     if (ii >= ni) return;
@@ -304,6 +309,7 @@ __device__ __forceinline__ double2 conj_prod(double vr, double vi, double wr, do
 // lane a row) add them in order; a thread per row and all its loads left 44 CTAs at 2,800 unknowns and 4 columns (36 us a launch, now 12.6 us; 893
 // unknowns, 61 columns 27 -> 19 us).
 constexpr int kChainRows = 32, kChainVec = 32;
+constexpr size_t kChainSmem = 2 * kChainVec * 2 * kChainRows * sizeof(double);       // combine_chain's static part
 template <bool FIN>
 __global__ void __launch_bounds__(kThreads) combine_chain(int n, int i0, int ni, int hld, int hoff,
                                                           const int32_t *__restrict__ act,
@@ -311,6 +317,7 @@ __global__ void __launch_bounds__(kThreads) combine_chain(int n, int i0, int ni,
                                                           const double2 *__restrict__ h, int ndot, double sign,
                                                           double *__restrict__ Y, int by_col,
                                                           double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    pdl_sync();
     extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
     __shared__ double ps[2][kChainVec][2][kChainRows];
     const double **col = reinterpret_cast<const double **>(sh + ni);
@@ -372,6 +379,7 @@ __global__ void __launch_bounds__(kThreads) combine_inner(int n, int i0, int ni,
                                                           const double2 *__restrict__ h, int ndot, double sign,
                                                           double *__restrict__ Y, int by_col, double *__restrict__ npart,
                                                           double2 *__restrict__ Hcol, int hstride, int accumulate) {
+    pdl_sync();
     constexpr int RB = kThreads / G;
     extern __shared__ double2 sh[];                       // ni coefficients, then ni column pointers
     __shared__ double2 red[G > 1 ? kThreads : 1];
@@ -445,6 +453,7 @@ __global__ void __launch_bounds__(CHUNKS * kThreads) mgs_column(int n, int j, co
                                                                 double *const *__restrict__ slabs,
                                                                 double *__restrict__ W, double2 *__restrict__ Hcol,
                                                                 int hstride) {
+    pdl_sync();
     constexpr int kWarps = kThreads / 32;
     __shared__ double2 red[2][CHUNKS][kWarps];
     const int k = blockIdx.x, c = act[k];
@@ -526,6 +535,7 @@ __device__ __forceinline__ double norm_chunk(int n, const double *__restrict__ w
 
 __global__ void __launch_bounds__(kThreads) norm_partial(int n, const double *__restrict__ W,
                                                          double *__restrict__ part) {
+    pdl_sync();
     const int k = blockIdx.y;
     const double s = norm_chunk(n, W + (int64_t)k * 2 * n, blockIdx.x);
     if (threadIdx.x == 0) part[(int64_t)k * gridDim.x + blockIdx.x] = s;
@@ -534,6 +544,7 @@ __global__ void __launch_bounds__(kThreads) norm_partial(int n, const double *__
 // `host`: the same norms in the run's pinned block
 __global__ void norm_finish(int nchunk, int count, const double *__restrict__ part,
                             double *__restrict__ out, double *__restrict__ host) {
+    pdl_sync();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     double s = 0.0;
@@ -709,6 +720,7 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
                                                              int hstride, double *__restrict__ cs,
                                                              double2 *__restrict__ sn, double2 *__restrict__ g,
                                                              int gstride, int cstride, double *__restrict__ resid) {
+    pdl_sync();
     constexpr bool kInner = sizeof(VT) == 4;
     __shared__ double total;
     __shared__ Rotation rot[kInner ? 1 : 32];
@@ -778,6 +790,7 @@ __global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t
                                                  double2 *const *__restrict__ Hcols, int hstride,
                                                  const double2 *__restrict__ g, int gstride,
                                                  double2 *__restrict__ y) {
+    pdl_sync();
     extern __shared__ double2 ys[];
     __shared__ double2 tri[kTriB][kTriB + 1];        // tri[column][row]
     const int k = blockIdx.x;
@@ -847,6 +860,7 @@ int tri_threads(int m) { return std::min(256, std::max(64, (m + 31) / 32 * 32));
 // R[k] = B[c] - AX[k] with c = act[k]; in place into AX.
 __global__ void residual(int n, const int32_t *__restrict__ act, const double *__restrict__ B,
                          double *__restrict__ AX) {
+    pdl_sync();
     int k = blockIdx.y, c = act[k];
     const double *b = B + (int64_t)c * 2 * n;
     double *r = AX + (int64_t)k * 2 * n;
@@ -857,6 +871,7 @@ __global__ void residual(int n, const int32_t *__restrict__ act, const double *_
 
 __global__ void gather_x(int n, const int32_t *__restrict__ act, const double *__restrict__ X,
                          double *__restrict__ out) {
+    pdl_sync();
     int k = blockIdx.y;
     const double *src = X + (int64_t)act[k] * 2 * n;
     double *dst = out + (int64_t)k * 2 * n;
@@ -869,6 +884,7 @@ __global__ void gather_x(int n, const int32_t *__restrict__ act, const double *_
 // when by_col (Y indexed by idx[k]).
 __global__ void scale_cols(int n, const int32_t *__restrict__ idx, const double *__restrict__ P,
                            double *__restrict__ Y, int by_col) {
+    pdl_sync();
     int k = blockIdx.y, c = idx[k];
     const double *p = P + (int64_t)c * 2 * n;
     double *y = Y + (int64_t)(by_col ? c : k) * 2 * n;
@@ -890,7 +906,7 @@ int combine_blocks(int n, int ni) { return n_blocks(n, kThreads / combine_groups
 // npart: norm partials of the last launch (FP32 basis).
 constexpr int kCombine = 1024;
 template <typename VT>
-int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const int32_t *act,
+int64_t combine_chunked(cudaStream_t st, int sms, int n, int i0, int ni, int count, const int32_t *act,
                         VT *const *slabs, const double2 *h, double sign, double *Y, int by_col,
                         int ndot = 0, double *npart = nullptr, double2 *Hcol = nullptr, int hstride = 0,
                         int accumulate = 0) {
@@ -901,15 +917,17 @@ int64_t combine_chunked(cudaStream_t st, int n, int i0, int ni, int count, const
         const size_t smem = cn * (sizeof(double2) + sizeof(VT *));
         if constexpr (std::is_same<VT, double>::value) {
             const dim3 grid(n_blocks(n, kChainRows), count);
-            (ndot ? combine_chain<true> : combine_chain<false>)<<<grid, kThreads, smem, st>>>(
-                n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, Hcol, hstride, accumulate);
+            // a few blocks an SM: unevenly spread they took 19.6 us at 2,800 unknowns x 4 columns, now 12.6
+            const size_t even = even_smem((int64_t)grid.x * count, sms, kChainSmem, smem);
+            launch_pdl((ndot ? combine_chain<true> : combine_chain<false>), grid, kThreads, even, st,
+                       n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, Hcol, hstride, accumulate);
         } else {
             const int G = combine_groups(n, ni);
             const dim3 grid(n_blocks(n, kThreads / G), count);
             double *np = c0 + cn == ni ? npart : nullptr;
 #define PLX_COMBINE(GG, FIN)                                                                                    \
-    combine_inner<GG, FIN><<<grid, kThreads, smem, st>>>(n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, Y, by_col, \
-                                                         np, Hcol, hstride, accumulate)
+    launch_pdl(combine_inner<GG, FIN>, grid, kThreads, smem, st, n, i0 + c0, cn, ni, c0, act, slabs, h, ndot, sign, \
+               Y, by_col, np, Hcol, hstride, accumulate)
             if (G == 4 && ndot) PLX_COMBINE(4, true);
             else if (G == 4) PLX_COMBINE(4, false);
             else if (ndot) PLX_COMBINE(1, true);
@@ -929,8 +947,8 @@ static void batch_norms(plx_geom *g, int count, const double *V, DevArray<double
     plx_ctx *ctx = g->ctx;
     const int n = g->n_var;
     int nchunk = n_blocks(n, kRows);
-    norm_partial<<<dim3(nchunk, count), kThreads, 0, ctx->stream>>>(n, V, part.p);
-    norm_finish<<<n_blocks(count, 128), 128, 0, ctx->stream>>>(nchunk, count, part.p, out.p, host);
+    launch_pdl(norm_partial, dim3(nchunk, count), kThreads, 0, ctx->stream, n, V, part.p);
+    launch_pdl(norm_finish, n_blocks(count, 128), 128, 0, ctx->stream, nchunk, count, part.p, out.p, host);
     ctx->launches += 2;
 }
 
@@ -954,13 +972,14 @@ class GmresRun final : public GmresStepper {
         res_.trace.assign(rq_.record_trace ? (size_t)C_ * m_ : 0, 0.0);
         if (C_ == 0) return;
         if (m_ < 1) throw Error(PLX_ERR_ARG, "GMRES dimension must be positive");
+        sms_ = sm_count(ctx_->device);
         nchunk_ = n_blocks(n, kRows);
         ndot_ = n_blocks(n, kDotRows);
         if ((size_t)(m_ + 1) * sizeof(double2) > 200 * 1024) throw Error(PLX_ERR_ARG, "GMRES dimension above 12800");
         once_per_device(reinterpret_cast<const void *>(tri_solve), ctx_->device, [] {
             PLX_CHECK_CUDA(cudaFuncSetAttribute(tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024));
-            PLX_CHECK_CUDA(cudaFuncSetAttribute(combine_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024));
+            for (auto kern : {combine_chain<true>, combine_chain<false>})
+                PLX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024));
         });
         hstride_ = m_ + 1;   // rows of an H column (0..m)
         d_act_.alloc(ctx_, C_);
@@ -1022,8 +1041,8 @@ class GmresRun final : public GmresStepper {
         const int n = g_->n_var;
         const int na = (int)act_.size();
         if (!x_ready_) {
-            gather_cols<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(n, d_act_.p, slabs_[j_].p,
-                                                                     jac_ ? Pinv_.p : nullptr, Xa_.p, split_);
+            launch_pdl(gather_cols<VT>, dim3(grid_rows(n), na), 256, 0, st_, n, d_act_.p, slabs_[j_].p,
+                       jac_ ? Pinv_.p : nullptr, Xa_.p, split_);
             ctx_->launches++;
         }
         return OpInput{g_, OpBatch{na, d_freq_act_.p}, Xa_.p, Wa_.p, work_.p, rq_.contraction, split_.hi != nullptr};
@@ -1045,21 +1064,21 @@ class GmresRun final : public GmresStepper {
             const int ni = i1 - i0;
             if (ni >= 8) {
                 const int nz = std::max(1, std::min(n_blocks(ni, kThreads / 32), n_blocks(592, ndot_ * na)));
-                dots_wide<VT><<<dim3(ndot_, na, nz), kThreads, 0, st_>>>(n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p,
-                                                                         part_.p);
+                launch_pdl(dots_wide<VT>, dim3(ndot_, na, nz), kThreads, 0, st_, n, i0, i1, d_act_.p, d_slabs_.p,
+                           Wa_.p, part_.p);
             } else {
-                dots_partial<VT><<<dim3(ndot_, na), kThreads, 0, st_>>>(n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p,
-                                                                        part_.p);
+                launch_pdl(dots_partial<VT>, dim3(ndot_, na), kThreads, 0, st_, n, i0, i1, d_act_.p, d_slabs_.p, Wa_.p,
+                           part_.p);
             }
             ctx_->launches++;
             const bool fin = ndot_ <= kCombineFin && ni <= kCombine;
             if (!fin) {
-                dots_finish<<<dim3(n_blocks(ni, 128), na), 128, 0, st_>>>(ndot_, ni, i0, d_act_.p, part_.p, hbuf_.p,
-                                                                           hcols_[j].p, hstride_, accumulate);
+                launch_pdl(dots_finish, dim3(n_blocks(ni, 128), na), 128, 0, st_, ndot_, ni, i0, d_act_.p, part_.p,
+                           hbuf_.p, hcols_[j].p, hstride_, accumulate);
                 ctx_->launches++;
             }
             if (last) nparts = combine_blocks(n, ni);
-            ctx_->launches += combine_chunked(st_, n, i0, ni, na, d_act_.p, d_slabs_.p, fin ? part_.p : hbuf_.p, -1.0,
+            ctx_->launches += combine_chunked(st_, sms_, n, i0, ni, na, d_act_.p, d_slabs_.p, fin ? part_.p : hbuf_.p, -1.0,
                                               Wa_.p, 0, fin ? ndot_ : 0, last ? nrm_part_.p : nullptr, hcols_[j].p,
                                               hstride_, accumulate);
         };
@@ -1074,7 +1093,7 @@ class GmresRun final : public GmresStepper {
         if (std::is_same<VT, double>::value) {
             nparts = 0;
             if (nchunk_ > kNormChunks) {
-                norm_partial<<<dim3(nchunk_, na), kThreads, 0, st_>>>(n, Wa_.p, nrm_part_.p);
+                launch_pdl(norm_partial, dim3(nchunk_, na), kThreads, 0, st_, n, Wa_.p, nrm_part_.p);
                 ctx_->launches++;
                 nparts = nchunk_;
             }
@@ -1082,8 +1101,8 @@ class GmresRun final : public GmresStepper {
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
         for (int k = 0; k < na; ++k) memcpy(host_.p + k, &kPending, 8);
         prof_begin(ctx_);
-        normalize_givens<VT><<<dim3(grid_rows(n), na), 256, 0, st_>>>(
-            n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p,
+        launch_pdl(
+            normalize_givens<VT>, dim3(grid_rows(n), na), 256, 0, st_, n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p,
             d_hcols_.p, hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, host_.p);
         ctx_->launches++;
         x_ready_ = true;
@@ -1114,11 +1133,11 @@ class GmresRun final : public GmresStepper {
             // inner solve of a refinement: take the least-squares solution as is
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            tri_solve<<<nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
-                                                                  hstride_, ybuf_.p);
-            ctx_->launches += 1 + combine_chunked(st_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
+            launch_pdl(tri_solve, nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
+                       hstride_, gv_.p, hstride_, ybuf_.p);
+            ctx_->launches += 1 + combine_chunked(st_, sms_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
             if (jac_) {
-                scale_cols<<<dim3(grid_rows(n), nt), 256, 0, st_>>>(n, d_cols_.p, Pinv_.p, d_X_, 1);
+                launch_pdl(scale_cols, dim3(grid_rows(n), nt), 256, 0, st_, n, d_cols_.p, Pinv_.p, d_X_, 1);
                 ctx_->launches++;
             }
             for (int c : trig) done[c] = 1;
@@ -1130,10 +1149,10 @@ class GmresRun final : public GmresStepper {
             x_ready_ = false;                 // the true residual's product uses the input buffer
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            tri_solve<<<nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_>>>(nt, j, d_cols_.p, d_hcols_.p, hstride_, gv_.p,
-                                                                  hstride_, ybuf_.p);
-            ctx_->launches += combine_chunked(st_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
-            gather_x<<<dim3(grid_rows(2LL * n), nt), 256, 0, st_>>>(n, d_cols_.p, d_X_, Xa_.p);
+            launch_pdl(tri_solve, nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
+                       hstride_, gv_.p, hstride_, ybuf_.p);
+            ctx_->launches += combine_chunked(st_, sms_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
+            launch_pdl(gather_x, dim3(grid_rows(2LL * n), nt), 256, 0, st_, n, d_cols_.p, d_X_, Xa_.p);
             ctx_->launches += 2;
             std::vector<int32_t> tf(nt);
             for (int t = 0; t < nt; ++t) tf[t] = rq_.freq[trig[t]];
@@ -1145,7 +1164,7 @@ class GmresRun final : public GmresStepper {
                            Contraction::FP64 == rq_.contraction || Contraction::FP64_OTF == rq_.contraction
                                ? rq_.contraction
                                : Contraction::FP64);
-            residual<<<dim3(grid_rows(2LL * n), nt), 256, 0, st_>>>(n, d_cols_.p, d_B_, Wa_.p);
+            launch_pdl(residual, dim3(grid_rows(2LL * n), nt), 256, 0, st_, n, d_cols_.p, d_B_, Wa_.p);
             ctx_->launches++;
             const double *tres = host_.p + C_;
             batch_norms(g_, nt, Wa_.p, nrm_part_, nrm_, host_.p + C_);
@@ -1180,7 +1199,8 @@ class GmresRun final : public GmresStepper {
         if constexpr (std::is_same<VT, double>::value) {
             const int n = g_->n_var;
             if (n > 4 * kDotRows) return false;
-#define PLX_MGS(Q) mgs_column<Q><<<na, Q * kThreads, 0, st_>>>(n, j, d_act_.p, d_slabs_.p, Wa_.p, hcols_[j].p, hstride_)
+#define PLX_MGS(Q)                                                                                             \
+    launch_pdl(mgs_column<Q>, na, Q * kThreads, 0, st_, n, j, d_act_.p, d_slabs_.p, Wa_.p, hcols_[j].p, hstride_)
             if (n <= kDotRows) PLX_MGS(1);
             else if (n <= 2 * kDotRows) PLX_MGS(2);
             else PLX_MGS(4);
@@ -1226,7 +1246,7 @@ class GmresRun final : public GmresStepper {
     const double *d_B_;
     double *d_X_;
     GmresResult &res_;
-    int C_ = 0, m_ = 0, j_ = 0, nchunk_ = 0, ndot_ = 0, hstride_ = 0;
+    int sms_ = 1, C_ = 0, m_ = 0, j_ = 0, nchunk_ = 0, ndot_ = 0, hstride_ = 0;
     bool jac_ = false;
     TcColumns split_{nullptr, nullptr, 0};   // tensor-core runs: the split rows of the next input
     bool x_ready_ = false;      // Xa holds the next product's input

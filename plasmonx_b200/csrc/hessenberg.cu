@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "pdl.cuh"
 #include "plx_internal.h"
 #include "warp_sums.cuh"
 
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
                                               double *__restrict__ beta, double *__restrict__ sub,
                                               double *__restrict__ yp, double *__restrict__ zp,
                                               double *__restrict__ sp) {
+    pdl_sync();
     extern __shared__ double sm[];
     __shared__ double red[kT / 32], yred[kT / kHR][kHR];
     double *vr = sm, *vc = vr + t.rt, *zs = vc + t.ct;        // rt, ct, 2 ct
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, doub
                                                 const double *__restrict__ vbuf, const double *__restrict__ beta,
                                                 const double *__restrict__ yp, const double *__restrict__ zp,
                                                 const double *__restrict__ sp, double *__restrict__ npart) {
+    pdl_sync();
     extern __shared__ double sm[];
     __shared__ double red[kT / 32];
     // rt, rt, ct, ct, and the partial sums' sums: 4 rt, 8 ct
@@ -543,8 +546,8 @@ void build_hessenberg(plx_geom *g) {
         const int c0 = (k + 1) / t.ct;                        // first column tile with columns right of k
         const dim3 grid(t.ncc - c0, t.nrc);
         double *np0 = npart.p + (k & 1) * t.nrc, *np1 = npart.p + ((k + 1) & 1) * t.nrc;
-        hh_gemv<<<grid, kT, sm_gemv, st>>>(t, k, c0, E.p, np0, vbuf.p, beta.p, sub.p, yp.p, zp.p, sp.p);
-        hh_update<<<grid, kT, sm_upd, st>>>(t, k, c0, E.p, vbuf.p, beta.p, yp.p, zp.p, sp.p, np1);
+        launch_pdl(hh_gemv, grid, kT, sm_gemv, st, t, k, c0, E.p, np0, vbuf.p, beta.p, sub.p, yp.p, zp.p, sp.p);
+        launch_pdl(hh_update, grid, kT, sm_upd, st, t, k, c0, E.p, vbuf.p, beta.p, yp.p, zp.p, sp.p, np1);
         ctx->launches += 2;
     }
     g->d_hess_q.alloc(ctx, (size_t)n * n);

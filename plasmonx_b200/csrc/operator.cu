@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "pair_tiles.cuh"
+#include "pdl.cuh"
 #include "plx_internal.h"
 #include "skinny.cuh"
 #include "warp_sums.cuh"
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(32 * kOtfWarps) otf_contract(int N, int wt, in
                                                                const int32_t *__restrict__ type,
                                                                const PairWidths *__restrict__ widths,
                                                                const double *__restrict__ X, double *__restrict__ S) {
+    pdl_sync();
     constexpr int NC = FMU ? 4 : 1;            // components per atom
     constexpr int V = NC * 2 * CB;             // values per target: [component][part][column]
     __shared__ double red[kOtfWarps][V];
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(256) charge_rows(int N, int nt, int nv, int co
                                                    const Cplx *__restrict__ wratio, const Cplx *__restrict__ dq,
                                                    const double *__restrict__ S, const double *__restrict__ X,
                                                    double *__restrict__ Y, double sign, int add_diag) {
+    pdl_sync();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= N) return;
@@ -357,6 +360,7 @@ __global__ void dipole_rows(int N, int nt, int nv, int count, const int32_t *__r
                             const double *__restrict__ frac, const Cplx *__restrict__ inv_alpha,
                             const double *__restrict__ S, const double *__restrict__ X,
                             double *__restrict__ Y) {
+    pdl_sync();
     int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int c = blockIdx.y;
     if (e >= 3LL * N || c >= count) return;
@@ -387,6 +391,7 @@ __global__ void iface_rows(int nx, int count, int nt, int nv, int64_t ldS, const
                            const int32_t *__restrict__ xcol, const int32_t *__restrict__ xtj,
                            const double *__restrict__ xkt, const Cplx *__restrict__ wratio,
                            const double *__restrict__ S, double *__restrict__ Y) {
+    pdl_sync();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
     if (t >= nx || c >= count) return;
@@ -587,7 +592,7 @@ void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const
     double *part = scratch.p;
     cudaStream_t st = ctx->stream;
     launch_product_partial(st, R, n, ks, kchunk, X, T, part);
-    skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, ks, part, S);
+    launch_pdl(skinny_reduce, n_blocks((int64_t)R * n, 256), 256, 0, st, n, R, ks, part, S);
     ctx->launches += 2;
     PLX_CHECK_CUDA(cudaGetLastError());
 }
@@ -634,14 +639,14 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
                 else PLX_OTF(64, false)
             }
 #undef PLX_OTF
-            skinny_reduce<<<n_blocks((int64_t)R * n, 256), 256, 0, st>>>(n, R, js, g->d_part.p, S);
+            launch_pdl(skinny_reduce, n_blocks((int64_t)R * n, 256), 256, 0, st, n, R, js, g->d_part.p, S);
             ctx->launches += 2;
             PLX_CHECK_CUDA(cudaGetLastError());
             return;
         }
         const int wt = otf_warps(N), blocks = n_blocks(N, kOtfWarps / wt);
 #define PLX_OTF(CB, F)                                                                                            \
-    otf_contract<CB, F><<<blocks, 32 * kOtfWarps, 0, st>>>(N, wt, count, n, g->n_types, g->d_pos.p, g->d_par.p, \
+    launch_pdl(otf_contract<CB, F>, blocks, 32 * kOtfWarps, 0, st, N, wt, count, n, g->n_types, g->d_pos.p, g->d_par.p, \
                                                            g->d_type.p, g->d_widths.p, X, S)
         if (fmu) {
             if (count == 1) PLX_OTF(1, true);
@@ -667,14 +672,14 @@ static void finish_rows(plx_geom *g, const OpBatch &b, const double *S, const do
     cudaStream_t st = ctx->stream;
     const int N = g->n_atoms, nv = g->n_var;
     dim3 gq(n_blocks((int64_t)N * 32, 256), n_blocks(b.count, kChargeCols));
-    (g->n_types > 1 ? charge_rows<true> : charge_rows<false>)<<<gq, 256, 0, st>>>(N, g->n_types, nv, b.count, b.d_freq,
-                                    g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p,
-                                    g->d_ktval.p, g->d_wratio.p, g->d_dq.p, S, X, Y, 1.0, 1);
+    launch_pdl(g->n_types > 1 ? charge_rows<true> : charge_rows<false>, gq, 256, 0, st, N, g->n_types, nv, b.count,
+               b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_wratio.p, g->d_dq.p, S,
+               X, Y, 1.0, 1);
     ctx->launches++;
     if (g->model == PLX_WFQFMU) {
         dim3 gm(n_blocks(3LL * N, 256), b.count);
-        dipole_rows<<<gm, 256, 0, st>>>(N, g->n_types, nv, b.count, b.d_freq, g->d_frac.p,
-                                        g->d_inv_alpha.p, S, X, Y);
+        launch_pdl(dipole_rows, gm, 256, 0, st, N, g->n_types, nv, b.count, b.d_freq, g->d_frac.p, g->d_inv_alpha.p, S,
+                   X, Y);
         ctx->launches++;
     }
     PLX_CHECK_CUDA(cudaGetLastError());
@@ -697,9 +702,9 @@ static void folded_finish(plx_geom *g, const OpBatch &b, const double *S, double
     if (g->n_xrows == 0) return;
     plx_ctx *ctx = g->ctx;
     prof_begin(ctx);
-    iface_rows<<<dim3(n_blocks(g->n_xrows, 128), b.count), 128, 0, ctx->stream>>>(
-        g->n_xrows, b.count, g->n_types, g->n_var, g->fold_rows, b.d_freq, g->d_type.p, g->d_xrow.p, g->d_xipos.p,
-        g->d_xrowptr.p, g->d_xcol.p, g->d_xtj.p, g->d_xkt.p, g->d_wratio.p, S, Y);
+    launch_pdl(iface_rows, dim3(n_blocks(g->n_xrows, 128), b.count), 128, 0, ctx->stream, g->n_xrows, b.count,
+               g->n_types, g->n_var, g->fold_rows, b.d_freq, g->d_type.p, g->d_xrow.p, g->d_xipos.p, g->d_xrowptr.p,
+               g->d_xcol.p, g->d_xtj.p, g->d_xkt.p, g->d_wratio.p, S, Y);
     ctx->launches++;
     PLX_CHECK_CUDA(cudaGetLastError());
     prof_end(ctx, PROF_ROWS, 0.0, 0.0);
@@ -806,9 +811,9 @@ void rhs_batch(plx_geom *g, const OpBatch &b, const int32_t *d_pol, double *Bout
         N, nv, b.count, d_pol, g->d_pos.p, g->e0, g->rhs_potential, mn[0], mn[1], mn[2], V.p);
     dim3 gq(n_blocks((int64_t)N * 32, 256), n_blocks(b.count, kChargeCols));
     // b_q = -Kop(w) V  (rhs_module.f90:140-390); no diagonal term
-    (g->n_types > 1 ? charge_rows<true> : charge_rows<false>)<<<gq, 256, 0, st>>>(N, g->n_types, nv, b.count, b.d_freq,
-                                    g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p,
-                                    g->d_ktval.p, g->d_wratio.p, g->d_dq.p, V.p, V.p, Bout, -1.0, 0);
+    launch_pdl(g->n_types > 1 ? charge_rows<true> : charge_rows<false>, gq, 256, 0, st, N, g->n_types, nv, b.count,
+               b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_wratio.p, g->d_dq.p,
+               V.p, V.p, Bout, -1.0, 0);
     ctx->launches += 2;
     if (g->model == PLX_WFQFMU) {
         dim3 gm(n_blocks(3LL * N, 256), b.count);

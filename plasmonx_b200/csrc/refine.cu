@@ -29,6 +29,7 @@
 #include <cmath>
 #include <memory>
 
+#include "pdl.cuh"
 #include "plx_internal.h"
 
 namespace plx {
@@ -37,6 +38,7 @@ namespace {
 
 __global__ void gather_idx(int n, const int32_t *__restrict__ idx, const double *__restrict__ src,
                            double *__restrict__ dst) {
+    pdl_sync();
     int k = blockIdx.y;
     const double *s = src + (int64_t)idx[k] * 2 * n;
     double *d = dst + (int64_t)k * 2 * n;
@@ -46,6 +48,7 @@ __global__ void gather_idx(int n, const int32_t *__restrict__ idx, const double 
 
 __global__ void scatter_add(int n, const int32_t *__restrict__ idx, const double *__restrict__ src,
                             double *__restrict__ dst) {
+    pdl_sync();
     int k = blockIdx.y;
     const double *s = src + (int64_t)k * 2 * n;
     double *d = dst + (int64_t)idx[k] * 2 * n;
@@ -56,6 +59,7 @@ __global__ void scatter_add(int n, const int32_t *__restrict__ idx, const double
 // out[k] = B[idx[k]] - AX[k] (compact restart right-hand sides)
 __global__ void compact_residual(int n, const int32_t *__restrict__ idx, const double *__restrict__ B,
                                  const double *__restrict__ AX, double *__restrict__ out) {
+    pdl_sync();
     int k = blockIdx.y;
     const double *b = B + (int64_t)idx[k] * 2 * n;
     const double *a = AX + (int64_t)k * 2 * n;
@@ -67,6 +71,7 @@ __global__ void compact_residual(int n, const int32_t *__restrict__ idx, const d
 // R[idx[k]] = B[idx[k]] - AX[k]
 __global__ void scatter_residual(int n, const int32_t *__restrict__ idx, const double *__restrict__ B,
                                  const double *__restrict__ AX, double *__restrict__ R) {
+    pdl_sync();
     int k = blockIdx.y;
     int c = idx[k];
     const double *b = B + (int64_t)c * 2 * n;
@@ -79,6 +84,7 @@ __global__ void scatter_residual(int n, const int32_t *__restrict__ idx, const d
 // ||v_idx[k]||_2 for every listed slot, one block per slot (fixed summation order).
 __global__ void column_norms(int n, const int32_t *__restrict__ idx, const double *__restrict__ V,
                              double *__restrict__ out) {
+    pdl_sync();
     int k = blockIdx.x;
     const double *v = V + (int64_t)idx[k] * 2 * n;
     double s = 0.0;
@@ -181,7 +187,7 @@ void RefineState::update_status() {
     if (idx.empty()) return;
     const int k = (int)idx.size();
     PLX_CHECK_CUDA(cudaMemcpyAsync(d_idx.p, idx.data(), k * 4, cudaMemcpyHostToDevice, st));
-    column_norms<<<k, 256, 0, st>>>(n, d_idx.p, R.p, nrm.p);
+    launch_pdl(column_norms, k, 256, 0, st, n, d_idx.p, R.p, nrm.p);
     ctx->launches++;
     std::vector<double> rn(k);
     PLX_CHECK_CUDA(cudaMemcpyAsync(rn.data(), nrm.p, k * 8, cudaMemcpyDeviceToHost, st));
@@ -245,7 +251,7 @@ bool OuterStep::begin() {
     }
     PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_idx.p, act_.data(), na * 4, cudaMemcpyHostToDevice, st));
     PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_fa.p, fa_.data(), na * 4, cudaMemcpyHostToDevice, st));
-    gather_idx<<<dim3(grid_cols(n), na), 256, 0, st>>>(n, S.d_idx.p, S.R.p, S.Ba.p);
+    launch_pdl(gather_idx, dim3(grid_cols(n), na), 256, 0, st, n, S.d_idx.p, S.R.p, S.Ba.p);
     ctx->launches++;
     cur_.resize(na);
     for (int k = 0; k < na; ++k) cur_[k] = k;
@@ -277,7 +283,7 @@ bool OuterStep::advance(OpInput *need) {
                 PLX_CHECK_CUDA(cudaMemcpyAsync(S.Dacc.p, S.Da.p, (size_t)na * 2 * n * 8, cudaMemcpyDeviceToDevice, st));
             } else {
                 PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_sub.p, cur_.data(), cur_.size() * 4, cudaMemcpyHostToDevice, st));
-                scatter_add<<<dim3(grid_cols(n), (unsigned)cur_.size()), 256, 0, st>>>(n, S.d_sub.p, S.Da.p,
+                launch_pdl(scatter_add, dim3(grid_cols(n), (unsigned)cur_.size()), 256, 0, st, n, S.d_sub.p, S.Da.p,
                                                                                        S.Dacc.p);
                 ctx->launches++;
             }
@@ -295,10 +301,10 @@ bool OuterStep::advance(OpInput *need) {
                 PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_sub.p, sub.data(), ns * 4, cudaMemcpyHostToDevice, st));
                 PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_fsub.p, fsub.data(), ns * 4, cudaMemcpyHostToDevice, st));
                 // Bc = b_cycle[sub] - A d_cycle[sub]   (inner contraction)
-                gather_idx<<<dim3(grid_cols(n), ns), 256, 0, st>>>(n, S.d_sub.p, S.Da.p, S.AXa.p);
+                launch_pdl(gather_idx, dim3(grid_cols(n), ns), 256, 0, st, n, S.d_sub.p, S.Da.p, S.AXa.p);
                 ctx->launches++;
                 apply_operator(g, OpBatch{ns, S.d_fsub.p}, S.AXa.p, S.Da.p, S.Wc.p, S.rq.inner_contraction);
-                compact_residual<<<dim3(grid_cols(n), ns), 256, 0, st>>>(n, S.d_sub.p, bc_, S.Da.p, S.AXa.p);
+                launch_pdl(compact_residual, dim3(grid_cols(n), ns), 256, 0, st, n, S.d_sub.p, bc_, S.Da.p, S.AXa.p);
                 ctx->launches++;
                 PLX_CHECK_CUDA(cudaMemcpyAsync(S.Bc.p, S.AXa.p, (size_t)ns * 2 * n * 8, cudaMemcpyDeviceToDevice, st));
                 bc_ = S.Bc.p;
@@ -322,11 +328,11 @@ bool OuterStep::advance(OpInput *need) {
         // x += d ; FP64 residual r = b - A x of the active columns
         PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_idx.p, act_.data(), na * 4, cudaMemcpyHostToDevice, st));
         PLX_CHECK_CUDA(cudaMemcpyAsync(S.d_fa.p, fa_.data(), na * 4, cudaMemcpyHostToDevice, st));
-        scatter_add<<<dim3(grid_cols(n), na), 256, 0, st>>>(n, S.d_idx.p, S.Da.p, S.X);
-        gather_idx<<<dim3(grid_cols(n), na), 256, 0, st>>>(n, S.d_idx.p, S.X, S.Ba.p);
+        launch_pdl(scatter_add, dim3(grid_cols(n), na), 256, 0, st, n, S.d_idx.p, S.Da.p, S.X);
+        launch_pdl(gather_idx, dim3(grid_cols(n), na), 256, 0, st, n, S.d_idx.p, S.X, S.Ba.p);
         ctx->launches += 2;
         apply_operator(g, OpBatch{na, S.d_fa.p}, S.Ba.p, S.AXa.p, S.Da.p, S.rq.outer_contraction);
-        scatter_residual<<<dim3(grid_cols(n), na), 256, 0, st>>>(n, S.d_idx.p, S.B, S.AXa.p, S.R.p);
+        launch_pdl(scatter_residual, dim3(grid_cols(n), na), 256, 0, st, n, S.d_idx.p, S.B, S.AXa.p, S.R.p);
         ctx->launches++;
         PLX_CHECK_CUDA(cudaGetLastError());
         for (int c : act_) S.slots[c].outer += 1;

@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "dmma.cuh"
+#include "pdl.cuh"
 
 namespace plx {
 namespace {
@@ -33,6 +34,7 @@ template <int MT, int NT, int D, int WR, int MB>
 __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kchunk, const double *__restrict__ Xt,
                                                            const double *__restrict__ T,
                                                            double *__restrict__ part) {
+    pdl_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kk = lane & 3, g = lane >> 2;
     const int col0 = (blockIdx.x * (4 / WR) + warp / WR) * 8 * NT, row0 = (blockIdx.y * WR + warp % WR) * 8 * MT;
     const int k0 = blockIdx.z * kchunk, k1 = min(n, k0 + kchunk);
@@ -84,9 +86,9 @@ __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kch
 inline void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, const double *X, const double *T,
                                    double *part) {
 #define PLX_PP(MT, NT, D, WR, MB)                                                                                  \
-    product_partial<MT, NT, D, WR, MB><<<dim3((n + 32 / WR * NT - 1) / (32 / WR * NT),                             \
-                                              (R + 8 * MT * WR - 1) / (8 * MT * WR), ks),                          \
-                                         128, 0, st>>>(R, n, kchunk, X, T, part)
+    launch_pdl(product_partial<MT, NT, D, WR, MB>,                                                                 \
+               dim3((n + 32 / WR * NT - 1) / (32 / WR * NT), (R + 8 * MT * WR - 1) / (8 * MT * WR), ks), 128, 0, st, R, \
+               n, kchunk, X, T, part)
     if (R <= 8) PLX_PP(1, 4, 4, 1, 1);
     else if (R <= 16) PLX_PP(2, 4, 4, 1, 1);
     else if (R <= 24) PLX_PP(3, 4, 4, 1, 3);
@@ -98,6 +100,7 @@ inline void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kc
 
 __global__ void skinny_reduce(int n, int R, int ks, const double *__restrict__ part,
                               double *__restrict__ S) {
+    pdl_sync();
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)R * n) return;
     // the loads of eight partial sums together, added in order (64 of them one by one: 6.9 us

@@ -38,6 +38,7 @@
 
 #include "operand.cuh"
 #include "pair_tiles.cuh"
+#include "pdl.cuh"
 #include "plx_internal.h"
 
 namespace plx {
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_contract_kernel(const __grid
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_sync();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(tmem_cols)
@@ -533,6 +535,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_contract_kernel(const __grid
 // their own).
 constexpr int kRedCols = 8;
 __global__ void __launch_bounds__(kBM) reduce_pieces(const __grid_constant__ TcLaunch p) {
+    pdl_sync();
     const int t = p.full + blockIdx.x;                       // index in the launch's list
     const int g = group_of_tile(p, t);
     const TcGroup &G = p.grp[g];
@@ -695,12 +698,6 @@ CUtensorMap make_map(const void *ptr, uint64_t inner, uint64_t outer, uint64_t l
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Error(PLX_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     return m;
-}
-
-int sm_count(int device) {
-    int v = 0;
-    PLX_CHECK_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device));
-    return v > 0 ? v : 1;
 }
 
 // Schedule of the launch's tiles on `sms` SMs (one CTA per SM, see TcLaunch): whole
@@ -967,11 +964,11 @@ void tc_contract_group(const std::vector<TcItem> &items) {
     once_per_device(reinterpret_cast<const void *>(kern), ctx->device, [&] {
         PLX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     });
-    kern<<<ctas, kThreadsTc, smem, ctx->stream>>>(L);
+    launch_pdl(kern, ctas, kThreadsTc, smem, ctx->stream, L);
     ctx->launches++;
     PLX_CHECK_CUDA(cudaGetLastError());
     if (split > 0) {
-        reduce_pieces<<<dim3(split, n_blocks(bn_max, kRedCols)), kBM, 0, ctx->stream>>>(L);
+        launch_pdl(reduce_pieces, dim3(split, n_blocks(bn_max, kRedCols)), kBM, 0, ctx->stream, L);
         ctx->launches++;
     }
     PLX_CHECK_CUDA(cudaGetLastError());
