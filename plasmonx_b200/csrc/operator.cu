@@ -279,6 +279,20 @@ __device__ __forceinline__ void charge_term(int nt, int ti, int tj, int f, doubl
     }
 }
 
+// y (times sign) + D_q(w) x of one row and column
+__device__ __forceinline__ void charge_store(int nv, int c, int i, const Cplx &d, const double *__restrict__ X,
+                                             double *__restrict__ Y, double sign, int add_diag, double yre, double yim) {
+    yre *= sign;
+    yim *= sign;
+    if (add_diag) {
+        const double xr = X[(int64_t)c * 2 * nv + i], xi = X[(int64_t)c * 2 * nv + nv + i];
+        yre += d.re * xr - d.im * xi;
+        yim += d.re * xi + d.im * xr;
+    }
+    Y[(int64_t)c * 2 * nv + i] = yre;
+    Y[(int64_t)c * 2 * nv + nv + i] = yim;
+}
+
 template <bool HETERO>
 __global__ void __launch_bounds__(256) charge_rows(int N, int nt, int nv, int count,
                                                    const int32_t *__restrict__ freq,
@@ -340,19 +354,105 @@ __global__ void __launch_bounds__(256) charge_rows(int N, int nt, int nv, int co
             yre += __shfl_xor_sync(0xffffffffu, yre, o);
             yim += __shfl_xor_sync(0xffffffffu, yim, o);
         }
-        if (lane == 0) {
-            yre *= sign;
-            yim *= sign;
-            if (add_diag) {
-                const Cplx d = dq[ti + nt * f];
-                const double xr = X[(int64_t)c * 2 * nv + i], xi = X[(int64_t)c * 2 * nv + nv + i];
-                yre += d.re * xr - d.im * xi;
-                yim += d.re * xi + d.im * xr;
-            }
-            Y[(int64_t)c * 2 * nv + i] = yre;
-            Y[(int64_t)c * 2 * nv + nv + i] = yim;
+        if (lane == 0) charge_store(nv, c, i, dq[ti + nt * f], X, Y, sign, add_diag, yre, yim);
+    }
+}
+
+// The same rows of one atom type for many columns, with columns across the lanes.
+// The row form gathers S at the row's atoms, a cache line per entry and column: at 893
+// sodium atoms (289 entries a row) x 61 columns it was bound by L1, 78 us.  Here S is
+// transposed first (St[atom][column], 16 bytes a column), so that an entry is one
+// coalesced read of 32 columns: 28 us with the transpose, bound by instruction issue
+// (a shuffle for the entry's place and two for its coefficient).  Four warps share a row
+// and 32 columns: warp m sums the entries of the row form's lanes m, m + 4, ..., eight
+// chains a thread, each in CSR order, and the chains are added in the butterfly's order
+// -- every result has the row form's bits.
+//
+// From 12 columns: the transposed form takes the same time for 1 to 32, the row form
+// grows with them (893 atoms, 8 / 12 / 32 columns: 18.5 / 25 / 70 us against 14 / 15 /
+// 16; 1,961 silver atoms: 25 / 36 / 90 against 30 / 31 / 32; 4,693 sodium atoms:
+// 49 / 72 / 183 against 67 / 69 / 72).
+constexpr int kColsMin = 12;
+__global__ void __launch_bounds__(128, 7) charge_cols(
+    int N, int nt, int nv, int count, const int32_t *__restrict__ freq, const int32_t *__restrict__ type,
+    const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col, const double *__restrict__ kval,
+    const Cplx *__restrict__ dq, const double2 *__restrict__ St, const double *__restrict__ X, double *__restrict__ Y,
+    double sign, int add_diag) {
+    pdl_sync();
+    __shared__ double2 part[4][32];
+    const int i = blockIdx.x, lane = threadIdx.x & 31, m = threadIdx.x >> 5;
+    const int c = blockIdx.y * 32 + lane;
+    const double2 *col_s = St + min(c, count - 1);
+    const double2 s = col_s[(int64_t)i * count];
+    const int e1 = rowptr[i + 1];
+    double yre[8], yim[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) yre[q] = yim[q] = 0.0;
+    // lane l (l mod 8) holds the warp's entry 4 l + m of the 32 in turn
+    int e = rowptr[i] + m + 4 * (lane & 7);
+    int at = 0;
+    double k = 0.0;
+    auto fetch = [&] {
+        at = (e < e1 ? col[e] : 0) * count;
+        k = e < e1 ? kval[e] : 0.0;
+    };
+    fetch();
+    int left = e1 - rowptr[i];
+    for (; left >= 32; left -= 32) {
+        double2 v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = col_s[__shfl_sync(0xffffffffu, at, q)];
+        const double kk = k;
+        e += 32;
+        fetch();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double kq = __shfl_sync(0xffffffffu, kk, q);
+            yre[q] = fma(kq, v[q].x - s.x, yre[q]);
+            yim[q] = fma(kq, v[q].y - s.y, yim[q]);
         }
     }
+    {
+        double2 v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = col_s[__shfl_sync(0xffffffffu, at, q)];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double kq = __shfl_sync(0xffffffffu, k, q);
+            if (4 * q + m < left) {
+                yre[q] = fma(kq, v[q].x - s.x, yre[q]);
+                yim[q] = fma(kq, v[q].y - s.y, yim[q]);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < o; ++q) {
+            yre[q] += yre[q + o];
+            yim[q] += yim[q + o];
+        }
+    part[m][lane] = make_double2(yre[0], yim[0]);
+    __syncthreads();
+    if (m != 0 || c >= count) return;
+    const double2 p0 = part[0][lane], p1 = part[1][lane], p2 = part[2][lane], p3 = part[3][lane];
+    charge_store(nv, c, i, dq[type[i] + nt * freq[c]], X, Y, sign, add_diag, (p0.x + p2.x) + (p1.x + p3.x),
+                 (p0.y + p2.y) + (p1.y + p3.y));
+}
+
+// St[i][r] = S[r][i] for the charges i < N of R rows of length nv.
+__global__ void __launch_bounds__(256) transpose_charges(int N, int nv, int R, const double *__restrict__ S,
+                                                         double *__restrict__ St) {
+    pdl_sync();
+    __shared__ double tile[32][33];
+    const int i0 = blockIdx.x * 32, r0 = blockIdx.y * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = y; q < 32; q += 8)
+        if (r0 + q < R && i0 + x < N) tile[q][x] = S[(int64_t)(r0 + q) * nv + i0 + x];
+    __syncthreads();
+#pragma unroll
+    for (int q = y; q < 32; q += 8)
+        if (i0 + q < N && r0 + x < R) St[(int64_t)(i0 + q) * R + r0 + x] = tile[x][q];
 }
 
 // Dipole rows: y = s + (sum_t f_t,i / alpha_t(w)) x.
@@ -666,16 +766,40 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
     stored_product(ctx, g->d_part, R, n, X, g->d_T.p, S);
 }
 
+// Whether charge_cols takes a batch (its places are 32-bit).
+static bool charges_by_column(const plx_geom *g, int count) {
+    return g->n_types == 1 && count >= kColsMin && (int64_t)g->n_atoms * count <= INT32_MAX;
+}
+
+// The charge rows of a batch; St: room for the transposed S (2 count N doubles), or null.
+static void charge_part(plx_geom *g, const OpBatch &b, const double *S, const double *X, double *Y, double sign,
+                        int add_diag, double *St) {
+    plx_ctx *ctx = g->ctx;
+    cudaStream_t st = ctx->stream;
+    const int N = g->n_atoms, nv = g->n_var;
+    if (charges_by_column(g, b.count) && St) {
+        const int R = 2 * b.count;
+        launch_pdl(transpose_charges, dim3(n_blocks(N, 32), n_blocks(R, 32)), 256, 0, st, N, nv, R, S, St);
+        launch_pdl(charge_cols, dim3(N, n_blocks(b.count, 32)), 128, 0, st, N, g->n_types, nv, b.count,
+                   b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_dq.p,
+                   reinterpret_cast<const double2 *>(St), X, Y, sign, add_diag);
+        ctx->launches += 2;
+        return;
+    }
+    const dim3 gq(n_blocks((int64_t)N * 32, 256), n_blocks(b.count, kChargeCols));
+    launch_pdl(g->n_types > 1 ? charge_rows<true> : charge_rows<false>, gq, 256, 0, st, N, g->n_types, nv, b.count,
+               b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_wratio.p, g->d_dq.p, S,
+               X, Y, sign, add_diag);
+    ctx->launches++;
+}
+
 static void finish_rows(plx_geom *g, const OpBatch &b, const double *S, const double *X,
                         double *Y) {
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     const int N = g->n_atoms, nv = g->n_var;
-    dim3 gq(n_blocks((int64_t)N * 32, 256), n_blocks(b.count, kChargeCols));
-    launch_pdl(g->n_types > 1 ? charge_rows<true> : charge_rows<false>, gq, 256, 0, st, N, g->n_types, nv, b.count,
-               b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_wratio.p, g->d_dq.p, S,
-               X, Y, 1.0, 1);
-    ctx->launches++;
+    // the product's partial sums have been added: their scratch holds the transpose
+    charge_part(g, b, S, X, Y, 1.0, 1, g->d_part.n >= (size_t)b.count * 2 * N ? g->d_part.p : nullptr);
     if (g->model == PLX_WFQFMU) {
         dim3 gm(n_blocks(3LL * N, 256), b.count);
         launch_pdl(dipole_rows, gm, 256, 0, st, N, g->n_types, nv, b.count, b.d_freq, g->d_frac.p, g->d_inv_alpha.p, S,
@@ -809,12 +933,16 @@ void rhs_batch(plx_geom *g, const OpBatch &b, const int32_t *d_pol, double *Bout
     V.alloc(ctx, (size_t)b.count * 2 * nv);
     potential_kernel<<<dim3(n_blocks(nv, 256), b.count), 256, 0, st>>>(
         N, nv, b.count, d_pol, g->d_pos.p, g->e0, g->rhs_potential, mn[0], mn[1], mn[2], V.p);
-    dim3 gq(n_blocks((int64_t)N * 32, 256), n_blocks(b.count, kChargeCols));
+    ctx->launches++;
     // b_q = -Kop(w) V  (rhs_module.f90:140-390); no diagonal term
-    launch_pdl(g->n_types > 1 ? charge_rows<true> : charge_rows<false>, gq, 256, 0, st, N, g->n_types, nv, b.count,
-               b.d_freq, g->d_type.p, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_ktval.p, g->d_wratio.p, g->d_dq.p,
-               V.p, V.p, Bout, -1.0, 0);
-    ctx->launches += 2;
+    DevArray<double> Vt;
+    if (charges_by_column(g, b.count)) {
+        try {
+            Vt.alloc(ctx, (size_t)b.count * 2 * N);
+        } catch (const Error &) {                     // no room: the row form needs none
+        }
+    }
+    charge_part(g, b, V.p, V.p, Bout, -1.0, 0, Vt.p);
     if (g->model == PLX_WFQFMU) {
         dim3 gm(n_blocks(3LL * N, 256), b.count);
         rhs_dipole<<<gm, 256, 0, st>>>(N, nv, b.count, d_pol, g->e0, Bout);
