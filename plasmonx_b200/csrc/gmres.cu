@@ -306,8 +306,9 @@ __device__ __forceinline__ double2 conj_prod(double vr, double vi, double wr, do
 // The FP64 basis (the plain form): every row is one chain over ii in ascending order.
 // A block owns 32 rows: all 256 threads load 32 vectors of them and leave their
 // products in shared memory, the next 32 vectors in flight, and two warps (re, im; a
-// lane a row) add them in order; a thread per row and all its loads left 44 CTAs at 2,800 unknowns and 4 columns (36 us a launch, now 12.6 us; 893
-// unknowns, 61 columns 27 -> 19 us).
+// lane a row) add them in order.  A thread per row and all its loads left 44 CTAs at
+// 2,800 unknowns and 4 columns (36 us a launch, now 12.6 us; 893 unknowns, 61 columns
+// 27 -> 19 us).
 constexpr int kChainRows = 32, kChainVec = 32;
 constexpr size_t kChainSmem = 2 * kChainVec * 2 * kChainRows * sizeof(double);       // combine_chain's static part
 template <bool FIN>
@@ -607,19 +608,50 @@ struct Rotation {
     double2 s, h;
     double c;
 };
+// A column's part of H, the rotations and g, and the first tile of the chain.
+struct GivensTile {
+    double2 *h, *sn, *g;
+    double *cs;
+    double2 a, g0, g1, si, hn;
+    double ci;
+    __device__ GivensTile(int c, int lane, int j, double2 *Hcol, int hstride, double *cs_, double2 *sn_, double2 *g_,
+                          int gstride, int cstride)
+        : h(Hcol + (int64_t)c * hstride), sn(sn_ + (int64_t)c * cstride), g(g_ + (int64_t)c * gstride),
+          cs(cs_ + (int64_t)c * cstride) {
+        a = h[0];                            // chain value entering the tile (same in every lane)
+        g0 = g[j];
+        g1 = g[j + 1];
+        ci = lane < j ? cs[lane] : 1.0;
+        si = lane < j ? sn[lane] : make_double2(0.0, 0.0);
+        hn = lane < j ? h[lane + 1] : make_double2(0.0, 0.0);
+    }
+};
+
+// The rotation (c, s) that takes (ca, b), b >= 0, to (r, 0): c = |ca| / r, s = ca / |ca| b / r.
+// Scaled by a power of two, with two reciprocal square roots; false where a square would leave
+// the range (the general form follows).
+__device__ __forceinline__ bool rotation(double2 ca, double b, double &cj, double2 &sj) {
+    const double m = fmax(fmax(fabs(ca.x), fabs(ca.y)), b);
+    if (!(m > 1e-290 && m < 1e290)) return false;
+    const double f = __hiloint2double((2046 - ((__double2hiint(m) >> 20) & 0x7ff)) << 20, 0);   // 2^-exponent, or half
+    const double x = ca.x * f, y = ca.y * f, z = b * f, a2 = fma(x, x, y * y);
+    if (!(a2 > 1e-260)) return false;
+    const double ia = rsqrt(a2), ir = rsqrt(fma(z, z, a2)), t = z * ir * ia;
+    cj = a2 * ia * ir;
+    sj = make_double2(x * t, y * t);
+    return true;
+}
+
 template <bool SCAN>
-__device__ void givens(int k, int c, int lane, int j, double norm, double2 *__restrict__ Hcol, int hstride,
-                       double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g, int gstride,
-                       int cstride, double *__restrict__ resid, Rotation *rot) {
-    double2 *h = Hcol + (int64_t)c * hstride;
-    double *csc = cs + (int64_t)c * cstride;
-    double2 *snc = sn + (int64_t)c * cstride;
-    double2 *gc = g + (int64_t)c * gstride;
-    double2 a = h[0];                        // chain value entering the tile (same in every lane)
-    double2 cb = make_double2(norm, 0.0), g0 = gc[j], g1 = gc[j + 1];
-    double ci = lane < j ? csc[lane] : 1.0;
-    double2 si = lane < j ? snc[lane] : make_double2(0.0, 0.0);
-    double2 hn = lane < j ? h[lane + 1] : make_double2(0.0, 0.0);
+__device__ void givens(int k, int lane, int j, double norm, const GivensTile &tile, double *__restrict__ resid,
+                       Rotation *rot) {
+    double2 *__restrict__ h = tile.h;
+    double *__restrict__ csc = tile.cs;
+    double2 *__restrict__ snc = tile.sn;
+    double2 *__restrict__ gc = tile.g;
+    double2 a = tile.a, g0 = tile.g0, g1 = tile.g1, si = tile.si, hn = tile.hn;
+    double2 cb = make_double2(norm, 0.0);
+    double ci = tile.ci;
     for (int i0 = 0; i0 < j; i0 += 32) {
         const int i = i0 + lane, in = i + 32;
         // the next tile's loads, in flight during this tile's chain
@@ -670,7 +702,8 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *__re
     double2 ca = a;
     double cj;
     double2 sj;
-    if (cabs_(ca) == 0.0) {
+    if (SCAN && rotation(ca, norm, cj, sj)) {
+    } else if (cabs_(ca) == 0.0) {
         cj = 0.0;
         sj = make_double2(1.0, 0.0);
     } else {
@@ -697,7 +730,7 @@ __device__ void givens(int k, int c, int lane, int j, double norm, double2 *__re
 
 // The end of an Arnoldi step: h_{j+1,j} = ||W[k]||, v_{j+1}[c] = W[k] / h_{j+1,j} (zero
 // when the norm is zero, as the reference leaves the zero-filled column untouched),
-// the Givens update of H's column j (one warp of a column's first block), and the
+// the Givens update of H's column j (one warp of a column's last block), and the
 // input X[k] = P v_{j+1} of the next product, split for the tensor cores.  One launch
 // in place of norm, scaling, Givens, gather, preconditioner and split.
 //
@@ -729,7 +762,17 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
         slabs[j + 1] = slab_next;
         Hcols[j] = Hcol;
     }
+    // the last block of a column does its Givens update; its loads are in flight during
+    // the norm, and so are the other blocks' first rows of W
+    const bool last = blockIdx.x == gridDim.x - 1;
     const double *w = W + (int64_t)k * 2 * n;
+    const int lane = threadIdx.x & 31, r0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const GivensTile tile(c, lane, last ? j : 0, Hcol, hstride, cs, sn, g, gstride, cstride);
+    double wr = 0.0, wi = 0.0;
+    if (!last && r0 < n) {
+        wr = w[r0];
+        wi = w[n + r0];
+    }
     double s = 0.0;
     if (kInner) {
         double dummy = 0.0;
@@ -746,12 +789,16 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
     if (threadIdx.x == 0) total = sqrt(s);
     __syncthreads();
     s = total;
+    if (last) {
+        if (threadIdx.x < 32) givens<kInner>(k, lane, j, s, tile, resid, rot);
+        return;
+    }
     const double inv = s != 0.0 ? 1.0 / s : 0.0;
     VT *v = slab_next + (int64_t)c * 2 * n;
     const double *p = P ? P + (int64_t)c * 2 * n : nullptr;
     double *x = X + (int64_t)k * 2 * n;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const VT vr = (VT)(s != 0.0 ? w[r] * inv : 0.0), vi = (VT)(s != 0.0 ? w[n + r] * inv : 0.0);
+    for (int r = r0; r < n;) {
+        const VT vr = (VT)(s != 0.0 ? wr * inv : 0.0), vi = (VT)(s != 0.0 ? wi * inv : 0.0);
         v[r] = vr;
         v[n + r] = vi;
         double re = (double)vr, im = (double)vi;
@@ -763,9 +810,12 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
         x[r] = re;
         x[n + r] = im;
         if (sp.hi) split_column(sp, k, r, re, im);
+        r += (gridDim.x - 1) * blockDim.x;
+        if (r < n) {
+            wr = w[r];
+            wi = w[n + r];
+        }
     }
-    if (blockIdx.x == 0 && threadIdx.x < 32)
-        givens<kInner>(k, c, threadIdx.x, j, s, Hcol, hstride, cs, sn, g, gstride, cstride, resid, rot);
 }
 
 // y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
@@ -1101,9 +1151,9 @@ class GmresRun final : public GmresStepper {
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
         for (int k = 0; k < na; ++k) memcpy(host_.p + k, &kPending, 8);
         prof_begin(ctx_);
-        launch_pdl(
-            normalize_givens<VT>, dim3(grid_rows(n), na), 256, 0, st_, n, j, d_act_.p, nparts, nrm_part_.p, Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p,
-            d_hcols_.p, hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, host_.p);
+        launch_pdl(normalize_givens<VT>, dim3(grid_rows(n) + 1, na), 256, 0, st_, n, j, d_act_.p, nparts, nrm_part_.p,
+                   Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p, d_hcols_.p,
+                   hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, host_.p);
         ctx_->launches++;
         x_ready_ = true;
         prof_end(ctx_, PROF_LSQ, 0.0, 0.0);
