@@ -947,6 +947,25 @@ __global__ void scale_cols(int n, const int32_t *__restrict__ idx, const double 
 
 int grid_rows(int64_t n2) { return (int)std::min<int64_t>(n_blocks(n2, 256), 1024); }
 
+// blockIdx.z of dots_wide() for `blocks` (row chunk, column) pairs and ni vectors: the
+// fewest rounds of `slots` resident blocks (four an SM, two with an FP64 basis) times
+// the vectors of a warp, half a vector for what a block does before them.  A split to a
+// fixed number of blocks ran 784 of them as 1.3 rounds (13,528 unknowns, 14 columns, 120
+// vectors: 40 us, now 35).
+int dots_split(int blocks, int ni, int slots) {
+    int best = 1;
+    int64_t least = INT64_MAX;
+    for (int nz = 1; nz <= std::min(64, n_blocks(ni, kThreads / 32)); ++nz) {
+        const int64_t rounds = n_blocks((int64_t)blocks * nz, slots);
+        const int64_t cost = rounds * (2 * n_blocks(ni, kThreads / 32 * nz) + 1);
+        if (cost < least) {
+            least = cost;
+            best = nz;
+        }
+    }
+    return best;
+}
+
 // Groups of threads of combine_inner() (see there).
 int combine_groups(int n, int ni) { return n <= 16384 && ni >= 16 ? 4 : 1; }
 int combine_blocks(int n, int ni) { return n_blocks(n, kThreads / combine_groups(n, ni)); }
@@ -1113,7 +1132,7 @@ class GmresRun final : public GmresStepper {
         auto project = [&](int i0, int i1, int accumulate, bool last) {
             const int ni = i1 - i0;
             if (ni >= 8) {
-                const int nz = std::max(1, std::min(n_blocks(ni, kThreads / 32), n_blocks(592, ndot_ * na)));
+                const int nz = dots_split(ndot_ * na, ni, (sizeof(VT) == 4 ? 4 : 2) * sms_);
                 launch_pdl(dots_wide<VT>, dim3(ndot_, na, nz), kThreads, 0, st_, n, i0, i1, d_act_.p, d_slabs_.p,
                            Wa_.p, part_.p);
             } else {
