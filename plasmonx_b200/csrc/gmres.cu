@@ -820,13 +820,14 @@ __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const
 
 // y = R^{-1} g for the triangular R = H(0..j, 0..j) (ztrsv 'U','N','N'), one block
 // per triggered column, y stored compactly [k][j+1].  Back substitution in
-// blocks of 32 columns: the 32 x 32 triangle is staged in shared memory and
+// blocks of 32 columns: the 32 x 32 triangle lies in shared memory and is
 // solved by one warp in registers, then the whole block subtracts the 32
 // solved unknowns from the rows above (each row in descending column order and
-// with the roundings of the unblocked substitution) while it stages the next triangle.  One
-// warp reading the columns of R from global memory, one dependent load per
-// unknown, took 326 us at 61-130 unknowns and 1,125 us at 700; now 100 and
-// 333 us (latency bound: ~32 dependent multiplications a block).
+// with the roundings of the unblocked substitution).  Those rows' entries (up to 256
+// rows) and the next triangle are loaded into registers before the substitution
+// starts, which left ~32 dependent multiplications a block: 31 us at 61-130 unknowns,
+// 118 at 700, 7.9 at 20-60 (102, 333 and 18 us with the loads after it; 326 and 1,125
+// by one warp with a dependent load per unknown).
 constexpr int kTriB = 32;
 
 // n / d rounded once from id = 1 / d rounded once (Markstein's theorem: the remainder
@@ -836,38 +837,54 @@ __device__ __forceinline__ double quotient(double n, double d, double id) {
     return fma(fma(-q, d, n), id, q);
 }
 
-__global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t *__restrict__ act,
-                                                 double2 *const *__restrict__ Hcols, int hstride,
-                                                 const double2 *__restrict__ g, int gstride,
-                                                 double2 *__restrict__ y) {
+constexpr int kTriThreads = 256;
+__global__ void __launch_bounds__(kTriThreads) tri_solve(int count, int j, const int32_t *__restrict__ act,
+                                                         double2 *const *__restrict__ Hcols, int hstride,
+                                                         const double2 *__restrict__ g, int gstride,
+                                                         double2 *__restrict__ y) {
     pdl_sync();
     extern __shared__ double2 ys[];
     __shared__ double2 tri[kTriB][kTriB + 1];        // tri[column][row]
+    constexpr int kWarps = kTriThreads / 32, kCols = kTriB / kWarps;      // columns of a triangle a warp loads
     const int k = blockIdx.x;
     if (k >= count) return;
     const int c = act[k];
     const int m = j + 1;
     const int64_t off = (int64_t)c * hstride;
-    auto stage = [&](int b0) {                       // triangle of columns and rows b0 .. b0 + 31
-        for (int e = threadIdx.x; e < kTriB * kTriB; e += blockDim.x) {
-            const int col = e / kTriB, row = e % kTriB;
-            tri[col][row] = (b0 + col < m && row <= col) ? Hcols[b0 + col][off + b0 + row] : make_double2(0.0, 0.0);
+    const int warp = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 next[kCols];                             // the next triangle, columns and rows b0 .. b0 + 31
+    auto fetch = [&](int b0) {
+#pragma unroll
+        for (int q = 0; q < kCols; ++q) {
+            const int col = warp + kWarps * q;
+            next[q] = b0 + col < m && l <= col ? Hcols[b0 + col][off + b0 + l] : zero;
         }
     };
-    for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = g[(int64_t)c * gstride + i];
+    auto store = [&] {
+#pragma unroll
+        for (int q = 0; q < kCols; ++q) tri[warp + kWarps * q][l] = next[q];
+    };
     int b0 = (m - 1) / kTriB * kTriB;
-    stage(b0);
+    fetch(b0);
+    for (int i = threadIdx.x; i < m; i += kTriThreads) ys[i] = g[(int64_t)c * gstride + i];
+    store();
     __syncthreads();
     for (; b0 >= 0; b0 -= kTriB) {
         const int nb = min(kTriB, m - b0);
-        if (threadIdx.x < 32) {
-            const int l = threadIdx.x;
-            double2 v = l < nb ? ys[b0 + l] : make_double2(0.0, 0.0);
-            const double2 r = l < nb ? tri[l][l] : make_double2(1.0, 0.0);
-            const double d = fma(r.x, r.x, __dmul_rn(r.y, r.y)), id = 1.0 / d;
+        // rows above and the next triangle, in flight during the substitution
+        double2 r[kTriB];
+#pragma unroll
+        for (int q = 0; q < kTriB; ++q)
+            r[q] = threadIdx.x < b0 && q < nb ? Hcols[b0 + q][off + threadIdx.x] : zero;
+        if (b0 > 0) fetch(b0 - kTriB);
+        if (warp == 0) {
+            double2 v = l < nb ? ys[b0 + l] : zero;
+            const double2 rd = l < nb ? tri[l][l] : make_double2(1.0, 0.0);
+            const double d = fma(rd.x, rd.x, __dmul_rn(rd.y, rd.y)), id = 1.0 / d;
             for (int i = nb - 1; i >= 0; --i) {
-                const double2 yi = shfl2(make_double2(quotient(fma(v.x, r.x, __dmul_rn(v.y, r.y)), d, id),
-                                                      quotient(fma(v.y, r.x, -__dmul_rn(v.x, r.y)), d, id)),
+                const double2 yi = shfl2(make_double2(quotient(fma(v.x, rd.x, __dmul_rn(v.y, rd.y)), d, id),
+                                                      quotient(fma(v.y, rd.x, -__dmul_rn(v.x, rd.y)), d, id)),
                                          i);
                 if (l == i) v = yi;
                 if (l < i) {
@@ -880,32 +897,39 @@ __global__ void __launch_bounds__(256) tri_solve(int count, int j, const int32_t
         }
         __syncthreads();
         if (b0 > 0) {
-            for (int l = threadIdx.x; l < b0; l += blockDim.x) {
-                double2 v = ys[l];
-                for (int i0 = nb; i0 > 0; i0 -= 8) {
-                    double2 r[8];
+            if (threadIdx.x < b0) {
+                double2 v = ys[threadIdx.x];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        r[q] = i0 - 1 - q >= 0 ? Hcols[b0 + i0 - 1 - q][off + l] : make_double2(0.0, 0.0);
+                for (int q = kTriB - 1; q >= 0; --q)
+                    if (q < nb) {
+                        const double2 p = prod(r[q].x, r[q].y, ys[b0 + q], false);
+                        v.x -= p.x;
+                        v.y -= p.y;
+                    }
+                ys[threadIdx.x] = v;
+            }
+            for (int row = threadIdx.x + kTriThreads; row < b0; row += kTriThreads) {
+                double2 v = ys[row];
+                for (int i0 = nb; i0 > 0; i0 -= 8) {
+                    double2 p[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) p[q] = i0 - 1 - q >= 0 ? Hcols[b0 + i0 - 1 - q][off + row] : zero;
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         if (i0 - 1 - q >= 0) {
-                            const double2 p = prod(r[q].x, r[q].y, ys[b0 + i0 - 1 - q], false);
-                            v.x -= p.x;
-                            v.y -= p.y;
+                            const double2 t = prod(p[q].x, p[q].y, ys[b0 + i0 - 1 - q], false);
+                            v.x -= t.x;
+                            v.y -= t.y;
                         }
                 }
-                ys[l] = v;
+                ys[row] = v;
             }
-            stage(b0 - kTriB);
+            store();
             __syncthreads();
         }
     }
-    for (int i = threadIdx.x; i < m; i += blockDim.x) y[(int64_t)k * m + i] = ys[i];
+    for (int i = threadIdx.x; i < m; i += kTriThreads) y[(int64_t)k * m + i] = ys[i];
 }
-
-// a thread per row above the last triangle, at most a block's worth
-int tri_threads(int m) { return std::min(256, std::max(64, (m + 31) / 32 * 32)); }
 
 // R[k] = B[c] - AX[k] with c = act[k]; in place into AX.
 __global__ void residual(int n, const int32_t *__restrict__ act, const double *__restrict__ B,
@@ -1202,7 +1226,7 @@ class GmresRun final : public GmresStepper {
             // inner solve of a refinement: take the least-squares solution as is
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            launch_pdl(tri_solve, nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
+            launch_pdl(tri_solve, nt, kTriThreads, (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
                        hstride_, gv_.p, hstride_, ybuf_.p);
             ctx_->launches += 1 + combine_chunked(st_, sms_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
             if (jac_) {
@@ -1218,7 +1242,7 @@ class GmresRun final : public GmresStepper {
             x_ready_ = false;                 // the true residual's product uses the input buffer
             const int nt = (int)trig.size();
             PLX_CHECK_CUDA(cudaMemcpyAsync(d_cols_.p, trig.data(), nt * 4, cudaMemcpyHostToDevice, st_));
-            launch_pdl(tri_solve, nt, tri_threads(j + 1), (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
+            launch_pdl(tri_solve, nt, kTriThreads, (j + 1) * sizeof(double2), st_, nt, j, d_cols_.p, d_hcols_.p,
                        hstride_, gv_.p, hstride_, ybuf_.p);
             ctx_->launches += combine_chunked(st_, sms_, n, 0, j + 1, nt, d_cols_.p, d_slabs_.p, ybuf_.p, 1.0, d_X_, 1);
             launch_pdl(gather_x, dim3(grid_rows(2LL * n), nt), 256, 0, st_, n, d_cols_.p, d_X_, Xa_.p);
