@@ -1305,7 +1305,7 @@ class GmresRun final : public GmresStepper {
     }
 
     // The residuals reach the host before the runtime reports the end of the kernel that
-    // wrote them: reading the words for up to about half a millisecond and then waiting
+    // wrote them: reading the words for up to about ten milliseconds and then waiting
     // for the stream brings the next product 4 us forward (12.2 -> 8 us after the step).
     // A residual with the pending word's bits costs that wait, nothing else.
     void await_residuals(int na) {
@@ -1330,7 +1330,7 @@ class GmresRun final : public GmresStepper {
     }
 
     static constexpr uint64_t kPending = 0xfff8a5c35a3c0001ull;      // a NaN that no kernel forms
-    static constexpr int kPolls = 1 << 14;
+    static constexpr int kPolls = 1 << 18;
 
     plx_geom *g_;
     plx_ctx *ctx_;
