@@ -166,9 +166,11 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
 // each remaining tile into sms / remaining equal pieces left 38 SMs of 148 idle at 55
 // tiles (13,528 unknowns: 156 us a launch, now 121 us) and 24 at 31 tiles (7,844
 // unknowns: 51.7 -> 47 us); grouped launches ran whole tiles only, 30 CTAs for six
-// geometries of 143 to 2,700 unknowns (25.9 -> 11 us).
+// geometries of 143 to 2,700 unknowns (25.9 -> 9.2 us).
 constexpr int kMaxGroups = 6;
-constexpr int kMinRun = 8;          // k-tiles: below, a piece's prologue and partial sums cost more than it saves
+// k-tiles a CTA at least.  Six small geometries: 11.2 us a launch with 8, 9.2 with 4, 8.4
+// with 2, which costs the pieces another microsecond.
+constexpr int kMinRun = 4;
 constexpr int kThreadsTc = 192;
 
 // The rest of an operator row after the contraction, applied where its sums are
