@@ -277,14 +277,22 @@ void fold_batch(plx_geom *g, int nc, const int32_t *d_rows, const int32_t *d_ord
     DevArray<double> d_C, d_csum;
     d_off.alloc(ctx, nc + 1);
     PLX_CHECK_CUDA(cudaMemcpyAsync(d_off.p, off.data(), (size_t)(nc + 1) * 4, cudaMemcpyHostToDevice, st));
-    const int most = (int)(kFoldBytes / (kCluster * sizeof(double)));
+    int most = (int)(kFoldBytes / (kCluster * sizeof(double)));
     for (int c0 = 0; c0 < nc;) {
         int c1 = c0 + 1;
         while (c1 < nc && off[c1 + 1] - off[c0] <= most) ++c1;
         const size_t len = std::max(1, off[c1] - off[c0]);
-        if (d_list.n < len) {
-            d_list.alloc(ctx, len);
-            d_C.alloc(ctx, len * kCluster);
+        if (d_list.n < len || d_C.n < len * kCluster) {
+            try {
+                d_list.alloc(ctx, len);
+                d_C.alloc(ctx, len * kCluster);
+            } catch (const Error &) {                 // little room: smaller batches, down to a cluster
+                d_list.release();
+                d_C.release();
+                if (c1 == c0 + 1) throw;
+                most /= 4;
+                continue;
+            }
         }
         if (d_csum.n < (size_t)(c1 - c0) * kCluster) d_csum.alloc(ctx, (size_t)(c1 - c0) * kCluster);
         PLX_CHECK_CUDA(cudaMemsetAsync(d_C.p, 0, len * kCluster * 8, st));

@@ -36,6 +36,7 @@ namespace {
 // ---------------------------------------------------------------------------
 constexpr int kOtfWarps = 8;
 constexpr int kOtfFewCols = 4;              // columns up to which it is used; the tiled form above
+constexpr int kOtfNoScratch = 16;           // columns up to which a product goes on without the tiled form's scratch
 
 // Warps per target atom: enough of them for ~24 warps on every SM.
 int otf_warps(int N) {
@@ -697,6 +698,33 @@ void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const
     PLX_CHECK_CUDA(cudaGetLastError());
 }
 
+// Matrix-free product four columns at a time; needs no scratch.
+static void otf_few_columns(plx_geom *g, int count, const double *X, double *S) {
+    plx_ctx *ctx = g->ctx;
+    const bool fmu = g->model == PLX_WFQFMU;
+    const int n = g->n_var, N = g->n_atoms;
+    const int wt = otf_warps(N), blocks = n_blocks(N, kOtfWarps / wt);
+    for (int c0 = 0; c0 < count; c0 += kOtfFewCols) {
+        const int cb = std::min(kOtfFewCols, count - c0);
+        const int64_t at = (int64_t)c0 * 2 * n;
+#define PLX_OTF(CB, F)                                                                                            \
+    launch_pdl(otf_contract<CB, F>, blocks, 32 * kOtfWarps, 0, ctx->stream, N, wt, cb, n, g->n_types, g->d_pos.p,    \
+               g->d_par.p, g->d_type.p, g->d_widths.p, X + at, S + at)
+        if (fmu) {
+            if (cb == 1) PLX_OTF(1, true);
+            else if (cb == 2) PLX_OTF(2, true);
+            else PLX_OTF(4, true);
+        } else {
+            if (cb == 1) PLX_OTF(1, false);
+            else if (cb == 2) PLX_OTF(2, false);
+            else PLX_OTF(4, false);
+        }
+#undef PLX_OTF
+        ctx->launches++;
+    }
+    PLX_CHECK_CUDA(cudaGetLastError());
+}
+
 void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on_the_fly) {
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
@@ -714,7 +742,15 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
             const int jchunk = n_blocks(n_blocks(N, js), ka) * ka;
             js = n_blocks(N, jchunk);
             const size_t need = (size_t)js * R * n;
-            if (g->d_part.n < need) g->d_part.alloc(ctx, need);
+            if (g->d_part.n < need) {
+                try {
+                    g->d_part.alloc(ctx, need);
+                } catch (const Error &) {
+                    if (count > kOtfNoScratch) throw;
+                    otf_few_columns(g, count, X, S);     // no room for the partial sums
+                    return;
+                }
+            }
             const int bm = R <= 16 ? 16 : R <= 32 ? 32 : (R <= 48 ? 48 : 64);
             const dim3 grid(tiles, n_blocks(R, bm), js);
 #define PLX_OTF(BMV, F)                                                                                            \
@@ -744,22 +780,7 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
             PLX_CHECK_CUDA(cudaGetLastError());
             return;
         }
-        const int wt = otf_warps(N), blocks = n_blocks(N, kOtfWarps / wt);
-#define PLX_OTF(CB, F)                                                                                            \
-    launch_pdl(otf_contract<CB, F>, blocks, 32 * kOtfWarps, 0, st, N, wt, count, n, g->n_types, g->d_pos.p, g->d_par.p, \
-                                                           g->d_type.p, g->d_widths.p, X, S)
-        if (fmu) {
-            if (count == 1) PLX_OTF(1, true);
-            else if (count == 2) PLX_OTF(2, true);
-            else PLX_OTF(4, true);
-        } else {
-            if (count == 1) PLX_OTF(1, false);
-            else if (count == 2) PLX_OTF(2, false);
-            else PLX_OTF(4, false);
-        }
-#undef PLX_OTF
-        ctx->launches++;
-        PLX_CHECK_CUDA(cudaGetLastError());
+        otf_few_columns(g, count, X, S);
         return;
     }
     if (!g->has_T) throw Error(PLX_ERR_ARG, "geometry was created without the dense T matrix");

@@ -64,8 +64,8 @@ struct DevArray {
     void alloc(plx_ctx *c, size_t count) {
         release();
         ctx = c;
-        n = count;
         p = count ? static_cast<T *>(dev_alloc(c, count * sizeof(T))) : nullptr;
+        n = count;                           // stays 0 when dev_alloc throws
     }
     void release() {
         if (p) dev_free(ctx, p, n * sizeof(T));

@@ -51,3 +51,21 @@ def test_inner_steps_match_the_fp64_operator(ctx, kind, n, shuffle, store_t):
         ref = sv.solve(precision='fp64_refined', **kw)
         got = sv.solve(precision='mixed_bf16x3', **kw)
     assert np.all(np.abs(got['steps'] - ref['steps']) <= 1), (got['steps'][:, 0], ref['steps'][:, 0])
+
+
+def test_little_room_folds_in_smaller_batches(ctx):
+    """1,961 atoms: the clusters' coefficients take about 13 MB together and 0.2 MB one by one.
+    The batch a cluster is folded in does not change its sums: the solution keeps its bits."""
+    p = configs.ag_sphere(radius=20.0, n_freq=1, method='iterative')
+    kw = dict(precision='mixed_bf16x3', pol_mask=1, want_x=True, max_outer=2, inner_krylov=16)
+    probe = Context(0)
+    with Solver(p, ctx=probe, store_t=True) as sv:
+        ref = sv.solve(**kw)
+        held = probe.bytes_in_use
+    probe.close()
+    tight = Context(0, hbm_budget=held + 5_000_000)
+    with Solver(p, ctx=tight, store_t=True) as sv:
+        got = sv.solve(**kw)
+    tight.close()
+    np.testing.assert_array_equal(got['status'], ref['status'])
+    np.testing.assert_array_equal(got['x'], ref['x'])
