@@ -1306,7 +1306,8 @@ class GmresRun final : public GmresStepper {
 
     // The residuals reach the host before the runtime reports the end of the kernel that
     // wrote them: reading the words for up to about ten milliseconds and then waiting
-    // for the stream brings the next product 4 us forward (12.2 -> 8 us after the step).
+    // for the stream brings the next product forward: 9.8 -> 5.4 us after the step of a
+    // matrix-free solve of 700 atoms, 12.2 -> 5.3 for six structures served together.
     // A residual with the pending word's bits costs that wait, nothing else.
     void await_residuals(int na) {
         const volatile uint64_t *w = reinterpret_cast<const volatile uint64_t *>(host_.p);

@@ -11,7 +11,7 @@
 //
 // Measured, the gaps gone and nothing else changed: serving six structures 195 -> 167
 // ms, a direct solve of 893 unknowns 16.3 -> 14.0, a mixed solve of 7,844 unknowns
-// 102 -> 94, two bow-ties of 13,528 unknowns 555 -> 519.
+// 102 -> 94, an alloy bow-tie of 13,528 unknowns 555 -> 519.
 //
 // Blocks that arrive early go to the SMs that have room first.  A kernel of two or
 // three blocks an SM can end up with most of them on a few SMs; even_smem() asks for so
