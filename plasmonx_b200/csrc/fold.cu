@@ -67,7 +67,8 @@ __global__ void union_count(int words, const int32_t *__restrict__ rows, const i
 }
 
 // The rows of T of the union's atoms (map: row of an atom, the atom itself when null;
-// padded to fours with the cluster's first atom, coefficient zero) and the coefficients C[union entry][32 rows], zeroed before; row sums of the coefficients.
+// padded to fours with the cluster's first atom, coefficient zero) and the coefficients
+// C[union entry][32 rows], zeroed before; row sums of the coefficients.
 __global__ void union_fill(int words, int c0, int hetero, const int32_t *__restrict__ rows,
                            const int32_t *__restrict__ order, const int32_t *__restrict__ rank,
                            const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
@@ -129,7 +130,8 @@ __global__ void union_fill(int words, int c0, int hetero, const int32_t *__restr
 constexpr int kFoldNT = 4;                           // 8-column tiles of a warp
 constexpr int kFoldCols = 4 * 8 * kFoldNT;           // columns of a block
 
-__global__ void __launch_bounds__(128, 4) fold_clusters(int n, int c0, const int32_t *__restrict__ map, const int32_t *__restrict__ rows,
+__global__ void __launch_bounds__(128, 4) fold_clusters(int n, int c0, const int32_t *__restrict__ map,
+                                                        const int32_t *__restrict__ rows,
                                                         const int32_t *__restrict__ off,
                                                         const int32_t *__restrict__ list,
                                                         const double *__restrict__ C, const double *__restrict__ csum,
