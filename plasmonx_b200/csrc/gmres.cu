@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) dots_partial(int n, int i0, int i1,
 // kernel above pays one per 128 rows and keeps only 8 loads in flight a warp).
 // Same chunking and partial layout as dots_partial.  A batch whose columns times
 // row chunks leave SMs idle spreads the vectors over blockIdx.z (the sums are the
-// same): 893 unknowns, 61 columns 47 -> 17 us a launch, 2,800 unknowns, 4
+// same): 893 unknowns, 61 columns 47 -> 16 us a launch, 2,800 unknowns, 4
 // columns (12 CTAs before) 86 -> 7.6 us.
 template <typename VT>
 __global__ void __launch_bounds__(kThreads) dots_wide(int n, int i0, int i1,
