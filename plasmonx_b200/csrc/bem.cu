@@ -448,13 +448,16 @@ void build_bem_ief(plx_geom *g) {
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     const int n = g->n_var;
-    g->d_M.alloc(ctx, (size_t)n * n);
-    g->d_DM.alloc(ctx, (size_t)n * n);
-    bem_sainv_kernel<<<dim3(n_blocks(n, 128), n), 128, 0, st>>>(n, g->d_pos.p, g->d_M.p);
+    DevArray<double> M, DM;                  // the geometry's once both are there
+    M.alloc(ctx, (size_t)n * n);
+    DM.alloc(ctx, (size_t)n * n);
+    bem_sainv_kernel<<<dim3(n_blocks(n, 128), n), 128, 0, st>>>(n, g->d_pos.p, M.p);
     ctx->launches++;
     // DM = D M (column-major: d_T row-major is D column-major)
-    bem_dgemm(g, g->d_T.p, g->d_M.p, g->d_DM.p);
+    bem_dgemm(g, g->d_T.p, M.p, DM.p);
     PLX_CHECK_CUDA(cudaGetLastError());
+    g->d_M.swap(M);
+    g->d_DM.swap(DM);
 }
 
 void bem_apply_rows(plx_geom *g, const OpBatch &b, const double *S, const double *X, double *Y) {

@@ -619,12 +619,15 @@ void diagonal_inverse(plx_geom *g, const OpBatch &b, double *Pinv) {
     plx_ctx *ctx = g->ctx;
     const int N = g->n_atoms, nt = g->n_types;
     if (!g->d_diag_a.p) {
-        g->d_diag_a.alloc(ctx, N);
-        g->d_diag_b.alloc(ctx, (size_t)N * nt);
+        DevArray<double> a, b_;              // the geometry's once both are there
+        a.alloc(ctx, N);
+        b_.alloc(ctx, (size_t)N * nt);
         diag_parts<<<n_blocks(N, 128), 128, 0, ctx->stream>>>(N, nt, g->d_pos.p, g->d_par.p, g->d_type.p,
                                                               g->d_rowptr.p, g->d_col.p, g->d_kval.p,
-                                                              g->d_ktval.p, g->d_diag_a.p, g->d_diag_b.p);
+                                                              g->d_ktval.p, a.p, b_.p);
         ctx->launches++;
+        g->d_diag_a.swap(a);
+        g->d_diag_b.swap(b_);
     }
     diag_inverse_kernel<<<dim3(n_blocks(g->n_var, 256), b.count), 256, 0, ctx->stream>>>(
         N, nt, g->n_var, b.count, nt > 1, b.d_freq, g->d_type.p, g->d_diag_a.p, g->d_diag_b.p, g->d_wratio.p,

@@ -73,6 +73,11 @@ struct DevArray {
         n = 0;
     }
     size_t bytes() const { return n * sizeof(T); }
+    void swap(DevArray &o) {
+        std::swap(ctx, o.ctx);
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+    }
 };
 
 // Pinned host doubles that kernels of the context write and the host reads after

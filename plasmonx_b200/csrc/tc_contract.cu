@@ -728,6 +728,17 @@ int make_schedule(TcLaunch &L, int sms) {
 }  // namespace
 
 
+// The word a launch reports a wait that ran out in; allocated before an operand, which is
+// complete once the geometry holds it.
+static void error_word(plx_geom *g) {
+    if (g->d_tc_err.p) return;
+    g->d_tc_err.alloc(g->ctx, 1);
+    PLX_CHECK_CUDA(cudaMemsetAsync(g->d_tc_err.p, 0, sizeof(int), g->ctx->stream));
+}
+
+// Operands are built in local arrays and handed to the geometry when complete: an
+// allocation that the budget refuses half-way leaves the geometry without an operand,
+// and a later call builds it again.
 void build_t_split(plx_geom *g) {
     if (g->d_Th.p) return;
     if (!g->has_T && is_bem(g)) throw Error(PLX_ERR_ARG, "BEM geometry without its Green-function matrix");
@@ -735,10 +746,12 @@ void build_t_split(plx_geom *g) {
     const int64_t ld = (n + kLdAlign - 1) / kLdAlign * kLdAlign;
     const int64_t rows = (n + kBM - 1) / kBM * kBM, ktiles = ld / kBK;
     g->ldk = ld;
-    g->d_Th.alloc(g->ctx, (size_t)(rows * ld));
-    g->d_Tl.alloc(g->ctx, (size_t)(rows * ld));
-    auto *hi = reinterpret_cast<__nv_bfloat16 *>(g->d_Th.p);
-    auto *lo = reinterpret_cast<__nv_bfloat16 *>(g->d_Tl.p);
+    error_word(g);
+    DevArray<uint16_t> Th, Tl;
+    Th.alloc(g->ctx, (size_t)(rows * ld));
+    Tl.alloc(g->ctx, (size_t)(rows * ld));
+    auto *hi = reinterpret_cast<__nv_bfloat16 *>(Th.p);
+    auto *lo = reinterpret_cast<__nv_bfloat16 *>(Tl.p);
     if (!g->has_T) {
         // on-the-fly geometry: the split is generated from the pair formulas
         split_tiled_gen<<<dim3((unsigned)ktiles, (unsigned)(rows / kBM)), 256, 0, g->ctx->stream>>>(
@@ -752,10 +765,8 @@ void build_t_split(plx_geom *g) {
     }
     g->ctx->launches++;
     PLX_CHECK_CUDA(cudaGetLastError());
-    if (!g->d_tc_err.p) {
-        g->d_tc_err.alloc(g->ctx, 1);
-        PLX_CHECK_CUDA(cudaMemsetAsync(g->d_tc_err.p, 0, sizeof(int), g->ctx->stream));
-    }
+    g->d_Th.swap(Th);
+    g->d_Tl.swap(Tl);
 }
 
 // Interface of an alloy: rows I with neighbours of another type, the atoms J
@@ -830,16 +841,18 @@ static void build_a_split(plx_geom *g) {
     const int64_t rows = (M + kBM - 1) / kBM * kBM, ktiles = ld / kBK;
     g->ldk = ld;
     g->fold_rows = M;
-    g->d_Ah.alloc(g->ctx, (size_t)(rows * ld));
-    g->d_Al.alloc(g->ctx, (size_t)(rows * ld));
+    error_word(g);
+    DevArray<uint16_t> Ah, Al;
+    Ah.alloc(g->ctx, (size_t)(rows * ld));
+    Al.alloc(g->ctx, (size_t)(rows * ld));
     // rows M..rows of the last m-tile are read by the kernel: zero them
-    PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Ah.p, 0, (size_t)(rows * ld) * 2, g->ctx->stream));
-    PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Al.p, 0, (size_t)(rows * ld) * 2, g->ctx->stream));
+    PLX_CHECK_CUDA(cudaMemsetAsync(Ah.p, 0, (size_t)(rows * ld) * 2, g->ctx->stream));
+    PLX_CHECK_CUDA(cudaMemsetAsync(Al.p, 0, (size_t)(rows * ld) * 2, g->ctx->stream));
     const int fmu = g->model == PLX_WFQFMU, N = g->n_atoms;
-    auto *hi = reinterpret_cast<__nv_bfloat16 *>(g->d_Ah.p);
-    auto *lo = reinterpret_cast<__nv_bfloat16 *>(g->d_Al.p);
+    auto *hi = reinterpret_cast<__nv_bfloat16 *>(Ah.p);
+    auto *lo = reinterpret_cast<__nv_bfloat16 *>(Al.p);
     cudaStream_t st = g->ctx->stream;
-    const FoldTarget out{g->d_Ah.p, g->d_Al.p, ktiles};
+    const FoldTarget out{Ah.p, Al.p, ktiles};
     if (M > N && g->has_T) {
         copy_rows_split<<<dim3((unsigned)(M - N), (unsigned)((n + 255) / 256)), 256, 0, st>>>(
             N, (int)n, ktiles, g->d_T.p, g->d_iface_atom.p, hi, lo);
@@ -853,10 +866,8 @@ static void build_a_split(plx_geom *g) {
     }
     fold_charge_rows(g, out);
     PLX_CHECK_CUDA(cudaGetLastError());
-    if (!g->d_tc_err.p) {
-        g->d_tc_err.alloc(g->ctx, 1);
-        PLX_CHECK_CUDA(cudaMemsetAsync(g->d_tc_err.p, 0, sizeof(int), g->ctx->stream));
-    }
+    g->d_Ah.swap(Ah);
+    g->d_Al.swap(Al);
 }
 
 int64_t tc_fold_rows(plx_geom *g) {
@@ -983,8 +994,13 @@ TcColumns tc_column_buffers(plx_geom *g, int count) {
     const size_t rows = 2 * (size_t)count + 16 * ((2 * (size_t)count + 255) / 256);
     const size_t need = rows * g->ldk;
     if (g->d_Xh.n < need) {
-        g->d_Xh.alloc(g->ctx, need);
-        g->d_Xl.alloc(g->ctx, need);
+        try {
+            g->d_Xh.alloc(g->ctx, need);
+            g->d_Xl.alloc(g->ctx, need);
+        } catch (...) {                      // both or none: the size of one stands for both
+            g->d_Xh.release();
+            throw;
+        }
         PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Xh.p, 0, need * 2, g->ctx->stream));
         PLX_CHECK_CUDA(cudaMemsetAsync(g->d_Xl.p, 0, need * 2, g->ctx->stream));
     }
