@@ -42,11 +42,10 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 }
 
 // A0 of one-type wFQ, column-major: A0(r, c) = sum_e K_e (T[j_e][c] - T[r][c])
-// (update_y_q of matrix_module.f90:1011-1098 applied to the columns of T); leading
-// dimension ld.  A block takes one row and kT columns, so that a neighbour's row of T is
+// (update_y_q of matrix_module.f90:1011-1098 applied to the columns of T).  A block takes one row and kT columns, so that a neighbour's row of T is
 // read contiguously and its coefficient from shared memory; a thread per row, gathering
 // down a column, took 1,024 us at 893 atoms, now 160 us.
-__global__ void __launch_bounds__(kT) wfq_a0(int N, int64_t ld, const int32_t *__restrict__ rowptr,
+__global__ void __launch_bounds__(kT) wfq_a0(int N, const int32_t *__restrict__ rowptr,
                                              const int32_t *__restrict__ col, const double *__restrict__ kval,
                                              const double *__restrict__ T, double *__restrict__ A) {
     __shared__ int32_t sj[kT];
@@ -73,12 +72,13 @@ __global__ void __launch_bounds__(kT) wfq_a0(int N, int64_t ld, const int32_t *_
         }
         for (; q < m; ++q) a += sk[q] * (T[(int64_t)sj[q] * N + cc] - trc);
     }
-    if (c < N) A[(int64_t)c * ld + r] = a;
+    if (c < N) A[(int64_t)c * N + r] = a;
 }
 
 // ---------------------------------------------------------------------------
-// The reduction.  E is column-major with 2 n rows: A in rows 0..n-1 and, below
-// it, Q (the identity at the start).  Step k eliminates column k of A below its
+// The reduction.  E = [A; Q] is column-major with 2 n rows: A in rows 0..n-1 and, below
+// it, Q (the identity at the start), each an n x n array of its own: A becomes H and Q's
+// array is Q^T row-major, so the reduction holds two matrices and leaves two.  Step k eliminates column k of A below its
 // subdiagonal with the reflector I - beta v v^T:
 //     A <- (I - beta v v^T) A (I - beta v v^T),   Q <- Q (I - beta v v^T).
 // With y = E v and z = A^T v of the matrix before the step both sides are one
@@ -99,6 +99,11 @@ constexpr int kHR = 64, kHC = 32;          // rows and columns a block's inner t
 struct HessTiles {
     int n, rt, ct, nrc, ncc;               // rows and columns a block, number of row and column tiles
 };
+// Row i of [A; Q]: its element in column j lies j n further on.
+template <typename P>
+__device__ __forceinline__ P e_row(P A, P Q, int n, int i) {
+    return i < n ? A + i : Q + (i - n);
+}
 
 HessTiles hess_tiles(int n) {
     HessTiles t;
@@ -111,11 +116,11 @@ HessTiles hess_tiles(int n) {
 }
 
 // Sum of squares of column 0 below its subdiagonal, per row tile.
-__global__ void hh_norm0(HessTiles t, const double *__restrict__ E, double *__restrict__ npart) {
+__global__ void hh_norm0(HessTiles t, const double *__restrict__ A, double *__restrict__ npart) {
     __shared__ double red[kT / 32];
     double s = 0.0;
     for (int i = blockIdx.x * t.rt + threadIdx.x; i < min(t.n, (int)(blockIdx.x + 1) * t.rt); i += blockDim.x)
-        if (i >= 2) s += E[i] * E[i];
+        if (i >= 2) s += A[i] * A[i];
     s = block_sum(s, red);
     if (threadIdx.x == 0) npart[blockIdx.x] = s;
 }
@@ -123,7 +128,8 @@ __global__ void hh_norm0(HessTiles t, const double *__restrict__ E, double *__re
 // y and z partial sums of step k over one tile, and v^T (tile) v.  Every block
 // forms the reflector itself from column k (which no later step changes) and the
 // column's norm; the first column tile's blocks store it.
-__global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const double *__restrict__ E,
+__global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const double *__restrict__ A,
+                                              const double *__restrict__ Q,
                                               const double *__restrict__ npart, double *__restrict__ vbuf,
                                               double *__restrict__ beta, double *__restrict__ sub,
                                               double *__restrict__ yp, double *__restrict__ zp,
@@ -133,11 +139,10 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
     __shared__ double red[kT / 32], yred[kT / kHR][kHR];
     double *vr = sm, *vc = vr + t.rt, *zs = vc + t.ct;        // rt, ct, 2 ct
     const int n = t.n;
-    const int64_t ld = 2 * (int64_t)n;
     const int cc = c0 + blockIdx.x, rc = blockIdx.y;
     const int i0 = rc * t.rt, i1 = min(2 * n, i0 + t.rt);
     const int j0 = cc * t.ct, j1 = min(n, j0 + t.ct);
-    const double *ck = E + (int64_t)k * ld;
+    const double *ck = A + (int64_t)k * n;
     const double x0 = ck[k + 1];
     double tail = 0.0;                                        // the same in every warp
     for (int r = threadIdx.x & 31; r < t.nrc; r += 32) tail += npart[r];
@@ -167,6 +172,7 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
     constexpr int NC = kHC / (kT / kHR);                      // columns a thread in the inner tile: 8
     for (int rs = 0; i0 + rs < i1; rs += kHR) {
         const int i = i0 + rs + row;
+        const double *e = e_row(A, Q, n, i);
         const bool in = i < i1, left = i0 + rs < n && i0 + rs + kHR > k + 1;
         const double vi = vr[rs + row];
         double y = 0.0;
@@ -175,7 +181,7 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
                 const int j = j0 + cs + cg * NC + q;
-                a[q] = in && j < j1 && j > k ? E[(int64_t)j * ld + i] : 0.0;
+                a[q] = in && j < j1 && j > k ? e[(int64_t)j * n] : 0.0;
             }
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
         if (threadIdx.x < kHR && in) {
             double s = 0.0;
             for (int c = 0; c < kT / kHR; ++c) s += yred[c][row];
-            yp[(int64_t)cc * ld + i] = s;
+            yp[(int64_t)cc * 2 * n + i] = s;
         }
         __syncthreads();
     }
@@ -209,7 +215,8 @@ __global__ void __launch_bounds__(kT) hh_gemv(HessTiles t, int k, int c0, const 
 
 // The rank-2 update of one tile, and the partial norm of column k + 1 below its
 // subdiagonal from the blocks that hold it.
-__global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, double *__restrict__ E,
+__global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, double *__restrict__ A,
+                                                double *__restrict__ Q,
                                                 const double *__restrict__ vbuf, const double *__restrict__ beta,
                                                 const double *__restrict__ yp, const double *__restrict__ zp,
                                                 const double *__restrict__ sp, double *__restrict__ npart) {
@@ -219,17 +226,17 @@ __global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, doub
     // rt, rt, ct, ct, and the partial sums' sums: 4 rt, 8 ct
     double *bv = sm, *bu = bv + t.rt, *vc = bu + t.rt, *zc = vc + t.ct, *yq = zc + t.ct, *zq = yq + 4 * t.rt;
     const int n = t.n;
-    const int64_t ld = 2 * (int64_t)n;
     const int cc = c0 + blockIdx.x, rc = blockIdx.y;
     const int i0 = rc * t.rt, i1 = min(2 * n, i0 + t.rt);
     const int j0 = cc * t.ct, j1 = min(n, j0 + t.ct);
     const int row = threadIdx.x % kHR, cg = threadIdx.x / kHR;
     constexpr int NC = kHC / (kT / kHR);
     double first[NC];                                         // the first inner tile, in flight from here
+    const double *e0 = e_row(A, Q, n, i0 + row);
 #pragma unroll
     for (int q = 0; q < NC; ++q) {
         const int j = j0 + cg * NC + q;
-        first[q] = i0 + row < i1 && j < j1 && j > k ? E[(int64_t)j * ld + i0 + row] : 0.0;
+        first[q] = i0 + row < i1 && j < j1 && j > k ? e0[(int64_t)j * n] : 0.0;
     }
     const double b = beta[0];
     const int nra = (n + t.rt - 1) / t.rt;                    // row tiles that hold rows of A
@@ -240,7 +247,7 @@ __global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, doub
         double y = 0.0;
         if (i0 + i < i1)
 #pragma unroll 8
-            for (int c = c0 + cg; c < t.ncc; c += kT / kHR) y += yp[(int64_t)c * ld + i0 + i];
+            for (int c = c0 + cg; c < t.ncc; c += kT / kHR) y += yp[(int64_t)c * 2 * n + i0 + i];
         yq[cg * t.rt + i] = y;
     }
     for (int j = threadIdx.x % kHC; j < t.ct; j += kHC) {     // eight threads a column
@@ -269,20 +276,21 @@ __global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, doub
     for (int rs = 0; i0 + rs < i1; rs += kHR) {
         const int i = i0 + rs + row;
         if (i >= i1) continue;
+        double *e = e_row(A, Q, n, i);
         const double v = bv[rs + row], u = bu[rs + row];
         for (int cs = 0; j0 + cs < j1; cs += kHC) {
             double a[NC];
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
                 const int j = j0 + cs + cg * NC + q;
-                a[q] = rs + cs == 0 ? first[q] : (j < j1 && j > k ? E[(int64_t)j * ld + i] : 0.0);
+                a[q] = rs + cs == 0 ? first[q] : (j < j1 && j > k ? e[(int64_t)j * n] : 0.0);
             }
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
                 const int j = j0 + cs + cg * NC + q;
                 if (j < j1 && j > k) {
                     const double x = a[q] - (v * zc[cs + cg * NC + q] + u * vc[cs + cg * NC + q]);
-                    E[(int64_t)j * ld + i] = x;
+                    e[(int64_t)j * n] = x;
                     if (j == k + 1 && i >= k + 3 && i < n) sq += x * x;
                 }
             }
@@ -294,35 +302,31 @@ __global__ void __launch_bounds__(kT) hh_update(HessTiles t, int k, int c0, doub
     }
 }
 
-__global__ void hess_identity(int n, double *__restrict__ E) {
+__global__ void hess_identity(int n, double *__restrict__ Q) {
     const int j = blockIdx.y;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        E[(int64_t)j * 2 * n + n + i] = i == j ? 1.0 : 0.0;
+        Q[(int64_t)j * n + i] = i == j ? 1.0 : 0.0;
 }
 
-// H row-major (the rows the Givens sweep reads), upper Hessenberg part, and Q and
-// Q^T row-major, from E: 32 x 32 tiles through shared memory.
-__global__ void hess_unpack(int n, const double *__restrict__ E, const double *__restrict__ sub,
-                            double *__restrict__ Hr, double *__restrict__ Q, double *__restrict__ Qt) {
-    __shared__ double th[32][33], tq[32][33];
-    const int64_t ld = 2 * (int64_t)n;
-    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + threadIdx.x, c = c0 + y;
-        if (r >= n || c >= n) continue;
-        th[y][threadIdx.x] = c >= r ? E[(int64_t)c * ld + r]
-                                    : (c == r - 1 ? (c + 2 < n ? sub[c] : E[(int64_t)c * ld + r]) : 0.0);
-        const double q = E[(int64_t)c * ld + n + r];
-        tq[y][threadIdx.x] = q;
-        Qt[(int64_t)c * n + r] = q;
-    }
+// The reduced A, column-major, to H row-major (the rows the Givens sweep reads) in
+// place, upper Hessenberg part: a block exchanges two mirrored 32 x 32 tiles.
+__global__ void hess_rows(int n, double *__restrict__ A, const double *__restrict__ sub) {
+    if (blockIdx.x < blockIdx.y) return;
+    __shared__ double tile[2][32][33];                        // rows of block x, columns of block y; the mirror
+    const int b[2] = {(int)blockIdx.x * 32, (int)blockIdx.y * 32};
+    for (int m = 0; m < 2; ++m)
+        for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+            const int r = b[m] + threadIdx.x, c = b[1 - m] + y;
+            if (r >= n || c >= n) continue;
+            const double a = A[(int64_t)c * n + r];
+            tile[m][y][threadIdx.x] = c >= r ? a : (c == r - 1 ? (c + 2 < n ? sub[c] : a) : 0.0);
+        }
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + y, c = c0 + threadIdx.x;
-        if (r >= n || c >= n) continue;
-        Hr[(int64_t)r * n + c] = th[threadIdx.x][y];
-        Q[(int64_t)r * n + c] = tq[threadIdx.x][y];
-    }
+    for (int m = 0; m < 2; ++m)                               // (on the diagonal both are the same tile)
+        for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+            const int r = b[m] + y, c = b[1 - m] + threadIdx.x;
+            if (r < n && c < n) A[(int64_t)r * n + c] = tile[m][threadIdx.x][y];
+        }
 }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -519,58 +523,60 @@ void build_hessenberg(plx_geom *g) {
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     const int n = g->n_var;
-    const int64_t ld = 2 * (int64_t)n;
     const HessTiles t = hess_tiles(n);
-    DevArray<double> E, vbuf, beta, sub, npart, yp, zp, sp;
-    E.alloc(ctx, (size_t)ld * n);
+    DevArray<double> A, Q, vbuf, beta, sub, npart, yp, zp, sp;
+    A.alloc(ctx, (size_t)n * n);
+    Q.alloc(ctx, (size_t)n * n);
     vbuf.alloc(ctx, n);
     beta.alloc(ctx, 1);
     sub.alloc(ctx, n);
     npart.alloc(ctx, 2 * (size_t)t.nrc);
-    yp.alloc(ctx, (size_t)t.ncc * ld);
+    yp.alloc(ctx, (size_t)t.ncc * 2 * n);
     zp.alloc(ctx, (size_t)t.nrc * n);
     sp.alloc(ctx, (size_t)t.nrc * t.ncc);
     if (is_bem(g)) {
         // D stored transposed (d_T[j][i] = D(i, j)) is D column-major
-        PLX_CHECK_CUDA(cudaMemcpy2DAsync(E.p, ld * 8, g->d_T.p, (size_t)n * 8, (size_t)n * 8, n,
-                                         cudaMemcpyDeviceToDevice, st));
+        PLX_CHECK_CUDA(cudaMemcpyAsync(A.p, g->d_T.p, (size_t)n * n * 8, cudaMemcpyDeviceToDevice, st));
     } else {
-        wfq_a0<<<dim3(n, n_blocks(n, kT)), kT, 0, st>>>(n, ld, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_T.p, E.p);
+        wfq_a0<<<dim3(n, n_blocks(n, kT)), kT, 0, st>>>(n, g->d_rowptr.p, g->d_col.p, g->d_kval.p, g->d_T.p, A.p);
         ctx->launches++;
     }
-    hess_identity<<<dim3(n_blocks(n, kT), n), kT, 0, st>>>(n, E.p);
-    hh_norm0<<<t.nrc, kT, 0, st>>>(t, E.p, npart.p);
+    hess_identity<<<dim3(n_blocks(n, kT), n), kT, 0, st>>>(n, Q.p);
+    hh_norm0<<<t.nrc, kT, 0, st>>>(t, A.p, npart.p);
     ctx->launches += 2;
     const size_t sm_gemv = (size_t)(t.rt + 3 * t.ct) * 8, sm_upd = (size_t)(6 * t.rt + 10 * t.ct) * 8;
     for (int k = 0; k + 2 < n; ++k) {
         const int c0 = (k + 1) / t.ct;                        // first column tile with columns right of k
         const dim3 grid(t.ncc - c0, t.nrc);
         double *np0 = npart.p + (k & 1) * t.nrc, *np1 = npart.p + ((k + 1) & 1) * t.nrc;
-        launch_pdl(hh_gemv, grid, kT, sm_gemv, st, t, k, c0, E.p, np0, vbuf.p, beta.p, sub.p, yp.p, zp.p, sp.p);
-        launch_pdl(hh_update, grid, kT, sm_upd, st, t, k, c0, E.p, vbuf.p, beta.p, yp.p, zp.p, sp.p, np1);
+        launch_pdl(hh_gemv, grid, kT, sm_gemv, st, t, k, c0, A.p, Q.p, np0, vbuf.p, beta.p, sub.p, yp.p, zp.p, sp.p);
+        launch_pdl(hh_update, grid, kT, sm_upd, st, t, k, c0, A.p, Q.p, vbuf.p, beta.p, yp.p, zp.p, sp.p, np1);
         ctx->launches += 2;
     }
-    g->d_hess_q.alloc(ctx, (size_t)n * n);
-    g->d_hess_qt.alloc(ctx, (size_t)n * n);
-    g->d_hess_rows.alloc(ctx, (size_t)n * n);
-    hess_unpack<<<dim3(n_blocks(n, 32), n_blocks(n, 32)), dim3(32, 8), 0, st>>>(n, E.p, sub.p, g->d_hess_rows.p,
-                                                                              g->d_hess_q.p, g->d_hess_qt.p);
+    hess_rows<<<dim3(n_blocks(n, 32), n_blocks(n, 32)), dim3(32, 8), 0, st>>>(n, A.p, sub.p);
     ctx->launches++;
     PLX_CHECK_CUDA(cudaGetLastError());
     PLX_CHECK_CUDA(cudaStreamSynchronize(st));
+    g->d_hess_qt.swap(Q);
+    g->d_hess_rows.swap(A);
 }
 
 // Solves A(w_f) x = b for the frequencies of `freqs` (cols right-hand sides each,
 // B and X [freqs.size() * cols][2][n], frequency-major).  Returns false when a
 // frequency's triangular factor has a zero on its diagonal (singular A(w)), or
-// when the reduction (five n x n matrices while it runs) does not fit the budget:
-// the caller then factors A(w) per frequency, which needs two.
+// when there is no room beside T for three n x n matrices (H, Q^T and one frequency's
+// triangular factor): the caller then factors A(w) per frequency, which needs two and
+// the LU's work space.
 static bool shifted_solve(plx_geom *g, const std::vector<int32_t> &freqs, int cols, const double *B, double *X) {
-    build_hessenberg(g);
     plx_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     const int n = g->n_var;
     const int F = (int)freqs.size();
+    const size_t rbytes = (size_t)n * (n + 1) / 2 * sizeof(double2);
+    auto room = [&] { return ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : 0; };
+    // no reduction for a solve that has no room
+    if (ctx->budget && room() < rbytes + (g->d_hess_rows.p ? 0 : 16 * (uint64_t)n * n)) return false;
+    build_hessenberg(g);
     if (F == 0) return true;
     const std::vector<Cplx> shifts = hessenberg_shifts(g);
     DevArray<Cplx> d_shift;
@@ -582,10 +588,7 @@ static bool shifted_solve(plx_geom *g, const std::vector<int32_t> &freqs, int co
         PLX_CHECK_CUDA(cudaFuncSetAttribute(hess_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     });
     // waves of frequencies whose triangular factors fit a quarter of the budget
-    const size_t rbytes = (size_t)n * (n + 1) / 2 * sizeof(double2);
-    const uint64_t avail = ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : 0;
-    const int wave = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)F, avail / 4 / rbytes));
-    DevArray<double> Y;
+    const int wave = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)F, room() / 4 / rbytes));
     DevArray<double2> R;
     DevArray<int32_t> d_f;
     DevArray<int> sing;
@@ -594,17 +597,20 @@ static bool shifted_solve(plx_geom *g, const std::vector<int32_t> &freqs, int co
     sing.alloc(ctx, 1);
     PLX_CHECK_CUDA(cudaMemcpyAsync(d_f.p, freqs.data(), F * 4, cudaMemcpyHostToDevice, st));
     PLX_CHECK_CUDA(cudaMemsetAsync(sing.p, 0, sizeof(int), st));
-    // Q^T b and x = Q y of every right-hand side as one product each
-    Y.alloc(ctx, (size_t)F * cols * 2 * n);
-    stored_product(ctx, g->d_part, 2 * F * cols, n, B, g->d_hess_q.p, Y.p);
+    // a wave's Q^T b and x = Q y are one product each, in X and with the triangular
+    // factors' memory for the partial sums (a product of the whole grid with memory of its
+    // own took 167 MB at 893 unknowns and 61 frequencies)
+    double *part = reinterpret_cast<double *>(R.p);
+    const size_t prows = (size_t)wave * n * (n + 1);
     for (int f0 = 0; f0 < F; f0 += wave) {
         const int nf = std::min(wave, F - f0);
-        hess_solve<<<nf, kSolveT, smem, st>>>(n, cols, d_f.p + f0, d_shift.p, g->d_hess_rows.p,
-                                              Y.p + (size_t)f0 * cols * 2 * n, R.p, sing.p);
+        double *x = X + (size_t)f0 * cols * 2 * n;
+        product_in_room(ctx, part, prows, 2 * nf * cols, n, B + (size_t)f0 * cols * 2 * n, g->d_hess_qt.p, true, x);
+        hess_solve<<<nf, kSolveT, smem, st>>>(n, cols, d_f.p + f0, d_shift.p, g->d_hess_rows.p, x, R.p, sing.p);
         ctx->launches++;
         PLX_CHECK_CUDA(cudaGetLastError());
+        product_in_room(ctx, part, prows, 2 * nf * cols, n, x, g->d_hess_qt.p, false, x);
     }
-    stored_product(ctx, g->d_part, 2 * F * cols, n, Y.p, g->d_hess_qt.p, X);
     int hs = 0;
     PLX_CHECK_CUDA(cudaMemcpyAsync(&hs, sing.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     PLX_CHECK_CUDA(cudaStreamSynchronize(st));
@@ -616,10 +622,8 @@ bool hessenberg_solve(plx_geom *g, const std::vector<int32_t> &freqs, int cols, 
         return shifted_solve(g, freqs, cols, B, X);
     } catch (const Error &e) {
         if (e.code != PLX_ERR_BUDGET && e.code != PLX_ERR_NOMEM) throw;
-        if (!g->d_hess_rows.p) {
-            g->d_hess_q.release();
-            g->d_hess_qt.release();
-        }
+        g->d_hess_qt.release();              // the LU gets the reduction's room
+        g->d_hess_rows.release();
         return false;
     }
 }

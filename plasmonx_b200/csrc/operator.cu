@@ -688,16 +688,29 @@ void contract_t(plx_geom *g, int count, const double *X, double *S, Contraction 
 // the split-K products of skinny.cuh, the partial sums in `scratch` (grown on demand).
 // A row's result does not depend on R.
 void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const double *X, const double *T, double *S) {
+    int ks, kchunk;
+    skinny_split(n, ks, kchunk);
+    const size_t need = (size_t)ks * R * n;
+    if (scratch.n < need) scratch.alloc(ctx, need);
+    product_in_room(ctx, scratch.p, need, R, n, X, T, false, S);
+}
+
+void product_in_room(plx_ctx *ctx, double *scratch, size_t room, int R, int n, const double *X, const double *T,
+                     bool transposed, double *S) {
     // K split: depends on n only (not on the batch)
     int ks, kchunk;
     skinny_split(n, ks, kchunk);
-    size_t need = (size_t)ks * R * n;
-    if (scratch.n < need) scratch.alloc(ctx, need);
-    double *part = scratch.p;
+    const int most = (int)std::min<size_t>((size_t)R, room / ((size_t)ks * n));
+    if (most < 1) throw Error(PLX_ERR_ARG, "no room for a row of the product");
     cudaStream_t st = ctx->stream;
-    launch_product_partial(st, R, n, ks, kchunk, X, T, part);
-    launch_pdl(skinny_reduce, n_blocks((int64_t)R * n, 256), 256, 0, st, n, R, ks, part, S);
-    ctx->launches += 2;
+    for (int r0 = 0; r0 < R; r0 += most) {
+        const int nr = std::min(most, R - r0);
+        const int64_t at = (int64_t)r0 * n;
+        if (transposed) launch_product_partial<true>(st, nr, n, ks, kchunk, X + at, T, scratch);
+        else launch_product_partial(st, nr, n, ks, kchunk, X + at, T, scratch);
+        launch_pdl(skinny_reduce, n_blocks((int64_t)nr * n, 256), 256, 0, st, n, nr, ks, scratch, S + at);
+        ctx->launches += 2;
+    }
     PLX_CHECK_CUDA(cudaGetLastError());
 }
 

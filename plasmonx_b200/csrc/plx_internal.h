@@ -211,9 +211,8 @@ struct plx_geom {
     plx::DevArray<double> d_part;
     // continuous batches open on this geometry (they own its frequency table)
     int open_batches = 0;
-    // Hessenberg reduction A0 = Q H Q^T of the scalar-shift models: Q and Q^T
-    // row-major, and H row-major
-    plx::DevArray<double> d_hess_q, d_hess_qt, d_hess_rows;
+    // Hessenberg reduction A0 = Q H Q^T of the scalar-shift models: Q^T and H row-major
+    plx::DevArray<double> d_hess_qt, d_hess_rows;
     // timing of the last plx_solve
     double last_ms = 0.0;
     int64_t last_launches = 0;
@@ -253,6 +252,10 @@ void apply_operator(plx_geom *g, const OpBatch &b, const double *X, double *Y, d
 void contract_t(plx_geom *g, int count, const double *X, double *S, Contraction how);
 //   S = X T for rows X [R][n] and a row-major n x n matrix in FP64
 void stored_product(plx_ctx *ctx, DevArray<double> &scratch, int R, int n, const double *X, const double *T, double *S);
+//   the same in `room` doubles of scratch (n^2 always suffice), rows at a time as they
+//   fit; transposed: with T^T given.  S may be X.
+void product_in_room(plx_ctx *ctx, double *scratch, size_t room, int R, int n, const double *X, const double *T,
+                     bool transposed, double *S);
 void rhs_batch(plx_geom *g, const OpBatch &b, const int32_t *d_pol, double *Bout);
 //   1 / diag(A(w_c)) for every column, [count][2][n] split complex.
 void diagonal_inverse(plx_geom *g, const OpBatch &b, double *Pinv);

@@ -28,9 +28,11 @@ constexpr int kSkinnyCols = 256;
 // HBM).  The matrix instruction reads eight times fewer operands per FMA.
 //   15,220 unknowns (T 1.85 GB): 6 rows 366 -> 281 us (6.6 TB/s), 12 rows 889 ->
 //   366, 32 rows 1,098 -> 686, 42 rows 1,470 -> 863, 512 rows 12.4 -> 7.9 ms (30 TF).
-// Rows beyond the batch and k beyond the chunk are zeros.  The order of an
+// TR: the matrix is given by its transpose (T[k][col] lies at T[col * n + k]), read in
+// 32-byte pieces; the sums are the same.  Rows beyond the batch and k beyond the chunk
+// are zeros.  The order of an
 // element's sum depends on n alone (skinny_split): not on R, MT, NT or its place.
-template <int MT, int NT, int D, int WR, int MB>
+template <int MT, int NT, int D, int WR, int MB, bool TR>
 __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kchunk, const double *__restrict__ Xt,
                                                            const double *__restrict__ T,
                                                            double *__restrict__ part) {
@@ -49,7 +51,9 @@ __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kch
         const bool in = k + kk < k1;
 #pragma unroll
         for (int t = 0; t < NT; ++t)
-            b[s][t] = in && col0 + 8 * t + g < n ? __ldg(T + (int64_t)(k + kk) * n + col0 + 8 * t + g) : 0.0;
+            b[s][t] = in && col0 + 8 * t + g < n ? __ldg(TR ? T + (int64_t)(col0 + 8 * t + g) * n + k + kk
+                                                            : T + (int64_t)(k + kk) * n + col0 + 8 * t + g)
+                                                 : 0.0;
 #pragma unroll
         for (int m = 0; m < MT; ++m)
             a[s][m] = in && row0 + 8 * m + g < R ? __ldg(Xt + (int64_t)(row0 + 8 * m + g) * n + k + kk) : 0.0;
@@ -83,10 +87,11 @@ __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kch
 // eights that hold the batch up to 48 rows (the fastest of the tilings tried at each
 // size, 2 to 5 each at 893, 7,844 and 15,220 unknowns); 32 rows a warp above, where
 // the smaller tile's four blocks an SM beat 64 x 64 tiles (30 against 26 TF).
-inline void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, const double *X, const double *T,
+template <bool TR = false>
+void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, const double *X, const double *T,
                                    double *part) {
 #define PLX_PP(MT, NT, D, WR, MB)                                                                                  \
-    launch_pdl(product_partial<MT, NT, D, WR, MB>,                                                                 \
+    launch_pdl(product_partial<MT, NT, D, WR, MB, TR>,                                                                 \
                dim3((n + 32 / WR * NT - 1) / (32 / WR * NT), (R + 8 * MT * WR - 1) / (8 * MT * WR), ks), 128, 0, st, R, \
                n, kchunk, X, T, part)
     if (R <= 8) PLX_PP(1, 4, 4, 1, 1);
