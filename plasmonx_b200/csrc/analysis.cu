@@ -274,13 +274,22 @@ void field_at_points(plx_geom *g, int pol, const double *d_x, int P, const doubl
             N, N, pol, g->e0, P, g->d_pos.p, g->d_par.p, x, d_pts, fo, de, nullptr);
         ctx->launches++;
     } else {
-        // a block for about every resident slot of the chip, at least a tile of atoms each
+        // a block for about every resident slot of the chip, at least a tile of atoms each;
+        // fewer parts where their sums (up to 10 MB) find no room, one needs none
         const int blocks = n_blocks(P, kPts);
-        int ny = std::max(1, std::min(n_blocks(N, kPts), 1184 / blocks));
-        const int achunk = n_blocks(n_blocks(N, ny), kPts) * kPts;
-        ny = n_blocks(N, achunk);
+        int ny = std::max(1, std::min(n_blocks(N, kPts), 1184 / blocks)), achunk;
         DevArray<double> part;
-        if (ny > 1) part.alloc(ctx, 8 * (size_t)P * ny);
+        for (;; ny /= 2) {
+            achunk = n_blocks(n_blocks(N, ny), kPts) * kPts;
+            ny = n_blocks(N, achunk);
+            if (ny == 1) break;
+            try {
+                part.alloc(ctx, 8 * (size_t)P * ny);
+                break;
+            } catch (const Error &e) {
+                if (e.code != PLX_ERR_BUDGET && e.code != PLX_ERR_NOMEM) throw;
+            }
+        }
         (fmu ? field_points<1, true> : field_points<1, false>)<<<dim3(blocks, ny), kPts, 0, ctx->stream>>>(
             N, achunk, pol, g->e0, P, g->d_pos.p, g->d_par.p, x, d_pts, fo, de, ny > 1 ? part.p : nullptr);
         ctx->launches++;
