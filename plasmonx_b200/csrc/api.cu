@@ -43,7 +43,7 @@ void plx::dev_free(plx_ctx *ctx, void *p, size_t bytes) {
     ctx->in_use -= bytes;
 }
 
-void plx::PinnedArray::alloc(plx_ctx *c, size_t count) {
+void plx::PinnedArray::alloc(plx_ctx *c, size_t count, bool pin) {
     release();
     ctx = c;
     if (count == 0) return;
@@ -58,7 +58,13 @@ void plx::PinnedArray::alloc(plx_ctx *c, size_t count) {
             }
         count = (count + 511) / 512 * 512;
     }
-    PLX_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), count * sizeof(double), cudaHostAllocDefault));
+    if (!pin) return;
+    void *q = nullptr;
+    if (cudaHostAlloc(&q, count * sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    p = static_cast<double *>(q);
     n = count;
 }
 

@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kThreads) norm_partial(int n, const double *__
     if (threadIdx.x == 0) part[(int64_t)k * gridDim.x + blockIdx.x] = s;
 }
 
-// `host`: the same norms in the run's pinned block
+// `host`: the same norms in the run's words
 __global__ void norm_finish(int nchunk, int count, const double *__restrict__ part,
                             double *__restrict__ out, double *__restrict__ host) {
     pdl_sync();
@@ -739,9 +739,9 @@ __device__ void givens(int k, int lane, int j, double norm, const GivensTile &ti
 // of W themselves (up to kNormChunks, in norm_partial's order).
 //
 // The launch also enters the new slab and H column in the address tables, which the
-// kernels of the next steps read, and leaves the residual estimates in pinned host
-// memory: three 8-byte copies in, one back and a clearing of the H column (every row
-// that is read has been written) cost a step about 20 us of gaps between the kernels.
+// kernels of the next steps read, and leaves the residual estimates in the run's words
+// (take_words): three 8-byte copies in, one back and a clearing of the H column (every
+// row that is read has been written) cost a step about 20 us of gaps between the kernels.
 constexpr int kNormChunks = 2;
 template <typename VT>
 __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,
@@ -1093,7 +1093,7 @@ class GmresRun final : public GmresStepper {
         std::vector<DevArray<double2>>(m_).swap(hcols_);
         d_slabs_.alloc(ctx_, m_ + 1);
         d_hcols_.alloc(ctx_, m_);
-        host_.alloc(ctx_, (size_t)2 * C_);
+        take_words();
         PLX_CHECK_CUDA(cudaMemsetAsync(d_X_, 0, (size_t)C_ * 2 * n * 8, st_));
         if (rq_.contraction == Contraction::TC3 || rq_.contraction == Contraction::TC1) split_ = tc_presplit(g_, C_);
         jac_ = rq_.jacobi && rq_.inner;
@@ -1108,13 +1108,12 @@ class GmresRun final : public GmresStepper {
         act_.resize(C_);
         for (int c = 0; c < C_; ++c) act_[c] = c;
         PLX_CHECK_CUDA(cudaMemcpyAsync(d_act_.p, act_.data(), C_ * 4, cudaMemcpyHostToDevice, st_));
-        batch_norms(g_, C_, d_B_, nrm_part_, nrm_, host_.p);   // B is [C] in column order == compact order here
+        batch_norms(g_, C_, d_B_, nrm_part_, nrm_, words());   // B is [C] in column order == compact order here
         slabs_[0].alloc(ctx_, (size_t)C_ * 2 * n);
         start_vectors<VT><<<dim3(grid_rows(2LL * n), C_), 256, 0, st_>>>(n, d_act_.p, nrm_.p, d_B_, slabs_[0].p,
                                                                       d_slabs_.p, gv_.p, hstride_);
         ctx_->launches++;
-        PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
-        const double *bnorm = host_.p;
+        const double *bnorm = read_words(0, C_);
         act_.clear();
         for (int c = 0; c < C_; ++c) {
             if (!std::isfinite(bnorm[c])) {
@@ -1192,11 +1191,12 @@ class GmresRun final : public GmresStepper {
             }
         }
         prof_end(ctx_, PROF_ORTHO, 0.0, 0.0);
-        for (int k = 0; k < na; ++k) memcpy(host_.p + k, &kPending, 8);
+        if (!host_.p) take_words();
+        for (int k = 0; host_.p && k < na; ++k) memcpy(host_.p + k, &kPending, 8);
         prof_begin(ctx_);
         launch_pdl(normalize_givens<VT>, dim3(grid_rows(n) + 1, na), 256, 0, st_, n, j, d_act_.p, nparts, nrm_part_.p,
                    Wa_.p, slabs_[j + 1].p, jac_ ? Pinv_.p : nullptr, Xa_.p, split_, d_slabs_.p, d_hcols_.p,
-                   hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, host_.p);
+                   hcols_[j].p, hstride_, cs_.p, sn_.p, gv_.p, hstride_, m_, words());
         ctx_->launches++;
         x_ready_ = true;
         prof_end(ctx_, PROF_LSQ, 0.0, 0.0);
@@ -1208,8 +1208,7 @@ class GmresRun final : public GmresStepper {
         const int n = g_->n_var;
         const int j = j_;
         const int na = (int)act_.size();
-        const double *resid = host_.p;
-        await_residuals(na);
+        const double *resid = await_residuals(na);
         std::vector<int32_t> trig;
         for (int k = 0; k < na; ++k) {
             int c = act_[k];
@@ -1259,9 +1258,8 @@ class GmresRun final : public GmresStepper {
                                : Contraction::FP64);
             launch_pdl(residual, dim3(grid_rows(2LL * n), nt), 256, 0, st_, n, d_cols_.p, d_B_, Wa_.p);
             ctx_->launches++;
-            const double *tres = host_.p + C_;
-            batch_norms(g_, nt, Wa_.p, nrm_part_, nrm_, host_.p + C_);
-            PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
+            batch_norms(g_, nt, Wa_.p, nrm_part_, nrm_, words() + C_);
+            const double *tres = read_words(C_, nt);
             for (int t = 0; t < nt; ++t)
                 if (tres[t] < rq_.tol) done[trig[t]] = 1;
                 else if (!std::isfinite(tres[t])) {
@@ -1309,7 +1307,11 @@ class GmresRun final : public GmresStepper {
     // for the stream brings the next product forward: 9.8 -> 5.4 us after the step of a
     // matrix-free solve of 700 atoms, 12.2 -> 5.3 for six structures served together.
     // A residual with the pending word's bits costs that wait, nothing else.
-    void await_residuals(int na) {
+    const double *await_residuals(int na) {
+        if (!host_.p) {
+            ++ctx_->copied_steps;
+            return read_words(0, na);
+        }
         const volatile uint64_t *w = reinterpret_cast<const volatile uint64_t *>(host_.p);
         int k = 0;
         for (int polls = 0; k < na && polls < kPolls;) {
@@ -1321,6 +1323,30 @@ class GmresRun final : public GmresStepper {
         }
         if (k < na) PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
         std::atomic_thread_fence(std::memory_order_acquire);
+        return host_.p;
+    }
+
+    // The words the kernels leave norms and residuals in: pinned host memory once the
+    // context has taken kCopiedSteps steps, device memory and a copy before that and
+    // where no memory can be pinned (tried again as many steps later).
+    void take_words() {
+        const bool pin = ctx_->copied_steps >= kCopiedSteps;
+        host_.alloc(ctx_, (size_t)2 * C_, pin);
+        if (host_.p) return;
+        if (pin) ctx_->copied_steps = 0;
+        if (!dev_words_.p) {
+            dev_words_.alloc(ctx_, (size_t)2 * C_);
+            copy_.resize((size_t)2 * C_);
+        }
+    }
+    double *words() { return host_.p ? host_.p : dev_words_.p; }
+    // `count` words from `first`, written by kernels already launched
+    const double *read_words(int first, int count) {
+        if (!host_.p)
+            PLX_CHECK_CUDA(cudaMemcpyAsync(copy_.data() + first, dev_words_.p + first, (size_t)count * 8,
+                                           cudaMemcpyDeviceToHost, st_));
+        PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
+        return (host_.p ? host_.p : copy_.data()) + first;
     }
 
     void upload_active() {
@@ -1346,6 +1372,8 @@ class GmresRun final : public GmresStepper {
     bool x_ready_ = false;      // Xa holds the next product's input
     std::vector<int32_t> act_;
     PinnedArray host_;          // residual estimates [C], true residuals [C]
+    DevArray<double> dev_words_;             // the same without pinned memory,
+    std::vector<double> copy_;               // and its copy
     DevArray<int32_t> d_act_, d_freq_act_, d_cols_;
     DevArray<double> Xa_, Wa_, work_, nrm_part_, nrm_, cs_, Pinv_;
     DevArray<double2> sn_, gv_, hbuf_, part_, ybuf_;

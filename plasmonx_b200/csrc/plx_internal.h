@@ -83,7 +83,8 @@ struct DevArray {
 // Pinned host doubles that kernels of the context write and the host reads after
 // a synchronisation (zero copy).  Blocks of up to kPinnedKeep doubles go back to
 // the context's list (kPinnedBlocks at most), which its destruction frees: pinning
-// memory costs more than a small solve's step.
+// memory costs more than a small solve's steps.  alloc() leaves p null where the list
+// has no block and `pin` is false, or where the system refuses to pin memory.
 struct PinnedArray {
     plx_ctx *ctx = nullptr;
     double *p = nullptr;
@@ -92,11 +93,19 @@ struct PinnedArray {
     PinnedArray(const PinnedArray &) = delete;
     PinnedArray &operator=(const PinnedArray &) = delete;
     ~PinnedArray() { release(); }
-    void alloc(plx_ctx *c, size_t count);
+    void alloc(plx_ctx *c, size_t count, bool pin);
     void release();
 };
 constexpr size_t kPinnedKeep = 8192;      // 64 KB
 constexpr size_t kPinnedBlocks = 32;
+// GMRES steps of a context that read their residuals by a copy before it pins memory
+// for them.  Pinning takes 1-3.4 ms, a step's copy 12-14 us more than reading pinned
+// words (262 steps at 893 unknowns: 43.2 against 39.6 ms): 96 steps cost about what the
+// pinning does, so a context that takes few steps never pays for it and one that takes
+// many pays about twice the cheaper form, once.  First solve of a new 8,000-tessera
+// surface (53 steps; 19.5 ms after it): 30.6 ms pinned from the first step, 29.4 now; of
+// 893 unknowns (262 steps; 39.6 ms): 45.2 and 45.3 (quartiles of 16 new contexts).
+constexpr int64_t kCopiedSteps = 96;
 
 }  // namespace plx
 
@@ -124,6 +133,7 @@ struct plx_ctx {
     uint32_t wait_limit = kDefaultWaitLimit;
     std::mutex pinned_mutex;
     std::vector<std::pair<double *, size_t>> pinned;   // free blocks of PinnedArray
+    int64_t copied_steps = 0;                          // see kCopiedSteps
     // contraction profiling (plx_profile_enable)
     bool profile = false;
     std::vector<cudaEvent_t> prof_events;   // pairs (start, stop), reused
