@@ -27,6 +27,7 @@
 #include <memory>
 #include <type_traits>
 
+#include "cpu_relax.h"
 #include "pdl.cuh"
 #include "plx_internal.h"
 
@@ -1318,7 +1319,7 @@ class GmresRun final : public GmresStepper {
             if (w[k] != kPending) ++k;
             else {
                 ++polls;
-                __builtin_ia32_pause();
+                cpu_relax();
             }
         }
         if (k < na) PLX_CHECK_CUDA(cudaStreamSynchronize(st_));
