@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(kTiledThreads) otf_tiled_partial(int R, int n,
     constexpr int CA = BN / NC;                // target atoms a block
     constexpr int MT = BM / 8, NT = BN / 32;   // 8 x 8 tiles of a warp
     __shared__ double As[BM][16 + 4];          // the paddings spread a fragment over the banks
-    __shared__ double Bs[16][BN + 4];
+    __shared__ __align__(16) double Bs[16][BN + 4];        // written two elements at a time
+    static_assert((BN + 4) % 2 == 0 && BN % 4 == 0, "a row of Bs and an atom's components start at 16 bytes");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kk = lane & 3, g = lane >> 2;
     const int row0 = blockIdx.y * BM, i0 = blockIdx.x * CA;
     const int jbeg = blockIdx.z * jchunk, jend = min(N, jbeg + jchunk);
