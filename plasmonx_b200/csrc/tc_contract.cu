@@ -17,7 +17,7 @@
 // epilogue, one thread of warp 4 issues the loads and one of warp 5 the MMAs.
 // Operand tiles are 32 elements (64 bytes) deep along k and are
 // loaded by TMA with the 64-byte swizzle that the UMMA descriptors describe;
-// the small stages allow 4-6 of them in flight.
+// the small stages allow 3-6 of them in flight with three products, 7 or 8 with one.
 // Every wait on an mbarrier is bounded.  The pipeline waits use the context's
 // limit (plx_set_wait_limit); a CTA whose wait runs out records an error code
 // and gives up, in this order: the MMA issuer still commits `drained`, which
@@ -193,7 +193,6 @@ struct TcGroup {
     int unit0;                  // k-tiles of the split tiles before the group
     const uint8_t *ah, *al;     // A high / low, tile-ordered and pre-swizzled (16 KB per stage tile)
     double *S;                  // [R][M] FP64
-    int *err;                   // the geometry's error word (first bounded wait that ran out)
     TcRows rows;
 };
 struct TcLaunch {
@@ -206,6 +205,7 @@ struct TcLaunch {
     int stages;                 // pipeline depth
     int bn_max;                 // shared-memory / tensor-memory sizing
     uint32_t wait_limit;
+    int *err;                   // first bounded wait that ran out: the first group's geometry's word, the launch's only one
 };
 
 // A piece of work of a CTA: k-tiles [kt0, kt0 + nk) of a group's tile.
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_contract_kernel(const __grid
     uint64_t *drained = freed + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *err = p.grp[0].err;
+    int *err = p.err;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -959,9 +959,10 @@ void tc_contract_group(const std::vector<TcItem> &items) {
         }
         L.tiles += (M + kBM - 1) / kBM * ntile;
         bn_max = std::max(bn_max, (bn + 31) / 32 * 32);
-        if (!g->d_tc_err.p) throw Error(PLX_ERR_CUDA, "tensor-core error word missing");
-        gp.err = g->d_tc_err.p;
     }
+    // callers poll the words of every geometry of the group
+    L.err = items[order[0]].g->d_tc_err.p;
+    if (!L.err) throw Error(PLX_ERR_CUDA, "tensor-core error word missing");
     L.bn_max = bn_max;
     const int ctas = make_schedule(L, sms);
     const int split = L.tiles - L.full;
