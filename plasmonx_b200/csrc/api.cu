@@ -99,6 +99,22 @@ plx_status guarded(plx_ctx *ctx, F &&f) {
     }
 }
 
+// The geometry's frequencies as they are, put back unless the change is done.
+struct KeepFrequencies {
+    plx_geom *g;
+    int n_freq;
+    std::vector<double> omega;
+    std::vector<Cplx> alpha_w;
+    bool done = false;
+    explicit KeepFrequencies(plx_geom *geom) : g(geom), n_freq(g->n_freq), omega(g->omega), alpha_w(g->alpha_w) {}
+    ~KeepFrequencies() {
+        if (done) return;
+        g->n_freq = n_freq;
+        g->omega.swap(omega);
+        g->alpha_w.swap(alpha_w);
+    }
+};
+
 void set_device(plx_ctx *ctx) { PLX_CHECK_CUDA(cudaSetDevice(ctx->device)); }
 
 // host interleaved complex (n) <-> device split [2][n]
@@ -351,7 +367,22 @@ plx_status plx_set_frequencies(plx_geom *g, int32_t n_freq, const double *omega,
             g->alpha_w.resize((size_t)g->n_types * n_freq);
             for (size_t e = 0; e < g->alpha_w.size(); ++e) g->alpha_w[e] = {alpha_w[2 * e], alpha_w[2 * e + 1]};
         }
-        upload_frequency_tables(g);
+        try {
+            upload_frequency_tables(g);
+            return;
+        } catch (const Error &e) {
+            if (e.code != PLX_ERR_BUDGET && e.code != PLX_ERR_NOMEM) throw;
+        }
+        // no room beside the old tables: without them, and with neither the geometry has no frequencies
+        g->d_dq.release();
+        g->d_inv_alpha.release();
+        g->d_wratio.release();
+        try {
+            upload_frequency_tables(g);
+        } catch (...) {
+            g->n_freq = 0;
+            throw;
+        }
     });
 }
 
@@ -913,32 +944,24 @@ plx_status plx_batch_add(plx_batch *b, int64_t tag, int32_t n_freq, const double
         r.n_freq = n_freq;
         r.pols = pols;
         const int per = is_bem(g) ? 1 : g->n_types;
+        KeepFrequencies keep(g);
         g->omega.insert(g->omega.end(), omega, omega + n_freq);
         if (alpha_w)
             for (size_t e = 0; e < (size_t)per * n_freq; ++e) g->alpha_w.push_back({alpha_w[2 * e], alpha_w[2 * e + 1]});
         g->n_freq += n_freq;
         upload_frequency_tables(g);
-        // slots: free ones first, then grown
+        // slots: free ones first, then grown; taken when the request is in place
         RefineState &S = b->st;
         int used = 0;
         for (const auto &s : S.slots) used += s.state != RefineState::Slot::FREE;
         S.grow(used + C);
-        for (int c = 0, s = 0; c < C; ++c) {
-            while (S.slots[s].state != RefineState::Slot::FREE) ++s;
-            RefineState::Slot &sl = S.slots[s];
-            sl = RefineState::Slot();
-            sl.state = RefineState::Slot::ACTIVE;
-            sl.freq = r.f0 + c / np;
-            sl.pol = pols[c % np];
-            sl.tol = tol;
-            sl.tag = tag;
-            r.slots.push_back(s);
-        }
+        for (int s = 0; (int)r.slots.size() < C; ++s)
+            if (S.slots[s].state == RefineState::Slot::FREE) r.slots.push_back(s);
         // right-hand sides into the slots; x = 0, r = b
         std::vector<int32_t> cf(C), cp(C);
         for (int c = 0; c < C; ++c) {
-            cf[c] = S.slots[r.slots[c]].freq;
-            cp[c] = S.slots[r.slots[c]].pol;
+            cf[c] = r.f0 + c / np;
+            cp[c] = pols[c % np];
         }
         DevArray<int32_t> dF, dP, dS;
         DevArray<double> Bt, Z;
@@ -959,8 +982,18 @@ plx_status plx_batch_add(plx_batch *b, int64_t tag, int32_t n_freq, const double
         ctx->launches += 3;
         PLX_CHECK_CUDA(cudaGetLastError());
         PLX_CHECK_CUDA(cudaStreamSynchronize(st));
-        b->req[tag] = std::move(r);
+        for (int c = 0; c < C; ++c) {
+            RefineState::Slot &sl = S.slots[r.slots[c]];
+            sl = RefineState::Slot();
+            sl.state = RefineState::Slot::ACTIVE;
+            sl.freq = cf[c];
+            sl.pol = cp[c];
+            sl.tol = tol;
+            sl.tag = tag;
+        }
         b->order.push_back(tag);
+        b->req[tag] = std::move(r);
+        keep.done = true;
     });
 }
 

@@ -209,12 +209,16 @@ void upload_pair_widths(plx_geom *g) {
 // wfq_module.f90:398-424); dipole diagonal sum_t f_t,i / alpha_t(w)
 // (wfqfmu_module.f90:698-746); Drude weights w_t = 2 n_t / (1/tau_t - i w)
 // (construct_H_minus_L_matrix, matrix_module.f90:435-482).
+//
+// The tables of g->n_freq frequencies replace the geometry's when they are all there: a
+// refused allocation leaves the ones it has.
 void upload_frequency_tables(plx_geom *g) {
     const int nt = g->n_types, F = g->n_freq;
+    DevArray<Cplx> d_dq, d_inv_alpha, d_wratio;
     if (is_bem(g)) {
         // z(w) = 2 pi (eps_s + eps(w)) / (eps_s - eps(w)) (new_gmres_diagonal_shift_bem,
         // bem_module.f90:977-997); alpha_w carries eps(w)
-        g->bem_z.resize(F);
+        std::vector<Cplx> z(F);
         for (int f = 0; f < F; ++f) {
             Cplx e = g->alpha_w[f];
             double nr = g->eps_solvent + e.re, ni = e.im;        // eps_s + eps
@@ -222,12 +226,14 @@ void upload_frequency_tables(plx_geom *g) {
             double m = dr * dr + di * di;
             double qr = (nr * dr + ni * di) / m, qi = (ni * dr - nr * di) / m;
             const double twopi = 6.283185307179586476925286766559;
-            g->bem_z[f] = {twopi * qr, twopi * qi};
+            z[f] = {twopi * qr, twopi * qi};
         }
-        g->d_dq.alloc(g->ctx, F);
-        PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_dq.p, g->bem_z.data(), F * sizeof(Cplx), cudaMemcpyHostToDevice,
+        d_dq.alloc(g->ctx, F);
+        PLX_CHECK_CUDA(cudaMemcpyAsync(d_dq.p, z.data(), F * sizeof(Cplx), cudaMemcpyHostToDevice,
                                        g->ctx->stream));
         PLX_CHECK_CUDA(cudaStreamSynchronize(g->ctx->stream));
+        g->bem_z.swap(z);
+        g->d_dq.swap(d_dq);
         return;
     }
     std::vector<Cplx> dq(nt * F), ia(nt * F), wr((size_t)nt * nt * F);
@@ -263,14 +269,17 @@ void upload_frequency_tables(plx_geom *g) {
             }
     }
     plx_ctx *ctx = g->ctx;
-    g->d_dq.alloc(ctx, nt * F);
-    g->d_inv_alpha.alloc(ctx, nt * F);
-    g->d_wratio.alloc(ctx, (size_t)nt * nt * F);
+    d_dq.alloc(ctx, nt * F);
+    d_inv_alpha.alloc(ctx, nt * F);
+    d_wratio.alloc(ctx, (size_t)nt * nt * F);
     cudaStream_t st = ctx->stream;
-    PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_dq.p, dq.data(), dq.size() * 16, cudaMemcpyHostToDevice, st));
-    PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_inv_alpha.p, ia.data(), ia.size() * 16, cudaMemcpyHostToDevice, st));
-    PLX_CHECK_CUDA(cudaMemcpyAsync(g->d_wratio.p, wr.data(), wr.size() * 16, cudaMemcpyHostToDevice, st));
+    PLX_CHECK_CUDA(cudaMemcpyAsync(d_dq.p, dq.data(), dq.size() * 16, cudaMemcpyHostToDevice, st));
+    PLX_CHECK_CUDA(cudaMemcpyAsync(d_inv_alpha.p, ia.data(), ia.size() * 16, cudaMemcpyHostToDevice, st));
+    PLX_CHECK_CUDA(cudaMemcpyAsync(d_wratio.p, wr.data(), wr.size() * 16, cudaMemcpyHostToDevice, st));
     PLX_CHECK_CUDA(cudaStreamSynchronize(st));
+    g->d_dq.swap(d_dq);
+    g->d_inv_alpha.swap(d_inv_alpha);
+    g->d_wratio.swap(d_wratio);
 }
 
 }  // namespace plx

@@ -155,6 +155,15 @@ int RefineState::grow(int need) {
     nB.alloc(ctx, (size_t)ncap * 2 * n);
     nX.alloc(ctx, (size_t)ncap * 2 * n);
     nR.alloc(ctx, (size_t)ncap * 2 * n);
+    try {
+        scratch(ncap);
+    } catch (...) {                          // the state as it was: what it held fits
+        nB.release();
+        nX.release();
+        nR.release();
+        if (cap > 0) scratch(cap);
+        throw;
+    }
     if (cap > 0) {
         const size_t b = (size_t)cap * 2 * n * 8;
         PLX_CHECK_CUDA(cudaMemcpyAsync(nB.p, ownB.p, b, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -173,7 +182,6 @@ int RefineState::grow(int need) {
     X = ownX.p;
     cap = ncap;
     slots.resize(cap);
-    scratch(cap);
     return cap;
 }
 
