@@ -268,6 +268,8 @@ void field_at_points(plx_geom *g, int pol, const double *d_x, int P, const doubl
     const bool fmu = g->model == PLX_WFQFMU;
     const auto *x = reinterpret_cast<const double2 *>(d_x);
     auto *fo = reinterpret_cast<double2 *>(d_field), *de = reinterpret_cast<double2 *>(d_dens);
+    // Numbers of blocks for a B200 (four and eight an SM); constant, because the parts fix the
+    // order of a point's sum and so its bits
     const int pairs = n_blocks(P, 2 * kPts);
     if (pairs >= 592) {
         (fmu ? field_points<2, true> : field_points<2, false>)<<<pairs, kPts, 0, ctx->stream>>>(

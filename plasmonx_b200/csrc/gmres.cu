@@ -742,7 +742,7 @@ __device__ void givens(int k, int lane, int j, double norm, const GivensTile &ti
 // The launch also enters the new slab and H column in the address tables, which the
 // kernels of the next steps read, and leaves the residual estimates in the run's words
 // (take_words): three 8-byte copies in, one back and a clearing of the H column (every
-// row that is read has been written) cost a step about 20 us of gaps between the kernels.
+// row that is read has been written) cost a step about 35 us of gaps between the kernels.
 constexpr int kNormChunks = 2;
 template <typename VT>
 __global__ void __launch_bounds__(kThreads) normalize_givens(int n, int j, const int32_t *__restrict__ act, int nparts,

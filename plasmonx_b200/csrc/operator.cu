@@ -38,7 +38,9 @@ constexpr int kOtfWarps = 8;
 constexpr int kOtfFewCols = 4;              // columns up to which it is used; the tiled form above
 constexpr int kOtfNoScratch = 16;           // columns up to which a product goes on without the tiled form's scratch
 
-// Warps per target atom: enough of them for ~24 warps on every SM.
+// Warps per target atom: enough of them for ~24 warps on every SM of a B200 (148).  The
+// split fixes the order of a target's sum, so it takes a constant, not the device's
+// number of SMs: a solve gives the same bits on every device.
 int otf_warps(int N) {
     int w = 1;
     while (w < kOtfWarps && (int64_t)N * w < 148 * 24) w *= 2;
@@ -752,7 +754,8 @@ void contract_t_impl(plx_geom *g, int count, const double *X, double *S, bool on
         const int N = g->n_atoms;
         if (count > kOtfFewCols) {
             // many columns: tiled product with T generated per slab; the split over the
-            // sources depends on the number of atoms only
+            // sources depends on the number of atoms only (592: four blocks an SM of a B200;
+            // constant for the same bits on every device)
             const int ca = fmu ? BN / 4 : BN, ka = fmu ? 4 : 16;
             const int tiles = n_blocks(N, ca);
             int js = std::max(1, std::min(64, (592 + tiles - 1) / tiles));

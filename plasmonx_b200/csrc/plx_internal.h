@@ -232,7 +232,7 @@ namespace plx {
 
 // How the T contraction of an operator application is computed.
 enum class Contraction : int {
-    FP64 = 0,       // stored T, FP64 on the CUDA cores
+    FP64 = 0,       // stored T, FP64 matrix instruction
     FP64_OTF = 1,   // tiles generated in the kernel, FP64
     TC3 = 2,        // stored T split in BF16 high/low, 3 tensor-core products
     TC1 = 3         // stored T rounded to BF16, 1 tensor-core product

@@ -124,8 +124,9 @@ __global__ void skinny_reduce(int n, int R, int ks, const double *__restrict__ p
     S[idx] = s;
 }
 
-// Number of K chunks and their length for a contraction of order n; depends on
-// n only, so that a column's sums do not depend on the batch it is part of.
+// Number of K chunks and their length for a contraction of order n; depends on n only
+// (592 blocks: four an SM of a B200, whatever the device), so that a column's sums depend
+// neither on the batch it is part of nor on the device.
 inline void skinny_split(int n, int &ks, int &kchunk) {
     const int cb = (n + kSkinnyCols - 1) / kSkinnyCols;
     ks = std::max(1, std::min(64, (592 + cb - 1) / cb));
