@@ -87,6 +87,11 @@ __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kch
 // eights that hold the batch up to 48 rows (the fastest of the tilings tried at each
 // size, 2 to 5 each at 893, 7,844 and 15,220 unknowns); 32 rows a warp above, where
 // the smaller tile's four blocks an SM beat 64 x 64 tiles (30 against 26 TF).
+// Chunks of up to 16 k (up to 1,024 unknowns) end after one round of loads, so a warp's
+// time is its latency and its stores: 16 x 16 tiles, four times as many blocks.  800
+// unknowns with the sum: 32 rows 18.0 -> 12.4 us, 48 rows 19.9 -> 15.3, 130 rows 31.0 ->
+// 29.5; 257 unknowns, 130 rows: 15.7 -> 11.6 (the CUDA-core form, 800 unknowns and 32
+// rows: 14.7).  At 1,400 unknowns (22 k) 130 rows take 57 us as below and 60 this way.
 template <bool TR = false>
 void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, const double *X, const double *T,
                                    double *part) {
@@ -95,6 +100,7 @@ void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, c
                dim3((n + 32 / WR * NT - 1) / (32 / WR * NT), (R + 8 * MT * WR - 1) / (8 * MT * WR), ks), 128, 0, st, R, \
                n, kchunk, X, T, part)
     if (R <= 8) PLX_PP(1, 4, 4, 1, 1);
+    else if (kchunk <= 16) PLX_PP(2, 2, 4, 2, 1);
     else if (R <= 16) PLX_PP(2, 4, 4, 1, 1);
     else if (R <= 24) PLX_PP(3, 4, 4, 1, 3);
     else if (R <= 32) PLX_PP(4, 4, 4, 1, 2);
