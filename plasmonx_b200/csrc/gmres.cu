@@ -1310,7 +1310,7 @@ class GmresRun final : public GmresStepper {
     // A residual with the pending word's bits costs that wait, nothing else.
     const double *await_residuals(int na) {
         if (!host_.p) {
-            ++ctx_->copied_steps;
+            --ctx_->copy_steps;
             return read_words(0, na);
         }
         const volatile uint64_t *w = reinterpret_cast<const volatile uint64_t *>(host_.p);
@@ -1327,14 +1327,13 @@ class GmresRun final : public GmresStepper {
         return host_.p;
     }
 
-    // The words the kernels leave norms and residuals in: pinned host memory once the
-    // context has taken kCopiedSteps steps, device memory and a copy before that and
-    // where no memory can be pinned (tried again as many steps later).
+    // The words the kernels leave norms and residuals in: pinned host memory, or device
+    // memory and a copy where none can be pinned (tried again kCopiedSteps steps later).
     void take_words() {
-        const bool pin = ctx_->copied_steps >= kCopiedSteps;
+        const bool pin = ctx_->copy_steps <= 0;
         host_.alloc(ctx_, (size_t)2 * C_, pin);
         if (host_.p) return;
-        if (pin) ctx_->copied_steps = 0;
+        if (pin) ctx_->copy_steps = kCopiedSteps;
         if (!dev_words_.p) {
             dev_words_.alloc(ctx_, (size_t)2 * C_);
             copy_.resize((size_t)2 * C_);

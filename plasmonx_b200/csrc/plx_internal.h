@@ -98,14 +98,13 @@ struct PinnedArray {
 };
 constexpr size_t kPinnedKeep = 8192;      // 64 KB
 constexpr size_t kPinnedBlocks = 32;
-// GMRES steps of a context that read their residuals by a copy before it pins memory
-// for them.  Pinning takes 1-3.4 ms, a step's copy 12-14 us more than reading pinned
-// words (262 steps at 893 unknowns: 43.2 against 39.6 ms): 96 steps cost about what the
-// pinning does, so a context that takes few steps never pays for it and one that takes
-// many pays about twice the cheaper form, once.  First solve of a new 8,000-tessera
-// surface (53 steps; 19.5 ms after it): 30.6 ms pinned from the first step, 29.4 now; of
-// 893 unknowns (262 steps; 39.6 ms): 45.2 and 45.3 (quartiles of 16 new contexts).
-constexpr int64_t kCopiedSteps = 96;
+// Steps that read their residuals by a copy after pinned memory was refused, before it is
+// tried again (a copy costs a step 12-14 us more: 262 steps at 893 unknowns 43.2 against
+// 39.6 ms).  Copies for a context's first 96 steps in place of pinning 4 KB at once, which
+// takes up to 3.4 ms where no other context holds pinned memory and next to nothing where
+// one does, were no better: first solve of a new 8,000-tessera surface 30.6 -> 29.4 ms
+// alone and 28.6 -> 29.2 beside another context, of 893 unknowns 45.2 -> 45.3 and 43 -> 44.
+constexpr int64_t kCopiedSteps = 256;
 
 }  // namespace plx
 
@@ -133,7 +132,7 @@ struct plx_ctx {
     uint32_t wait_limit = kDefaultWaitLimit;
     std::mutex pinned_mutex;
     std::vector<std::pair<double *, size_t>> pinned;   // free blocks of PinnedArray
-    int64_t copied_steps = 0;                          // see kCopiedSteps
+    int64_t copy_steps = 0;                            // see kCopiedSteps
     // contraction profiling (plx_profile_enable)
     bool profile = false;
     std::vector<cudaEvent_t> prof_events;   // pairs (start, stop), reused
