@@ -30,8 +30,8 @@ constexpr int kSkinnyCols = 256;
 //   366, 32 rows 1,098 -> 686, 42 rows 1,470 -> 863, 512 rows 12.4 -> 7.9 ms (30 TF).
 // TR: the matrix is given by its transpose (T[k][col] lies at T[col * n + k]), read in
 // 32-byte pieces; the sums are the same.  Rows beyond the batch and k beyond the chunk
-// are zeros.  The order of an
-// element's sum depends on n alone (skinny_split): not on R, MT, NT or its place.
+// are zeros.  The order of an element's sum depends on n alone (skinny_split): not on R,
+// MT, NT or its place.
 template <int MT, int NT, int D, int WR, int MB, bool TR>
 __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kchunk, const double *__restrict__ Xt,
                                                            const double *__restrict__ T,
@@ -85,22 +85,24 @@ __global__ void __launch_bounds__(128, MB) product_partial(int R, int n, int kch
 
 // Launches the partial products of R rows over ks chunks.  Row tiles: the fewest
 // eights that hold the batch up to 48 rows (the fastest of the tilings tried at each
-// size, 2 to 5 each at 893, 7,844 and 15,220 unknowns); 32 rows a warp above, where
+// size, 2 to 5 each at 7,844 and 15,220 unknowns); 32 rows a warp above, where
 // the smaller tile's four blocks an SM beat 64 x 64 tiles (30 against 26 TF).
 // Chunks of up to 16 k (up to 1,024 unknowns) end after one round of loads, so a warp's
-// time is its latency and its stores: 16 x 16 tiles, four times as many blocks.  800
-// unknowns with the sum: 32 rows 18.0 -> 12.4 us, 48 rows 19.9 -> 15.3, 130 rows 31.0 ->
-// 29.5; 257 unknowns, 130 rows: 15.7 -> 11.6 (the CUDA-core form, 800 unknowns and 32
-// rows: 14.7).  At 1,400 unknowns (22 k) 130 rows take 57 us as below and 60 this way.
+// time is its latency and its stores, and 16 x 16 tiles, four times as many blocks, are
+// faster until there are blocks enough without them.  Times with the sum, in those tiles
+// against the ones above: 257 unknowns, 130 rows 11.7 against 16.0 us, 366 rows 19.6
+// against 24.1; 800 unknowns, 32 rows 12.3 against 18.1, 48 rows 15.3 against 19.9 (the
+// CUDA-core form, 34 rows: 14.9), 366 rows 82.5 against 74.2; 893 unknowns, 130 rows 33.7
+// against 35.7, 366 rows 99 against 95; 1,400 unknowns (22 k), 130 rows 64 against 57.
 template <bool TR = false>
 void launch_product_partial(cudaStream_t st, int R, int n, int ks, int kchunk, const double *X, const double *T,
-                                   double *part) {
+                            double *part) {
 #define PLX_PP(MT, NT, D, WR, MB)                                                                                  \
     launch_pdl(product_partial<MT, NT, D, WR, MB, TR>,                                                                 \
                dim3((n + 32 / WR * NT - 1) / (32 / WR * NT), (R + 8 * MT * WR - 1) / (8 * MT * WR), ks), 128, 0, st, R, \
                n, kchunk, X, T, part)
     if (R <= 8) PLX_PP(1, 4, 4, 1, 1);
-    else if (kchunk <= 16) PLX_PP(2, 2, 4, 2, 1);
+    else if (kchunk <= 16 && (int64_t)R * n <= 160000) PLX_PP(2, 2, 4, 2, 1);
     else if (R <= 16) PLX_PP(2, 4, 4, 1, 1);
     else if (R <= 24) PLX_PP(3, 4, 4, 1, 3);
     else if (R <= 32) PLX_PP(4, 4, 4, 1, 2);
